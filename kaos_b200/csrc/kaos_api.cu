@@ -47,7 +47,7 @@ static size_t ena_push_smem(int nq, int ntubes) {
 // k_cx_convert's shared memory: conversions still owed per cell, per-warp
 // per-cell counts (8 warps), the chunk's Qindk1
 static size_t cx_convert_smem(int nq) {
-  return ((size_t)9 * nq + CX_CHUNK) * sizeof(unsigned);
+  return ((size_t)cx_qs_word(nq) + CX_CHUNK) * sizeof(unsigned);
 }
 
 // Positive root u = r/RE of q^2 u^4 + u/p - 1 = 0: closed form of the

@@ -279,16 +279,20 @@ __device__ __forceinline__ void cx_convert_ion(const CxArgs &a, const TubeD &T,
 // conversions in order; they take consecutive ENA slots from cxbase in index
 // order and are converted by all threads at once.
 constexpr int CX_WARPS = 8;  // 256-thread blocks
+// First word of the staged Qindk1 in k_cx_convert's shared memory: behind the
+// owed and the per-warp counts, on a 16-byte boundary for any cell count (the
+// staging stores are 16 bytes wide).
+__host__ __device__ constexpr int cx_qs_word(int nq) { return ((1 + CX_WARPS) * nq + 3) & ~3; }
 static_assert(CX_CHUNK <= (1 << 14), "conversion list packs (cell << 14) | index");
 __device__ __forceinline__ void cx_convert_chunk(const CxArgs &a, int c, int t) {
   // a copy: every barrier below would otherwise reload the fields from
   // global memory, and the staging traffic evicts them from L1
   const TubeD T = a.tubes[t];
   __syncthreads();  // the previous chunk of this block is done with smem
-  extern __shared__ unsigned sm_[];
+  extern __shared__ __align__(16) unsigned sm_[];
   unsigned *need = sm_;             // conversions this chunk owes per cell
   unsigned *wcnt = sm_ + a.nqmax;   // [CX_WARPS][nq]: counts, then ranks
-  int *qs = (int *)(wcnt + CX_WARPS * a.nqmax);  // Qindk1, then the lists
+  int *qs = (int *)(sm_ + cx_qs_word(a.nqmax));  // Qindk1, then the lists
   __shared__ unsigned wconv[CX_WARPS];
   const int64_t beg = a.cx_start[c];
   const int nk = (int)min((int64_t)CX_CHUNK, a.nlive[t] - beg);

@@ -206,3 +206,17 @@ def test_moments_all_equals_each_selector():
     with pytest.raises(ValueError):
         s.moments_all(out=np.zeros((3, tube.nq)))
     s.close()
+
+
+@pytest.mark.parametrize("nq", [29, 30, 31])
+def test_charge_exchange_odd_cell_counts(nq):
+    """Selection chunks with full, 16-byte aligned segments in tubes whose
+    cell count is no multiple of four (the staged Qindk1 follow 9 words per
+    cell in shared memory)."""
+    mi = ModelInput(h=0.01, ndatfac=3, ION2VPERPflag=1, QEXCHANGEflag=1)
+    spec = TubeSpec(L=4.0, nq=nq, n_particles=9000, q_ub=0.15, H=600e3,
+                    neut_n0=3e18, neut_H=300e3)
+    s, o = _run_one(mi, spec, make_vgrid(True, 16, 16, 24, 8e3), 7)
+    assert s.count(0)[1] > 0
+    _compare(s, 0, o)
+    s.close()
