@@ -233,7 +233,10 @@ int kaos_set_fields(kaos_handle *h, int32_t tube, const double *EAmag,
  * ComputationalTimeStepLoop (_8_KineticSolver.f90:54-239): charge exchange,
  * BoundaryConditionsSub, AmbipolarEfieldSub/GravfieldSub, KineticSolverA/B
  * (push, injection, counts, distribution functions, moments).  The first
- * call performs the n=1 step of KineticSolverASub. */
+ * call performs the n=1 step of KineticSolverASub.  In mixed precision,
+ * consecutive ordinary steps of a call (no master step among them, no ion to
+ * convert to an ENA in the interval) run in one launch with each ion's state
+ * in registers; results do not depend on how steps are spread over calls. */
 int kaos_step(kaos_handle *h, int64_t nsteps);
 
 /* Number of computational steps taken so far (reference n - 1). */
@@ -308,7 +311,8 @@ int kaos_get_boundary_ena(kaos_handle *h, int32_t tube, int64_t *lb_out,
 int kaos_get_timing(kaos_handle *h, double *ms, int64_t *launches);
 
 /* Device time (ms) spent in the particle push kernels alone during the last
- * kaos_step call (CUDA events around each push launch) and their count.
+ * kaos_step call (CUDA events around each push launch) and the number of
+ * those launches (a run of ordinary steps is one launch, see kaos_step).
  * Steps replayed from CUDA graphs carry no per-push events and are not
  * included. */
 int kaos_get_push_timing(kaos_handle *h, double *ms, int64_t *launches);
@@ -343,7 +347,8 @@ int kaos_sample_rng(int32_t kind, uint64_t seed, uint64_t id0, uint32_t step,
  * directly (0, default).  With graphs on, each kind of step (ordinary runs
  * of up to 8 steps, the step before a master step, the master step) is
  * captured once per ion/ENA buffer parity and replayed; the step number
- * lives in device memory, so a replay needs no host update.  Results are
+ * lives in device memory, so a replay needs no host update.  Ordinary steps
+ * that one launch takes together (kaos_step) are launched directly.  Results are
  * identical to the direct launches.  Step 1 always runs directly.  No
  * reference counterpart (the Fortran loop calls each routine per step,
  * _8_KineticSolver.f90:54-239). */
@@ -359,8 +364,9 @@ int kaos_set_graph(kaos_handle *h, int32_t on);
  * one (0 = the same as bits 1-2).  chunk = 0 or mode < 0 re-arms the
  * autotuner, which is on by default: before the first step after step 1 it
  * times the push of every candidate on a copy of the ion state and keeps
- * the fastest, then the master-step variant's budget alone.  Results do not depend on the shape.  No reference
- * counterpart (the reference has one MPI rank per core,
+ * the fastest, then the master-step variant's budget alone.  Runs of steps
+ * (kaos_step) have a shape of their own.  Results do not depend on the
+ * shape.  No reference counterpart (the reference has one MPI rank per core,
  * _8_KineticSolver.f90:43-44). */
 int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode);
 

@@ -47,6 +47,11 @@ struct PushArgs {
   int cx_stride, cx_chunk;
   // graph replay: the step number is read from device memory
   const uint32_t *dstep;
+  // a run of nsub ordinary steps in one launch (k_push32 RUN): steps step ..
+  // step + nsub - 1; the last one is the step write_qind / write_qk4 are for
+  unsigned nsub;
+  // not null: the launch leaves its last step number there (graph replay)
+  uint32_t *dstep_w;
   // Philox key schedule of the seed: key words of round r at rk[2r], rk[2r+1]
   uint32_t rk[20];
 };
@@ -916,8 +921,16 @@ __device__ __forceinline__ void start_bins(const PushArgs &a, const Ions &I,
 // picks one.  K64 (precision mode KAOS_PREC_MIXED_K64) computes the heating
 // kick in FP64 from the FP64 state, with the FP64 path's formula and Philox
 // draw; the rest of the step is unchanged.
-template <bool THREE_D, int NT, int MINB, bool PERSIST, bool MASTER, bool K64>
+//
+// RUN: nsub ordinary steps per launch.  Between two master steps whose
+// interval converts no ion the steps of different ions are independent, so an
+// ion's state stays in registers from its first to its last step of the run:
+// it is loaded and stored once instead of once per step, and every step does
+// the arithmetic of the one-step variant in the same order (bit-identical
+// results however a run is cut, tests/test_gpu_runs.py).
+template <bool THREE_D, int NT, int MINB, bool PERSIST, bool MASTER, bool K64, bool RUN>
 __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
+  static_assert(!(RUN && (MASTER || PERSIST)), "runs hold ordinary steps, one item per block");
   // master-step work (field re-interpolation, binning) only in the MASTER
   // variant: the ordinary step carries none of its code or registers
   const bool bin = MASTER && a.bin, prologue = MASTER && a.prologue,
@@ -935,7 +948,9 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   const float h = (float)a.h, hh = 0.5f * h, h6 = h / 6.0f, hsq2 = 0.5f * h * h;
   const float hh6 = h * h6;
   const double hd = a.h;
-  const uint32_t step = a.dstep ? *a.dstep : a.step;
+  const uint32_t step0 = a.dstep ? *a.dstep : a.step;
+  const unsigned nsub = RUN ? a.nsub : 1u;
+  if (a.dstep_w && blockIdx.x == 0 && threadIdx.x == 0) *a.dstep_w = step0 + nsub - 1u;
   const float fRE = (float)RE;
   const ForceC fc = force_c(a.ff);
   Ions I = a.ion;
@@ -998,7 +1013,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     }
     tcur = t;
   }
-  if (a.cxc)
+  if (!RUN && a.cxc)
     for (int k = threadIdx.x; k < T.nq; k += blockDim.x) HC[k] = 0u;
   BinWin W{};
   if (bin) {
@@ -1026,13 +1041,14 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   int32_t *__restrict__ QI = I.qind + base;
   const uint64_t *__restrict__ ID = I.id + base;
   // Software pipeline: the state of the next ion of this thread is loaded
-  // before the current one is pushed, so its HBM latency overlaps the work.
+  // before the current one is pushed, so its HBM latency overlaps the work
+  // (not in a run, whose steps hide it and need the registers).
   double n_x = XDEAD, n_vp = 0.0;
   double2 n_v = make_double2(0.0, 0.0);
   float2 n_f = make_float2(0.f, 0.f);
   uint64_t n_id = 0;
   float n_qk = 0.f;  // q_k4 of the master-step field re-interpolation
-  if ((int)threadIdx.x < nk) {
+  if (!RUN && (int)threadIdx.x < nk) {
     const unsigned k = threadIdx.x;
     n_x = X[k];
     n_vp = VP[k];
@@ -1043,13 +1059,20 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   }
   for (unsigned k = threadIdx.x; k < (unsigned)nk; k += NT) {
     const int64_t j = base + k;  // the ion's slot (2D grid: its stale bins)
-    const double x0 = n_x;
-    const double vpar = n_vp;
-    const double v1 = n_v.x, v2 = n_v.y;
+    if (RUN) {
+      n_x = X[k];
+      n_vp = VP[k];
+      n_v = V12[k];
+      n_f = FF[k];
+      if (a.icr) n_id = ID[k];
+    }
+    double x0 = n_x;
+    double vpar = n_vp;
+    double v1 = n_v.x, v2 = n_v.y;
     float aea = n_f.x, ag = n_f.y;
     const uint64_t pid = n_id;
     const float qk0 = n_qk;
-    if (k + NT < (unsigned)nk) {
+    if (!RUN && k + NT < (unsigned)nk) {
       const unsigned kn = k + NT;
       n_x = X[kn];
       n_vp = VP[kn];
@@ -1059,8 +1082,18 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       if (prologue) n_qk = QK[kn];
     }
     if (x0 < XDEAD_LIM) continue;  // slot marked DEAD
-    const int c0 = x_cell(x0, T.nq);
-    const double o0 = x0 - (double)c0;  // exact
+    int c0 = x_cell(x0, T.nq);
+    double c0d = (double)c0;
+    // a run on the 2D grid keeps the last speeds inside the grid and searches
+    // their bins once, after its last step: the stale-index rule keeps the
+    // bins of the last value inside
+    double l_vp = 0.0, l_s = 0.0;
+    bool in_vp = false, in_s = false;
+#pragma unroll 1
+    for (unsigned m = 0;;) {
+    const uint32_t step = step0 + m;
+    const bool last = !RUN || m + 1u == nsub;
+    const double o0 = x0 - c0d;  // exact
     if (prologue) field_prologue32(a.ff, T, E, Cc, FE, qk0, c0, qs_ms, aea, ag);
     // ---- start-of-step position: q, then (r, theta) by FP64 Newton -------
     const double q0 = fma(o0, DQ[c0], QL[c0]);
@@ -1114,7 +1147,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       start_bins<THREE_D>(a, I, j, VE1, VE2, VEP, VT1, VT2, VTP, vpar, v1, v2, b1, b2, bp);
       if (bin) accumulate_win(a.acc, T, W, qi, b1, b2, bp, a.exporting);
       if (a.write_qind) QI[k] = qi;
-      continue;
+      break;
     }
     double v1n = v1, v2n = v2;  // after the wave-heating kick
     // (the FP64 kick of K64 runs after the position and V|| stores below:
@@ -1140,7 +1173,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       }
     }
     // stored at once: the kicked pair holds no registers through the RK
-    if (!K64 && a.icr) V12[k] = make_double2(v1n, v2n);
+    if (!RUN && !K64 && a.icr) V12[k] = make_double2(v1n, v2n);
     // ---- the stage accelerations ----------------------------------------
     // a|| = M + s C0 + ce1 AEA with the signed mirror term M (cos(theta) in
     // place of s |cos|: smooth through the equator), the hemisphere sign s
@@ -1168,7 +1201,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     const float a2 = fmaf(dM, ds2, M1) + (z2 <= 0.0f ? -C0 : C0) + Ce;
     const float a4 = fmaf(dM, ds4, M1) + (z4 <= 0.0f ? -C0 : C0) + Ce;
     // q at the k4 point: dq/ds = -RE^2 sqrt(ell) / r^3 along e1
-    if (a.write_qk4)
+    if (last && a.write_qk4)
       QK[k] = fmaf(-(float)(RE * RE) * (g1.ell * g1.isl) * (g1.ir * g1.ir * g1.ir), ds4, g1.q);
     // ---- displacement h/6 (V_R + 4 (V_R + h/2 A1) + (V_R + h A2)) ---------
     // = h V|| e1 (FP64, above) + h^2/6 (2 a1 + a2) e1 (FP32; the k2 point's
@@ -1185,30 +1218,53 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     // and an offset strictly inside (0, 1) there decides it without the
     // edge search; escaped ions keep the end cell and an offset outside
     const int cs = qi >= 0 ? qi : c0;
-    double od = (qN - QL[cs]) * IDQ[cs];
-    int cpos = cs;
-    if (!(od > 1e-9 && od < 1.0 - 1e-9)) {
+    // (the product rounded on its own on every path: no fused multiply-add
+    // with the cell number)
+    double od = __dmul_rn(qN - QL[cs], IDQ[cs]);
+    double xN;
+    if (od > 1e-9 && od < 1.0 - 1e-9) {
+      // (a run: qi = c0 has been the cell of x0 all along unless the start
+      // lay next to an edge; the sum stays strictly inside the cell)
+      if (RUN) {
+        if (cs != c0) { c0 = cs; c0d = (double)cs; }
+        xN = c0d + od;
+      } else {
+        xN = (double)cs + od;
+      }
+    } else {
       const int cN = cell_search_from(E, T.nq, T.sgn * qN, cs);
-      cpos = cN >= 0 ? cN : (cN == BELOW ? 0 : T.nq - 1);
-      od = (qN - QL[cpos]) * IDQ[cpos];
+      const int cpos = cN >= 0 ? cN : (cN == BELOW ? 0 : T.nq - 1);
+      od = __dmul_rn(qN - QL[cpos], IDQ[cpos]);
+      xN = (double)cpos + od;
+      if (RUN) {  // the cell as the next step reads it from the coordinate
+        c0 = x_cell(xN, T.nq);
+        c0d = (double)c0;
+      }
     }
-    const double xN = (double)cpos + od;
     // ---- V|| along the new field direction ------------------------------
     const float dth = (zf * fmaf(h, VRr, ddr) - rf * fmaf(h, VRz, ddz)) * (g1.ir * g1.ir);
     const float dal = 3.0f * fmaf(g1.ct, g1.ct, 1.0f) * (g1.isl * g1.isl) * dth;
     const float dv = fmaf(h6, a1 + 4.0f * a2 + a4, -0.5f * vparf * dal * dal);
     const double vparN = vpar + (double)dv;
-    if (bin || !THREE_D) {
+    if (RUN && !THREE_D) {
+      if (vpar >= VEP[0] && vpar <= VEP[c_vg.npar]) { l_vp = vpar; in_vp = true; }
+      if (m == 0u || a.icr) {  // (the speed changes only by the kicks)
+        const double sp = vperp_mag(v1, v2);
+        if (sp >= VE1[0] && sp <= VE1[c_vg.n1]) { l_s = sp; in_s = true; }
+      }
+    } else if (bin || !THREE_D) {
       int b1, b2, bp;
       start_bins<THREE_D>(a, I, j, VE1, VE2, VEP, VT1, VT2, VTP, vpar, v1, v2, b1, b2, bp);
       if (bin) accumulate_win(a.acc, T, W, qi, b1, b2, bp, a.exporting);
     }
-    if (!isfinite(vparN) || !isfinite(xN)) atomicOr(a.status, ST_NAN);
-    X[k] = xN;
-    VP[k] = vparN;
-    if (prologue) FF[k] = make_float2(aea, ag);
-    if (a.write_qind) QI[k] = qi;
-    if (a.cxc && qi >= 0) atomicAdd(&HC[qi], 1u);
+    if (!RUN) {
+      if (!isfinite(vparN) || !isfinite(xN)) atomicOr(a.status, ST_NAN);
+      X[k] = xN;
+      VP[k] = vparN;
+      if (prologue) FF[k] = make_float2(aea, ag);
+    }
+    if (last && a.write_qind) QI[k] = qi;
+    if (!RUN && a.cxc && qi >= 0) atomicAdd(&HC[qi], 1u);
     if (K64 && a.icr) {
       if (qi >= 0) {
         // FP64 kick at the start-of-step point: Omega = (q/m) MDIP sqrt(ell)
@@ -1227,11 +1283,31 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
           heat<double>(a, step, hc, pid, invsumds64, Om, invOm, fabs(vpar), v1n, v2n);
         }
       }
-      V12[k] = make_double2(v1n, v2n);
+      if (!RUN) V12[k] = make_double2(v1n, v2n);
+    }
+    if (!RUN) break;
+    x0 = xN;
+    vpar = vparN;
+    v1 = v1n;
+    v2 = v2n;
+    if (++m == nsub || x0 < XDEAD_LIM) break;
+    }  // steps of the run
+    if (RUN) {  // a value that is not finite stays so to the end of the run
+      if (!isfinite(vpar) || !isfinite(x0)) atomicOr(a.status, ST_NAN);
+      X[k] = x0;
+      VP[k] = vpar;
+      if (a.icr) V12[k] = make_double2(v1, v2);
+      if (!THREE_D) {
+        const int old = I.vb[j];
+        const int bp = in_vp ? vbin_tab(VTP, VEP, c_vg.npar, l_vp) : (old & 0xffff) - 1;
+        const int b1 = in_s ? vbin_tab(VT1, VE1, c_vg.n1, l_s) : (old >> 16) - 1;
+        const int nw = ((b1 + 1) << 16) | (bp + 1);
+        if (nw != old) I.vb[j] = nw;
+      }
     }
   }
   if (bin) bin_win_flush(a.acc, T, W);
-  if (a.cxc) flush_cx_counts(a, t, beg, T.nq, HC);
+  if (!RUN && a.cxc) flush_cx_counts(a, t, beg, T.nq, HC);
   if (!PERSIST) break;  // one item per block: no loop-carried state
   }  // work items
 }

@@ -1,0 +1,89 @@
+"""Runs of ordinary steps in one launch: the state after kaos_step(n) equals
+that of n calls of kaos_step(1) bit for bit, however the run is cut, for
+every precision mode, both velocity grids, heating on and off, escaping ions
+and speeds that leave the grid."""
+import numpy as np
+import pytest
+
+from kaos_b200 import build as kbuild
+from kaos_b200 import grids
+from kaos_b200.grids import TubeSpec, make_tube, make_vgrid
+from kaos_b200.lib import Solver
+from kaos_b200.model_input import KAOS_PREC_FP64, KAOS_PREC_MIXED, KAOS_PREC_MIXED_K64, ModelInput
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _build():
+    kbuild.build()
+
+
+def _solver(mi, tubes, init, vg, graph=False):
+    s = Solver(mi, tubes, vg)
+    for k, a in enumerate(init):
+        s.load(k, *a)
+    s.set_graph(graph)
+    return s
+
+
+def _state(s, n):
+    out = []
+    for k in range(n):
+        p = s.state(k)
+        # (a mixed run stores Qindk1 only for the master step that reads it)
+        out += [p[x] for x in ("q", "vpar", "vperp1", "vperp2")]
+        out += [s.moments_all(k), s.counts(k), s.boundary(k)]
+    return out
+
+
+PRECS = (KAOS_PREC_FP64, KAOS_PREC_MIXED, KAOS_PREC_MIXED_K64)
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("three_d", [True, False])
+@pytest.mark.parametrize("heating", [True, False])
+def test_runs_equal_single_steps(prec, three_d, heating):
+    # two tubes, ion counts around the work-item sizes; a velocity grid that
+    # many ions leave (the 2D grid's stale bins matter)
+    mi = ModelInput(h=0.5, ndatfac=7, ION2VPERPflag=1 if three_d else 0,
+                    ICRflag=1 if heating else 0, precision=prec)
+    specs = [TubeSpec(L=3.0, nq=nq, n_particles=n, q_ub=0.5, H=400e3, Ti=5.0 * 1.602e-19 / 138e-25,
+                      heat_rate_eV_s=2.0 if heating else 0.0) for nq, n in ((24, 1025), (31, 257))]
+    tubes = [make_tube(sp, mi) for sp in specs]
+    for t in tubes:
+        t.nsnormCLB = 9.0
+    vg = make_vgrid(True, 16, 16, 24, 9e3) if three_d else make_vgrid(False, 12, 0, 24, 7e3)
+    init = [grids.initial_particles(t, sp, mi, seed=3) for t, sp in zip(tubes, specs)]
+    a, b = _solver(mi, tubes, init, vg), _solver(mi, tubes, init, vg)
+    g = _solver(mi, tubes, init, vg, graph=True)
+    done = 0
+    for n in (1, 13, 2, 1, 4, 14, 6):  # cuts inside and at the ends of intervals
+        a.step(n)
+        g.step(n)
+        for _ in range(n):
+            b.step(1)
+        done += n
+        for x, y, z in zip(_state(a, 2), _state(b, 2), _state(g, 2)):
+            assert np.array_equal(x, y), done
+            assert np.array_equal(x, z), done
+    assert a.boundary(0)[:2].sum() > 0  # ions escaped
+    for s in (a, b, g):
+        s.close()
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 5000])
+def test_run_ion_counts(n):
+    mi = ModelInput(h=0.01, ndatfac=5, ION2VPERPflag=1, ICRflag=1, precision=KAOS_PREC_MIXED)
+    spec = TubeSpec(L=4.0, nq=24, n_particles=6000, q_ub=0.15, H=600e3, heat_rate_eV_s=5.0)
+    t = make_tube(spec, mi)
+    init = [tuple(x[:n] for x in grids.initial_particles(t, spec, mi, seed=2))]
+    vg = make_vgrid(True, 16, 16, 24, 8e3)
+    a, b = _solver(mi, [t], init, vg), _solver(mi, [t], init, vg)
+    a.step(14)
+    for _ in range(14):
+        b.step(1)
+    for x, y in zip(_state(a, 1), _state(b, 1)):
+        assert np.array_equal(x, y)
+    a.close()
+    b.close()
