@@ -233,8 +233,8 @@ int kaos_set_fields(kaos_handle *h, int32_t tube, const double *EAmag,
  * ComputationalTimeStepLoop (_8_KineticSolver.f90:54-239): charge exchange,
  * BoundaryConditionsSub, AmbipolarEfieldSub/GravfieldSub, KineticSolverA/B
  * (push, injection, counts, distribution functions, moments).  The first
- * call performs the n=1 step of KineticSolverASub.  In mixed precision,
- * consecutive ordinary steps of a call (no master step among them, no ion to
+ * call performs the n=1 step of KineticSolverASub.
+ * Consecutive ordinary steps of a call (no master step among them, no ion to
  * convert to an ENA in the interval) run in one launch with each ion's state
  * in registers; results do not depend on how steps are spread over calls. */
 int kaos_step(kaos_handle *h, int64_t nsteps);

@@ -400,8 +400,13 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
        {KAOS_K32(true, false, true), KAOS_K32(true, true, true)}}};
 #undef KAOS_K32
   const int nt = rs == 2 ? 128 : PUSH_THREADS;
-  static const KFn k64[2][2] = {{k_push64<false, false>, k_push64<false, true>},
-                                {k_push64<true, false>, k_push64<true, true>}};
+  static const KFn k64[2][2] = {
+      {k_push64<false, 256, 2, false, false>, k_push64<false, 256, 2, true, false>},
+      {k_push64<true, 256, 2, false, false>, k_push64<true, 256, 2, true, false>}};
+  // FP64 runs: 80 registers (24 warps per SM) spill 32 B; the 124-register
+  // build (16 warps) spills nothing and is 5 % slower on 1e7 ions, 13 % on 1e5
+  static const KFn k64run[2] = {k_push64<false, 256, 3, false, true>,
+                                k_push64<true, 256, 3, false, true>};
   // runs of steps: [FP64 heating kick][three_d]; 256 threads x 3 blocks per
   // SM (64-register and 128-thread builds measured the same within 2 % on
   // 1e7 ions, the latter 20 % slower on batches of uneven tubes)
@@ -410,7 +415,7 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
        k_push32<true, 256, 3, false, false, false, true>},
       {k_push32<false, 256, 3, false, false, true, true>,
        k_push32<true, 256, 3, false, false, true, true>}};
-  const KFn fn = run ? k32run[h->kick64][h->three_d]
+  const KFn fn = run ? (h->mixed ? k32run[h->kick64][h->three_d] : k64run[h->three_d])
                      : (h->mixed ? k32[h->kick64][ms][h->three_d][rs][ps] : k64[h->three_d][ps]);
   if (smem > 48 * 1024)
     CK(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1065,7 +1070,7 @@ int step_once(kaos_handle *h) {
 // stays below 0.1 s.
 constexpr int64_t RUN_MAX = 64;
 int64_t run_length(const kaos_handle *h, int64_t n, int64_t most) {
-  if (!h->mixed || n < 2 || (h->P.QEXCHANGEflag == 1 && !h->cx_idle)) return 0;
+  if (n < 2 || (h->P.QEXCHANGEflag == 1 && !h->cx_idle)) return 0;
   int64_t g = 0;
   most = std::min(most, RUN_MAX);
   while (g < most && !is_master(h, n + g)) ++g;

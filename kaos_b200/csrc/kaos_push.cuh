@@ -714,22 +714,26 @@ __device__ __forceinline__ HeatC<T> heat_consts(const CellTables &c, int64_t g) 
 }
 
 // ---------------------------------------------------------------------------
-// FP64 kernel: ions stored as meridian-plane (rho, z) in FP64.
-template <bool THREE_D, bool PERSIST>
-__global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
+// FP64 kernel: ions stored as meridian-plane (rho, z) in FP64.  RUN: nsub
+// ordinary steps per launch with the ion's state in registers, as in k_push32.
+template <bool THREE_D, int NT, int MINB, bool PERSIST, bool RUN>
+__global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
   extern __shared__ double sm[];
   const int nqmax = a.nqs;
   double *E = sm, *Cc = sm + nqmax + 1;
   unsigned *HC = (unsigned *)(Cc + nqmax);
   const double h = a.h, hh = 0.5 * a.h, h6 = a.h / 6.0, hsq2 = 0.5 * a.h * a.h;
-  const uint32_t step = a.dstep ? *a.dstep : a.step;
+  const uint32_t step0 = a.dstep ? *a.dstep : a.step;
+  const unsigned nsub = RUN ? a.nsub : 1u;
+  if (a.dstep_w && blockIdx.x == 0 && threadIdx.x == 0) *a.dstep_w = step0 + nsub - 1u;
+  const bool bin = !RUN && a.bin, prologue = !RUN && a.prologue, bin_only = !RUN && a.bin_only;
   Ions I = a.ion;
   TubeD T;
   int tcur = -1;
   // velocity-cell edges for the bin searches: shared memory serves the
   // threads' different addresses in parallel (constant memory serialises)
   __shared__ double VE1[MAXV + 1], VE2[MAXV + 1], VEP[MAXV + 1];
-  if (a.bin || !THREE_D) load_vgrid_smem(c_vg.e1, c_vg.e2, c_vg.epar, VE1, VE2, VEP);
+  if (bin || !THREE_D) load_vgrid_smem(c_vg.e1, c_vg.e2, c_vg.epar, VE1, VE2, VEP);
   // one work item per block, or a persistent grid striding over the items
   for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
   const int t = a.blk_tube[item];
@@ -742,10 +746,10 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
     load_tube_smem(a, t, T, E, Cc);
     tcur = t;
   }
-  if (a.cxc)
+  if (!RUN && a.cxc)
     for (int k = threadIdx.x; k < T.nq; k += blockDim.x) HC[k] = 0u;
   BinWin W{};
-  if (a.bin)
+  if (bin)
     W = bin_win_init(HC + nqmax, a.ion.qind[T.off + beg], T.nq);
   __syncthreads();
   const double ipG = 1.0 / T.pG, invsumds = 1.0 / T.sumdsICR;
@@ -753,12 +757,20 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
   const double c_invOm = T.ms / (T.qs * MDIP);
   for (int64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
     const int64_t j = T.off + i;
-    const int qprev = I.qind[j];
+    int qprev = I.qind[j];
     if (qprev == DEAD) continue;
-    const double rho = I.rho[j], z = I.z[j], vpar = I.vpar[j];
+    double rho = I.rho[j], z = I.z[j], vpar = I.vpar[j];
     double v1 = I.v1[j], v2 = I.v2[j];
     double aea = I.aea[j], ag = I.ag[j];
-    if (a.prologue) field_prologue(a, T, E, Cc, I.qk4[j], qprev, aea, ag);
+    const uint64_t pid = a.icr ? I.id[j] : 0;
+    if (prologue) field_prologue(a, T, E, Cc, I.qk4[j], qprev, aea, ag);
+    // (2D grid, a run: the last speeds inside the grid, as in k_push32)
+    double l_vp = 0.0, l_s = 0.0;
+    bool in_vp = false, in_s = false;
+#pragma unroll 1
+    for (unsigned m = 0;;) {
+    const uint32_t step = step0 + m;
+    const bool last = !RUN || m + 1u == nsub;
     // Vperp^2 without a fused multiply-add: its square root is the 2D grid's
     // binned speed (vperp_mag), the same value on every path
     const double vp2 = __dadd_rn(__dmul_rn(v1, v1), __dmul_rn(v2, v2));
@@ -766,8 +778,14 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
     const Geo<double> g1 = geo(rho, z);
     const int qi = cell_search_from(E, T.nq, T.sgn * g1.q, qprev);
     int b1 = -1, b2 = -1, bp = -1;
-    if (THREE_D) {
-      if (a.bin) {
+    if (RUN && !THREE_D) {
+      if (vpar >= VEP[0] && vpar <= VEP[c_vg.npar]) { l_vp = vpar; in_vp = true; }
+      if (m == 0u || a.icr) {  // (the speed changes only by the kicks)
+        const double sp = sqrt(vp2);
+        if (sp >= VE1[0] && sp <= VE1[c_vg.n1]) { l_s = sp; in_s = true; }
+      }
+    } else if (THREE_D) {
+      if (bin) {
         bp = vbin(VEP, c_vg.npar, vpar);
         b1 = vbin(VE1, c_vg.n1, v1);
         b2 = vbin(VE2, c_vg.n2, v2);
@@ -779,12 +797,12 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
       bp = np_ >= 0 ? np_ : (old & 0xffff) - 1;
       b1 = n1_ >= 0 ? n1_ : (old >> 16) - 1;
       const int nw = ((b1 + 1) << 16) | (bp + 1);
-      if (nw != old && !a.bin_only) I.vb[j] = nw;
+      if (nw != old && !bin_only) I.vb[j] = nw;
     }
-    if (a.bin) accumulate_win(a.acc, T, W, qi, b1, b2, bp, a.exporting);
-    if (a.bin_only) {
+    if (bin) accumulate_win(a.acc, T, W, qi, b1, b2, bp, a.exporting);
+    if (bin_only) {
       if (a.write_qind) I.qind[j] = qi;
-      continue;
+      break;
     }
     const double a1 = apar(g1, vp2, aea, ag, a.ff);
     // wave heating (the mirror force keeps the pre-kick Vperp)
@@ -795,7 +813,7 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
       const double r = 1.0 / g1.ir;
       const double invOm = c_invOm * (r * r * r) * g1.isl;
       const HeatC<double> hc = heat_consts<double>(a.ct, (int64_t)T.coff + qi);
-      heat<double>(a, step, hc, I.id[j], invsumds, Om, invOm, fabs(vpar), v1n, v2n);
+      heat<double>(a, step, hc, pid, invsumds, Om, invOm, fabs(vpar), v1n, v2n);
     }
     // ---- k2: half step along V_R (KineticUpdateB) -----------------------
     const double VRr = vpar * g1.er, VRz = vpar * g1.ez;
@@ -805,7 +823,7 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
     const double A1r = a1 * g1.er, A1z = a1 * g1.ez;
     const Geo<double> g4 = geo(rho + h * VRr + hsq2 * A1r, z + h * VRz + hsq2 * A1z);
     const double a4 = apar(g4, vp2, aea, ag, a.ff);
-    if (a.write_qk4) {
+    if (last && a.write_qk4) {
       I.qk4[j] = g4.q;
       if (I.rho4) {  // KineticUpdateC stores the k4 geometry for collisions
         I.rho4[j] = rho + h * VRr + hsq2 * A1r;
@@ -836,6 +854,17 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
     // ---- V|| along the new field direction ------------------------------
     const double isl = rsqrt(1.0 + 3.0 * ctn * ctn);
     const double vparN = (3.0 * ctn * st * isl) * VNr + ((3.0 * ctn * ctn - 1.0) * isl) * VNz;
+    if (RUN && !last) {
+      rho = rhoN;
+      z = zN;
+      vpar = vparN;
+      v1 = v1n;
+      v2 = v2n;
+      qprev = qi;
+      ++m;
+      continue;
+    }
+    // (in a run a value that is not finite stays so to its end)
     if (!isfinite(vparN) || !isfinite(zN)) atomicOr(a.status, ST_NAN);
     I.rho[j] = rhoN;
     I.z[j] = zN;
@@ -844,15 +873,24 @@ __global__ void __launch_bounds__(256, 2) k_push64(PushArgs a) {
       I.v1[j] = v1n;
       I.v2[j] = v2n;
     }
-    if (a.prologue) {
+    if (prologue) {
       I.aea[j] = aea;
       I.ag[j] = ag;
     }
     if (a.write_qind) I.qind[j] = qi;
-    if (a.cxc && qi >= 0) atomicAdd(&HC[qi], 1u);
+    if (!RUN && a.cxc && qi >= 0) atomicAdd(&HC[qi], 1u);
+    if (RUN && !THREE_D) {
+      const int old = I.vb[j];
+      bp = in_vp ? vbin(VEP, c_vg.npar, l_vp) : (old & 0xffff) - 1;
+      b1 = in_s ? vbin(VE1, c_vg.n1, l_s) : (old >> 16) - 1;
+      const int nw = ((b1 + 1) << 16) | (bp + 1);
+      if (nw != old) I.vb[j] = nw;
+    }
+    break;
+    }  // steps of the run
   }
-  if (a.bin) bin_win_flush(a.acc, T, W);
-  if (a.cxc) flush_cx_counts(a, t, beg, T.nq, HC);
+  if (bin) bin_win_flush(a.acc, T, W);
+  if (!RUN && a.cxc) flush_cx_counts(a, t, beg, T.nq, HC);
   if (!PERSIST) break;  // one item per block: no loop-carried state
   }  // work items
 }
