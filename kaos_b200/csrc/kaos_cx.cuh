@@ -15,7 +15,7 @@
 // parallel selection of the first owed ions per cell in each listed chunk,
 // equal to a walk in index order.
 #pragma once
-#include "kaos_push.cuh"
+#include "kaos_tube.cuh"
 
 namespace kaos {
 
@@ -636,67 +636,58 @@ __global__ void __launch_bounds__(256, 3) k_push_ena(EnaArgs a) {
 // marginals (ZerothENAMoment .. SecondPHIENAMoment _8_10_1 .. _8_10_8 with
 // NonUniform3DIntegratorSub _8_9): integrands hVp hVq hVphi F (.) at the
 // bin centres, M1 = MM/M0, M2 = 6.242e18 (ms/2) MM/M0 centred on M1.  One
-// warp per cell.
+// warp per cell, as k_cell_moments.
 __global__ void __launch_bounds__(256) k_ena_moments(const TubeD *tubes,
                                                      const int *cell_tube,
                                                      CellTables c, Accum acc) {
-  const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  __shared__ BinCentres C;  // par: Vq, v1: Vp, v2: Vphi
+  load_centres(C, c_evg);
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const int64_t NC = c.ncell_total;
-  if (g >= NC) return;  // whole warp
-  const TubeD &T = tubes[cell_tube[g]];
-  const double ms = T.ms;
-  const double w = T.nsnormfac / c.d3xC[g];
-  const double NqENA = (double)acc.ecnt[g] * w;
-  const unsigned *mp = acc.emp + g * MAXV, *mq = acc.emq + g * MAXV,
-                 *mph = acc.emph + g * MAXV;
   const int np = c_evg.n1, nq = c_evg.npar, nph = c_evg.n2;
-  auto centre = [](const double *e, int k) { return 0.5 * (e[k] + e[k + 1]); };
-  double N = 0.0, Sp = 0.0, Sq = 0.0, Sph = 0.0;
-  for (int k = lane; k < np; k += 32) {
-    N += (double)mp[k];
-    Sp += w * centre(c_evg.e1, k) * (double)mp[k];
-  }
-  for (int k = lane; k < nq; k += 32) Sq += w * centre(c_evg.epar, k) * (double)mq[k];
-  for (int k = lane; k < nph; k += 32) Sph += w * centre(c_evg.e2, k) * (double)mph[k];
-  N = warp_sum(N);
-  Sp = warp_sum(Sp);
-  Sq = warp_sum(Sq);
-  Sph = warp_sum(Sph);
-  const double M0 = (NqENA == 0.0) ? 0.0 : w * N;
-  double m1p = 0.0, m1q = 0.0, m1ph = 0.0, tp = 0.0, tq = 0.0, tph = 0.0;
-  if (M0 != 0.0) {
-    m1p = Sp / M0;
-    m1q = Sq / M0;
-    m1ph = Sph / M0;
-    for (int k = lane; k < np; k += 32) {
-      const double d = m1p - centre(c_evg.e1, k);
-      tp += w * fabs(d * d) * (double)mp[k];
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < NC; g += nw) {
+    const unsigned ne = acc.ecnt[g];
+    double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // the rows KAOS_ENA_NQ ..
+    if (ne) {
+      const TubeD &T = tubes[cell_tube[g]];
+      const double ms = T.ms, w = T.nsnormfac / c.d3xC[g];
+      M[0] = (double)ne * w;
+      unsigned mp[VLANE], mq[VLANE], mph[VLANE], n = 0;
+      lane_counts(mp, acc.emp + g * MAXV, np, lane);
+      lane_counts(mq, acc.emq + g * MAXV, nq, lane);
+      lane_counts(mph, acc.emph + g * MAXV, nph, lane);
+      double S[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int i = 0; i < VLANE; ++i) {
+        const int k = lane + 32 * i;
+        n += mp[i];
+        if (k < np) S[0] += w * C.v1[k] * (double)mp[i];
+        if (k < nq) S[1] += w * C.par[k] * (double)mq[i];
+        if (k < nph) S[2] += w * C.v2[k] * (double)mph[i];
+      }
+      const double M0 = M[0] == 0.0 ? 0.0 : w * (double)__reduce_add_sync(0xffffffffu, n);
+      M[1] = M0;
+      if (M0 != 0.0) {
+        warp_sums(S);
+        for (int k = 0; k < 3; ++k) M[2 + k] = S[k] / M0;
+        double Q[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < VLANE; ++i) {
+          const int k = lane + 32 * i;
+          if (k < np) { const double d = M[2] - C.v1[k]; Q[0] += w * fabs(d * d) * (double)mp[i]; }
+          if (k < nq) { const double d = M[3] - C.par[k]; Q[1] += w * fabs(d * d) * (double)mq[i]; }
+          if (k < nph) { const double d = M[4] - C.v2[k]; Q[2] += w * fabs(d * d) * (double)mph[i]; }
+        }
+        warp_sums(Q);
+        const double f = 6.242e18 * (ms / 2.0) / M0;
+        M[5] = (Q[0] + Q[1] + Q[2]) * f;
+        for (int k = 0; k < 3; ++k) M[6 + k] = Q[k] * f;
+      }
     }
-    for (int k = lane; k < nq; k += 32) {
-      const double d = m1q - centre(c_evg.epar, k);
-      tq += w * fabs(d * d) * (double)mq[k];
-    }
-    for (int k = lane; k < nph; k += 32) {
-      const double d = m1ph - centre(c_evg.e2, k);
-      tph += w * fabs(d * d) * (double)mph[k];
-    }
-    tp = warp_sum(tp);
-    tq = warp_sum(tq);
-    tph = warp_sum(tph);
-  }
-  if (lane == 0) {
-    const double eV = 6.242e18, f = M0 != 0.0 ? eV * (ms / 2.0) / M0 : 0.0;
-    double *mom = c.mom;
-    mom[KAOS_ENA_NQ * NC + g] = NqENA;
-    mom[KAOS_ENA_M0 * NC + g] = M0;
-    mom[KAOS_ENA_M1P * NC + g] = m1p;
-    mom[KAOS_ENA_M1Q * NC + g] = m1q;
-    mom[KAOS_ENA_M1PHI * NC + g] = m1ph;
-    mom[KAOS_ENA_M2 * NC + g] = (tp + tq + tph) * f;
-    mom[KAOS_ENA_M2P * NC + g] = tp * f;
-    mom[KAOS_ENA_M2Q * NC + g] = tq * f;
-    mom[KAOS_ENA_M2PHI * NC + g] = tph * f;
+    const double v = lane_value(M, lane);
+    if (lane < 9) c.mom[(KAOS_ENA_NQ + lane) * NC + g] = v;
   }
 }
 

@@ -140,208 +140,173 @@ __global__ void k_fields(TubeArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// Moments of one cell from its count and per-axis binning marginals
+// (ZerothIonMoment .. SecondParIonMoment _8_6_1-_8_6_6 with the
+// NonUniform2D/3D integrators _8_5_*): every integrand there is a sum of
+// single-axis terms at the bin centres, so the marginals carry all the
+// information.  One warp per cell, lanes over the bins; a lane's counts (at
+// most MAXV / 32 per axis) are loaded once, the sums of the axes run side by
+// side, and the bin centres come from shared memory.  (Latency bound: read
+// twice from global memory with the edges in constant memory, whose lanes'
+// different addresses serialise, 73k cells took 223 us, now 103.)
+struct BinCentres {
+  double par[MAXV], v1[MAXV], v2[MAXV];
+};
+// All threads of the block; the caller synchronises.
+__device__ __forceinline__ void load_centres(BinCentres &C, const VGridC &vg) {
+  for (int k = threadIdx.x; k < MAXV; k += blockDim.x) {
+    if (k < vg.npar) C.par[k] = 0.5 * (vg.epar[k] + vg.epar[k + 1]);
+    if (k < vg.n1) C.v1[k] = 0.5 * (vg.e1[k] + vg.e1[k + 1]);
+    if (k < vg.n2) C.v2[k] = 0.5 * (vg.e2[k] + vg.e2[k + 1]);
+  }
+}
+
+constexpr int VLANE = MAXV / 32;  // bins per lane and axis
+
+// This lane's counts of one axis.
+__device__ __forceinline__ void lane_counts(unsigned m[VLANE], const unsigned *src, int n,
+                                            int lane) {
+#pragma unroll
+  for (int i = 0; i < VLANE; ++i) {
+    const int k = lane + 32 * i;
+    m[i] = k < n ? src[k] : 0u;
+  }
+}
 // The one occupied bin of a marginal (all the cell's ions share it), or -1.
 // A cell whose ions share one bin of an axis has that bin's centre as its
 // first moment along the axis (the exact value of the ratio of sums), so the
 // centred second-moment integrand of that bin is zero and falls back to the
 // uncentred one (_8_6_6_SecondParIonMoment.f90:90-99) on every path.
-__device__ __forceinline__ int warp_single_bin(const unsigned *m, int n) {
+__device__ __forceinline__ int warp_single_bin(const unsigned m[VLANE], int lane) {
   int nz = 0, last = -1;
-  for (int k = threadIdx.x & 31; k < n; k += 32)
-    if (m[k]) { ++nz; last = k; }
+#pragma unroll
+  for (int i = 0; i < VLANE; ++i)
+    if (m[i]) { ++nz; last = lane + 32 * i; }
+  nz = __reduce_add_sync(0xffffffffu, nz);
+  last = __reduce_max_sync(0xffffffffu, last);
+  return nz == 1 ? last : -1;
+}
+template <int N>
+__device__ __forceinline__ void warp_sums(double (&x)[N]) {
   for (int o = 16; o > 0; o >>= 1) {
-    nz += __shfl_xor_sync(0xffffffffu, nz, o);
-    last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
+#pragma unroll
+    for (int k = 0; k < N; ++k) x[k] += __shfl_xor_sync(0xffffffffu, x[k], o);
   }
-  return nz == 1 ? last : -1;
 }
 
-__device__ __forceinline__ int single_bin(const unsigned *m, int n) {
-  int nz = 0, last = -1;
-  for (int k = 0; k < n; ++k)
-    if (m[k]) { ++nz; last = k; }
-  return nz == 1 ? last : -1;
-}
-
-// Moments of one cell from its count and binning marginals, for the
-// allocation-free statistics entry point (ZerothIonMoment
-// .. SecondParIonMoment _8_6_1-_8_6_6 with the NonUniform2D/3D integrators
-// _8_5_*): every integrand there is a sum of single-axis terms at the bin
-// centres, so the per-axis marginal counts carry all the information.
-// M[] is indexed by the KAOS_M* selectors 0..9.
-__device__ void cell_moments(double w, double cnt, const unsigned *mp,
-                             const unsigned *m1, const unsigned *m2,
-                             const double *epar, const double *e1,
-                             const double *e2, int npar, int n1, int n2,
-                             int three_d, int cenpar, int cenperp, double ms,
-                             double M[10]) {
+// M[] is indexed by the KAOS_M* selectors 0..9; every lane gets it.
+__device__ __forceinline__ void warp_cell_moments(const BinCentres &C, const unsigned *mp_,
+                                                  const unsigned *m1_, const unsigned *m2_,
+                                                  int npar, int n1, int n2, double w,
+                                                  double NqRT, int three_d, int cenpar,
+                                                  int cenperp, double ms, double M[10]) {
+  const int lane = threadIdx.x & 31;
   for (int k = 0; k < 10; ++k) M[k] = 0.0;
-  const double NqRT = cnt * w;
-  double Nin = 0.0;
-  for (int k = 0; k < npar; ++k) Nin += (double)mp[k];
+  unsigned mp[VLANE], m1[VLANE], m2[VLANE];
+  lane_counts(mp, mp_, npar, lane);
+  lane_counts(m1, m1_, n1, lane);
+  lane_counts(m2, m2_, three_d ? n2 : 0, lane);
+  unsigned nin = 0;
+  double S[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < VLANE; ++i) {
+    const int k = lane + 32 * i;
+    nin += mp[i];
+    if (k < npar) S[0] += C.par[k] * (double)mp[i];
+    if (k < n1) S[1] += C.v1[k] * (double)m1[i];
+    if (three_d && k < n2) S[2] += C.v2[k] * (double)m2[i];
+  }
+  const double Nin = (double)__reduce_add_sync(0xffffffffu, nin);
   if (NqRT == 0.0 || Nin == 0.0) return;
+  warp_sums(S);
+  const int kp = warp_single_bin(mp, lane), k1 = warp_single_bin(m1, lane),
+            k2 = warp_single_bin(m2, lane);
   const double M0 = w * Nin;
-  double Sp = 0.0, S1 = 0.0;
-  for (int k = 0; k < npar; ++k) Sp += 0.5 * (epar[k] + epar[k + 1]) * mp[k];
-  for (int k = 0; k < n1; ++k) S1 += 0.5 * (e1[k] + e1[k + 1]) * m1[k];
-  const int kp = single_bin(mp, npar), k1 = single_bin(m1, n1);
-  const double M1par = kp >= 0 ? 0.5 * (epar[kp] + epar[kp + 1]) : (w * Sp) / M0;
-  double Tp = 0.0, Tq = 0.0, T1 = 0.0, T1c = 0.0;
-  // centred integrand; for M2|| a bin whose centred value is exactly zero
-  // falls back to the uncentred one (_8_6_6_SecondParIonMoment.f90:90-99).
-  // The total-energy integrand also carries the Vperp terms, so it is never
-  // zero and keeps the centred value (Tq).
-  for (int k = 0; k < npar; ++k) {
-    if (!mp[k]) continue;
-    const double vc = 0.5 * (epar[k] + epar[k + 1]);
-    const double d = cenpar ? (vc - M1par) : vc;
-    double d2 = d * d;
-    Tq += d2 * mp[k];
-    if (d2 == 0.0) d2 = vc * vc;
-    Tp += d2 * mp[k];
-  }
-  const double M1p1 = k1 >= 0 ? 0.5 * (e1[k1] + e1[k1 + 1]) : (w * S1) / M0;
-  for (int k = 0; k < n1; ++k) {
-    if (!m1[k]) continue;
-    const double vc = 0.5 * (e1[k] + e1[k + 1]);
-    T1 += vc * vc * m1[k];
-    const double d = vc - M1p1;
-    double d2 = d * d;
-    if (d2 == 0.0) d2 = vc * vc;
-    T1c += d2 * m1[k];
-  }
-  M[KAOS_M0] = M0;
-  M[KAOS_M1PAR] = M1par;
-  M[KAOS_M2PAR] = (ms / 2.0) * ((w * Tp) / M0);
-  if (three_d) {
-    double S2 = 0.0, T2 = 0.0, T2c = 0.0;
-    for (int k = 0; k < n2; ++k) S2 += 0.5 * (e2[k] + e2[k + 1]) * m2[k];
-    const int k2 = single_bin(m2, n2);
-    const double M1p2 = k2 >= 0 ? 0.5 * (e2[k2] + e2[k2 + 1]) : (w * S2) / M0;
-    for (int k = 0; k < n2; ++k) {
-      if (!m2[k]) continue;
-      const double vc = 0.5 * (e2[k] + e2[k + 1]);
-      T2 += vc * vc * m2[k];
-      const double d = vc - M1p2;
+  const double M1par = kp >= 0 ? C.par[kp] : (w * S[0]) / M0;
+  const double M1p1 = k1 >= 0 ? C.v1[k1] : (w * S[1]) / M0;
+  const double M1p2 = k2 >= 0 ? C.v2[k2] : (w * S[2]) / M0;
+  // Q: plain or centred squares (Tp falls back to the uncentred value in a
+  // bin whose centred one is zero, _8_6_6_SecondParIonMoment.f90:90-99; the
+  // total-energy integrand also carries the Vperp terms, so it is never zero
+  // and keeps the centred value Tq)
+  double Q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // Tp Tq T1 T1c T2 T2c
+#pragma unroll
+  for (int i = 0; i < VLANE; ++i) {
+    const int k = lane + 32 * i;
+    if (mp[i]) {
+      const double vc = C.par[k], d = cenpar ? (vc - M1par) : vc;
+      double d2 = d * d;
+      Q[1] += d2 * mp[i];
+      if (d2 == 0.0) d2 = vc * vc;
+      Q[0] += d2 * mp[i];
+    }
+    if (m1[i]) {
+      const double vc = C.v1[k], d = vc - M1p1;
+      Q[2] += vc * vc * m1[i];
       double d2 = d * d;
       if (d2 == 0.0) d2 = vc * vc;
-      T2c += d2 * m2[k];
+      Q[3] += d2 * m1[i];
     }
+    if (m2[i]) {
+      const double vc = C.v2[k], d = vc - M1p2;
+      Q[4] += vc * vc * m2[i];
+      double d2 = d * d;
+      if (d2 == 0.0) d2 = vc * vc;
+      Q[5] += d2 * m2[i];
+    }
+  }
+  warp_sums(Q);
+  M[KAOS_M0] = M0;
+  M[KAOS_M1PAR] = M1par;
+  M[KAOS_M2PAR] = (ms / 2.0) * ((w * Q[0]) / M0);
+  if (three_d) {
     M[KAOS_M1PERP1] = M1p1;
     M[KAOS_M1PERP2] = M1p2;
-    M[KAOS_M2] = (ms / 2.0) * ((w * (T1 + T2 + Tq)) / M0);
-    M[KAOS_M2PERP1] = (ms / 2.0) * ((w * (cenperp ? T1c : T1)) / M0);
-    M[KAOS_M2PERP2] = (ms / 2.0) * ((w * (cenperp ? T2c : T2)) / M0);
+    M[KAOS_M2] = (ms / 2.0) * ((w * (Q[2] + Q[4] + Q[1])) / M0);
+    M[KAOS_M2PERP1] = (ms / 2.0) * ((w * (cenperp ? Q[3] : Q[2])) / M0);
+    M[KAOS_M2PERP2] = (ms / 2.0) * ((w * (cenperp ? Q[5] : Q[4])) / M0);
   } else {
     M[KAOS_M1PERP] = M1p1;
-    M[KAOS_M2] = (ms / 2.0) * ((w * (T1 + Tq)) / M0);
-    M[KAOS_M2PERP] = (ms / 2.0) * ((w * (cenperp ? T1c : T1)) / M0);
+    M[KAOS_M2] = (ms / 2.0) * ((w * (Q[2] + Q[1])) / M0);
+    M[KAOS_M2PERP] = (ms / 2.0) * ((w * (cenperp ? Q[3] : Q[2])) / M0);
   }
+}
+// Element `lane` of a warp-uniform array of N values (one store for all).
+template <int N>
+__device__ __forceinline__ double lane_value(const double (&M)[N], int lane) {
+  double v = M[0];
+#pragma unroll
+  for (int k = 1; k < N; ++k) v = lane == k ? M[k] : v;
+  return v;
 }
 
 // ---------------------------------------------------------------------------
-// Moments of one master step from the binning marginals (ZerothIonMoment ..
-// SecondParIonMoment _8_6_1-_8_6_6 with the NonUniform2D/3D integrators
-// _8_5_*): one warp per cell, lanes over the velocity bins.  Every
-// integrand there is a sum of single-axis terms at the bin centres, so the
-// per-axis marginal counts carry all the information.
-__global__ void __launch_bounds__(256) k_cell_moments(TubeArgs a,
-                                                      const int *cell_tube) {
-  const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Moments of one master step, a grid striding over the cells.
+__global__ void __launch_bounds__(256) k_cell_moments(TubeArgs a, const int *cell_tube) {
+  __shared__ BinCentres C;
+  load_centres(C, c_vg);
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const CellTables &c = a.ct;
   const int64_t NC = c.ncell_total;
-  if (g >= NC) return;  // whole warp
-  const TubeD &T = a.tubes[cell_tube[g]];
-  const double ms = T.ms;
   const int n1 = c_vg.n1, n2 = c_vg.n2, npar = c_vg.npar;
-  const double w = T.nsnormfac / c.d3xC[g];
-  const double NqRT = (double)a.acc.cnt[g] * w;
-  const unsigned *mp = a.acc.mpar + g * npar, *m1 = a.acc.m1 + g * n1;
-  const unsigned *m2 = a.three_d ? a.acc.m2 + g * n2 : nullptr;
-  double Nin = 0.0, Sp = 0.0, S1 = 0.0, S2 = 0.0;
-  for (int k = lane; k < npar; k += 32) {
-    const double m = (double)mp[k];
-    Nin += m;
-    Sp += 0.5 * (c_vg.epar[k] + c_vg.epar[k + 1]) * m;
-  }
-  for (int k = lane; k < n1; k += 32) S1 += 0.5 * (c_vg.e1[k] + c_vg.e1[k + 1]) * (double)m1[k];
-  if (m2)
-    for (int k = lane; k < n2; k += 32) S2 += 0.5 * (c_vg.e2[k] + c_vg.e2[k + 1]) * (double)m2[k];
-  Nin = warp_sum(Nin);
-  Sp = warp_sum(Sp);
-  S1 = warp_sum(S1);
-  S2 = warp_sum(S2);
-  // the one occupied bin of each axis, or -1 (see warp_single_bin)
-  const int kp = warp_single_bin(mp, npar), k1 = warp_single_bin(m1, n1);
-  const int k2 = m2 ? warp_single_bin(m2, n2) : -1;
-  double M[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (NqRT != 0.0 && Nin != 0.0) {
-    const double M0 = w * Nin;
-    const double M1par = kp >= 0 ? 0.5 * (c_vg.epar[kp] + c_vg.epar[kp + 1]) : (w * Sp) / M0;
-    const double M1p1 = k1 >= 0 ? 0.5 * (c_vg.e1[k1] + c_vg.e1[k1 + 1]) : (w * S1) / M0;
-    const double M1p2 = k2 >= 0 ? 0.5 * (c_vg.e2[k2] + c_vg.e2[k2 + 1]) : (w * S2) / M0;
-    // centred integrand; for M2|| a bin whose centred value is exactly zero
-    // falls back to the uncentred one (_8_6_6_SecondParIonMoment.f90:90-99).
-    // The total-energy integrand also carries the Vperp terms, so it is
-    // never zero and keeps the centred value (Tq).
-    double Tp = 0.0, Tq = 0.0, T1 = 0.0, T1c = 0.0, T2 = 0.0, T2c = 0.0;
-    for (int k = lane; k < npar; k += 32) {
-      if (!mp[k]) continue;
-      const double vc = 0.5 * (c_vg.epar[k] + c_vg.epar[k + 1]);
-      const double d = a.cenpar ? (vc - M1par) : vc;
-      double d2 = d * d;
-      Tq += d2 * mp[k];
-      if (d2 == 0.0) d2 = vc * vc;
-      Tp += d2 * mp[k];
-    }
-    for (int k = lane; k < n1; k += 32) {
-      if (!m1[k]) continue;
-      const double vc = 0.5 * (c_vg.e1[k] + c_vg.e1[k + 1]);
-      T1 += vc * vc * m1[k];
-      const double d = vc - M1p1;
-      double d2 = d * d;
-      if (d2 == 0.0) d2 = vc * vc;
-      T1c += d2 * m1[k];
-    }
-    if (m2)
-      for (int k = lane; k < n2; k += 32) {
-        if (!m2[k]) continue;
-        const double vc = 0.5 * (c_vg.e2[k] + c_vg.e2[k + 1]);
-        T2 += vc * vc * m2[k];
-        const double d = vc - M1p2;
-        double d2 = d * d;
-        if (d2 == 0.0) d2 = vc * vc;
-        T2c += d2 * m2[k];
-      }
-    Tp = warp_sum(Tp);
-    Tq = warp_sum(Tq);
-    T1 = warp_sum(T1);
-    T1c = warp_sum(T1c);
-    T2 = warp_sum(T2);
-    T2c = warp_sum(T2c);
-    M[KAOS_M0] = M0;
-    M[KAOS_M1PAR] = M1par;
-    M[KAOS_M2PAR] = (ms / 2.0) * ((w * Tp) / M0);
-    if (a.three_d) {
-      M[KAOS_M1PERP1] = M1p1;
-      M[KAOS_M1PERP2] = M1p2;
-      M[KAOS_M2] = (ms / 2.0) * ((w * (T1 + T2 + Tq)) / M0);
-      M[KAOS_M2PERP1] = (ms / 2.0) * ((w * (a.cenperp ? T1c : T1)) / M0);
-      M[KAOS_M2PERP2] = (ms / 2.0) * ((w * (a.cenperp ? T2c : T2)) / M0);
-    } else {
-      M[KAOS_M1PERP] = M1p1;
-      M[KAOS_M2] = (ms / 2.0) * ((w * (T1 + Tq)) / M0);
-      M[KAOS_M2PERP] = (ms / 2.0) * ((w * (a.cenperp ? T1c : T1)) / M0);
-    }
-  }
-  if (lane == 0) {
-    double *mom = c.mom;
-    for (int k = 0; k < 10; ++k) mom[k * NC + g] = M[k];
-    mom[KAOS_NQ * NC + g] = NqRT;
-    c.M0prev[g] = M[KAOS_M0];
-    mom[KAOS_EAMAG * NC + g] = c.EAmag[g];
-    mom[KAOS_EGMAG * NC + g] = c.EG[g];
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < NC; g += nw) {
+    const TubeD &T = a.tubes[cell_tube[g]];
+    const double w = T.nsnormfac / c.d3xC[g];
+    const double NqRT = (double)a.acc.cnt[g] * w;
+    double M[14];
+    warp_cell_moments(C, a.acc.mpar + g * npar, a.acc.m1 + g * n1,
+                      a.three_d ? a.acc.m2 + g * n2 : nullptr, npar, n1, n2, w, NqRT,
+                      a.three_d, a.cenpar, a.cenperp, T.ms, M);
+    M[KAOS_NQ] = NqRT;
+    M[KAOS_EAMAG] = c.EAmag[g];
+    M[KAOS_EGMAG] = c.EG[g];
+    M[13] = M[KAOS_M0];  // M0prev, not a row (KAOS_M0FILT is the field kernel's)
+    static_assert(KAOS_NQ == 10 && KAOS_EAMAG == 11 && KAOS_EGMAG == 12, "row order");
+    const double v = lane_value(M, lane);
+    if (lane < 13) c.mom[lane * NC + g] = v;
+    else if (lane == 13) c.M0prev[g] = v;
   }
 }
 

@@ -83,3 +83,51 @@ def test_noalloc_rejects_oversize_grid():
                                 C.addressof(dummy), None, 1, C.addressof(dummy),
                                 None, None)
     assert rc == 1  # KAOS_ERR_PARAM
+
+
+@pytest.mark.parametrize("nq,n1,n2,npar,n", [
+    (512, 128, 128, 128, 40_000),  # four parts of cells
+    (194, 128, 8, 127, 6_000),     # one cell more than a part holds
+    (193, 127, 128, 9, 1025),      # a part exactly full; one ion over a block
+    (6, 2, 2, 2, 1),               # the smallest tube, one ion
+    (97, 31, 0, 53, 100_003),      # 2D grid, ragged
+])
+def test_noalloc_matches_handle_sizes(nq, n1, n2, npar, n):
+    """Cells and bins around the block-private counters' part sizes, ions
+    outside the velocity grid among them (3D): the counts of the handle path
+    exactly, its moments within 1e-10."""
+    import torch
+    kbuild.build()
+    L = klib.load()
+    d3 = n2 > 0
+    mi = grids.ModelInput(ION2VPERPflag=1 if d3 else 0, MOMENTFILTERflag=0)
+    spec = grids.TubeSpec(L=4.0, nq=nq, n_particles=n, q_ub=0.15, H=600e3)
+    tube = grids.make_tube(spec, mi)
+    tube.capacity = n
+    vmax = 2.5e3 if d3 else 2e4  # (2D: the handle keeps a first bin outside)
+    lin = lambda k, a: np.linspace(a, vmax, k + 1)
+    vg = grids.VGrid(e1=lin(n1, -vmax if d3 else 0.0), e2=lin(n2, -vmax) if d3 else None,
+                     epar=lin(npar, -vmax))
+    rng = np.random.default_rng(nq)
+    q = rng.uniform(tube.qGH[-1], tube.qGL[0], n)
+    v = rng.normal(size=(3, n)) * 1.3e3
+    s = klib.Solver(mi, [tube], vg)
+    s.load(0, q, *v)
+    s.step(1)
+    ref, ref_counts = s.moments_all()[:KAOS_NQ + 1].copy(), s.counts()
+    s.close()
+    t = lambda a: torch.as_tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")
+    arr = [t(np.append(tube.qGL, tube.qGH[-1])), t(tube.d3xC), t(q), t(v[0]), t(v[1]), t(v[2])]
+    out = torch.full((KAOS_NQ + 1, nq), -1.0, dtype=torch.float64, device="cuda")
+    cnt = torch.full((nq,), -1, dtype=torch.int64, device="cuda")
+    pc, vgc = mi.to_c(), vg.to_c()
+    ptr = [a.data_ptr() for a in arr]
+    rc = L.kaos_moments_noalloc(C.addressof(pc), C.addressof(vgc), nq, ptr[0], ptr[1],
+                                tube.nsnormfac, *ptr[2:], n, out.data_ptr(), cnt.data_ptr(), None)
+    assert rc == 0
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(cnt.cpu().numpy(), ref_counts)
+    got = out.cpu().numpy()
+    for k in range(KAOS_NQ + 1):
+        scale = max(np.max(np.abs(ref[k])), 1e-300)
+        assert np.max(np.abs(got[k] - ref[k])) / scale <= MOM_TOL, k
