@@ -374,8 +374,7 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
   }
   if (timed) CK(cudaEventRecord(h->pev[2 * h->npev], h->s));
   size_t smem = (size_t)(2 * nq + 1) * sizeof(double) + (size_t)nq * sizeof(unsigned);
-  if (h->mixed)  // + one double of padding before the 16-byte aligned floats
-    smem += (size_t)(6 * nq + 1) * sizeof(double) + (size_t)10 * nq * sizeof(float);
+  if (h->mixed) smem += (size_t)nq * (sizeof(CellS) + sizeof(float2));
   smem += (size_t)BIN_WIN * (1 + h->vg.npar + h->vg.n1 + (h->three_d ? h->vg.n2 : 0)) *
           sizeof(unsigned);  // block-private binning window
   const bool bins_variant = a.bin || a.prologue || a.bin_only || !h->three_d;

@@ -935,6 +935,17 @@ __device__ __forceinline__ void start_bins(const PushArgs &a, const Ions &I,
   }
 }
 
+// What the mixed push reads of an ion's cell, in shared memory: one record of
+// 16-byte loads from one address (the arrays per quantity it replaces took a
+// load and an address each; 80 bytes a record keeps neighbouring cells'
+// loads on different banks).
+struct __align__(16) CellS {
+  double ql, dq;   // lower edge, width in q
+  double ul, ud;   // quadratic guess of the quartic root: uL, uH - uL
+  double uc, idq;  // ... its curvature term; 1 / dq
+  float hk[8];     // heat32's constants
+};
+
 // ---------------------------------------------------------------------------
 // Mixed kernel: FP32 arithmetic on FP64 state.  The position is one FP64
 // cell coordinate x = cell + offset in q within the cell; V|| and the Vperp
@@ -975,13 +986,10 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
              bin_only = MASTER && a.bin_only;
   extern __shared__ __align__(16) double sm[];
   const int nqmax = a.nqs;
-  double *E = sm, *Cc = sm + nqmax + 1;
-  double *UL = Cc + nqmax, *UD = UL + nqmax, *UC = UD + nqmax, *QL = UC + nqmax,
-         *IDQ = QL + nqmax, *DQ = IDQ + nqmax;
-  // 8 floats per cell (heat32), 16-byte aligned; then the cell fields
-  // (EAmag, EG) of the field re-interpolation
-  float *HK = (float *)(sm + ((8 * nqmax + 2) & ~1));
-  float2 *FE = (float2 *)(HK + 8 * nqmax);
+  CellS *CS = (CellS *)sm;
+  double *E = (double *)(CS + nqmax), *Cc = E + nqmax + 1;
+  // the cell fields (EAmag, EG) of the field re-interpolation
+  float2 *FE = (float2 *)(Cc + nqmax);
   unsigned *HC = (unsigned *)(FE + nqmax);
   const float h = (float)a.h, hh = 0.5f * h, h6 = h / 6.0f, hsq2 = 0.5f * h * h;
   const float hh6 = h * h6;
@@ -1029,23 +1037,24 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     for (int k = threadIdx.x; k < T.nq; k += blockDim.x) {
       const int64_t g = T.coff + k;
       const double ql = a.ct.qGL[g], qh = a.ct.qGH[g];
-      QL[k] = ql;
-      DQ[k] = qh - ql;
-      IDQ[k] = 1.0 / (qh - ql);
-      UL[k] = a.ct.uL[g];
-      UD[k] = a.ct.uH[g] - a.ct.uL[g];
+      CellS &C = CS[k];
+      C.ql = ql;
+      C.dq = qh - ql;
+      C.idq = 1.0 / (qh - ql);
+      C.ul = a.ct.uL[g];
+      C.ud = a.ct.uH[g] - a.ct.uL[g];
       // quadratic in the offset through the edges and the midpoint
-      UC[k] = 4.0 * a.ct.uM[g] - 2.0 * (a.ct.uL[g] + a.ct.uH[g]);
+      C.uc = 4.0 * a.ct.uM[g] - 2.0 * (a.ct.uL[g] + a.ct.uH[g]);
       if (a.icr) {
         const double lam = a.ct.lambdaPerp[g];
-        HK[8 * k + 0] = (float)a.ct.hK1[g];
-        HK[8 * k + 1] = (float)a.ct.hK2[g];
-        HK[8 * k + 2] = (float)a.ct.hc1[g];
-        HK[8 * k + 3] = (float)a.ct.hc2[g];
-        HK[8 * k + 4] = a.icrcoh ? (float)a.ct.hiom0[g] : lg2f((float)a.ct.hiom0[g]);
-        HK[8 * k + 5] = (float)lam;
-        HK[8 * k + 6] = lam != 0.0 ? (float)log2(2.0 * PI / lam) : 0.0f;
-        HK[8 * k + 7] = 0.0f;
+        C.hk[0] = (float)a.ct.hK1[g];
+        C.hk[1] = (float)a.ct.hK2[g];
+        C.hk[2] = (float)a.ct.hc1[g];
+        C.hk[3] = (float)a.ct.hc2[g];
+        C.hk[4] = a.icrcoh ? (float)a.ct.hiom0[g] : lg2f((float)a.ct.hiom0[g]);
+        C.hk[5] = (float)lam;
+        C.hk[6] = lam != 0.0 ? (float)log2(2.0 * PI / lam) : 0.0f;
+        C.hk[7] = 0.0f;
       }
       if (prologue) FE[k] = make_float2((float)a.ct.EAmag[g], (float)a.ct.EG[g]);
     }
@@ -1134,10 +1143,12 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     const double o0 = x0 - c0d;  // exact
     if (prologue) field_prologue32(a.ff, T, E, Cc, FE, qk0, c0, qs_ms, aea, ag);
     // ---- start-of-step position: q, then (r, theta) by FP64 Newton -------
-    const double q0 = fma(o0, DQ[c0], QL[c0]);
+    const double2 cq = *(const double2 *)&CS[c0].ql, cu = *(const double2 *)&CS[c0].ul,
+                  cc = *(const double2 *)&CS[c0].uc;
+    const double q0 = fma(o0, cq.y, cq.x);
     // per-cell quadratic guess u(o) = uL + o (uH - uL) + o (1 - o) UC
     const double u = quartic_newton_chord(
-        q0, ipG, fma(o0, fma(1.0 - o0, UC[c0], UD[c0]), UL[c0]));
+        q0, ipG, fma(o0, fma(1.0 - o0, cc.x, cu.y), cu.x));
     const double s2 = u * ipG;  // sin^2(theta)
     // sqrt(s2): FP32 seed and one FP64 Newton step (relative error ~1e-14)
     const float s2f = (float)s2;
@@ -1195,7 +1206,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       const float sl = g1.ell * g1.isl;
       const float ir3 = g1.ir * g1.ir * g1.ir;
       const float Om = qs_ms * (float)MDIP * sl * ir3;
-      const float *hk = HK + 8 * qi;
+      const float *hk = CS[qi].hk;
       if (!a.icrcoh) {
         float dv1, dv2;
         heat32(a, step, hk, pid, invsumds, ylim, Om, fabsf(vparf), vp2, dv1, dv2);
@@ -1256,9 +1267,14 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     // and an offset strictly inside (0, 1) there decides it without the
     // edge search; escaped ions keep the end cell and an offset outside
     const int cs = qi >= 0 ? qi : c0;
+    double cql = cq.x, cidq = cc.y;
+    if (cs != c0) {
+      cql = CS[cs].ql;
+      cidq = CS[cs].idq;
+    }
     // (the product rounded on its own on every path: no fused multiply-add
     // with the cell number)
-    double od = __dmul_rn(qN - QL[cs], IDQ[cs]);
+    double od = __dmul_rn(qN - cql, cidq);
     double xN;
     if (od > 1e-9 && od < 1.0 - 1e-9) {
       // (a run: qi = c0 has been the cell of x0 all along unless the start
@@ -1272,7 +1288,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     } else {
       const int cN = cell_search_from(E, T.nq, T.sgn * qN, cs);
       const int cpos = cN >= 0 ? cN : (cN == BELOW ? 0 : T.nq - 1);
-      od = __dmul_rn(qN - QL[cpos], IDQ[cpos]);
+      od = __dmul_rn(qN - CS[cpos].ql, CS[cpos].idq);
       xN = (double)cpos + od;
       if (RUN) {  // the cell as the next step reads it from the coordinate
         c0 = x_cell(xN, T.nq);
