@@ -90,6 +90,7 @@ struct kaos_handle {
   int ntubes = 0;
   int mixed = 0;
   int kick64 = 0;  // mixed push with the FP64 heating kick
+  int heat_lam = 0, heat_chi = 0;  // PushArgs: seen in any tube's tables so far
   int three_d = 1;
   int nv = 0;
   int64_t ncell = 0;
@@ -276,7 +277,7 @@ int max_nq(const kaos_handle *h) {
   return m;
 }
 
-// Ions per work item of a run of steps (256-thread blocks, 3 per SM): one
+// Ions per work item of a run of steps (256-thread blocks, 4 per SM): one
 // ion per thread while that is what it takes to fill the SMs, four once there
 // are several waves of blocks, which then build their tube's tables a quarter
 // as often.  The 19-step runs of a master interval, us per interval: 1e6 ions
@@ -286,6 +287,14 @@ int run_chunk(const kaos_handle *h) {
   int64_t cap = 0;
   for (const TubeD &T : h->th) cap += T.cap;
   return cap < (int64_t)1 << 21 ? 256 : 1024;
+}
+
+// What the heating tables of a tube ask of the kick (PushArgs).
+void note_heating(kaos_handle *h, const kaos_tube_c &T) {
+  for (int k = 0; k < T.nq; ++k) {
+    if (T.lambdaPerp && T.lambdaPerp[k] != 0.0) h->heat_lam = 1;
+    if ((T.ChiPerp1 ? T.ChiPerp1[k] : 0.0) != (T.ChiPerp2 ? T.ChiPerp2[k] : 0.0)) h->heat_chi = 1;
+  }
 }
 
 PushArgs push_args(kaos_handle *h, bool run = false) {
@@ -311,6 +320,8 @@ PushArgs push_args(kaos_handle *h, bool run = false) {
   a.ff.eambsign = h->P.EAMBSIGNflag == 1;
   a.icr = h->P.ICRflag == 1;
   a.icrcoh = h->P.ICRCOHERENCEflag == 1;
+  a.heat_lam = h->heat_lam;
+  a.heat_chi = h->heat_chi;
   a.status = h->d_status;
   a.exporting = h->export_on;
   a.cxc = nullptr;  // set by the pushes whose Qindk1 feeds a selection
@@ -375,7 +386,9 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
   if (timed) CK(cudaEventRecord(h->pev[2 * h->npev], h->s));
   size_t smem = (size_t)(2 * nq + 1) * sizeof(double) + (size_t)nq * sizeof(unsigned);
   if (h->mixed) smem += (size_t)nq * (sizeof(CellS) + sizeof(float2));
-  smem += (size_t)BIN_WIN * (1 + h->vg.npar + h->vg.n1 + (h->three_d ? h->vg.n2 : 0)) *
+  if (h->mixed && a.nsub > 1)  // a run: cell records and edges
+    smem = (size_t)nq * sizeof(CellS) + (size_t)(nq + 1) * sizeof(double);
+  else smem += (size_t)BIN_WIN * (1 + h->vg.npar + h->vg.n1 + (h->three_d ? h->vg.n2 : 0)) *
           sizeof(unsigned);  // block-private binning window
   const bool bins_variant = a.bin || a.prologue || a.bin_only || !h->three_d;
   if (h->mixed && bins_variant) smem += BINS_SMEM_BYTES;  // FP64 edges + tables
@@ -406,14 +419,16 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
   // build (16 warps) spills nothing and is 5 % slower on 1e7 ions, 13 % on 1e5
   static const KFn k64run[2] = {k_push64<false, 256, 3, false, true>,
                                 k_push64<true, 256, 3, false, true>};
-  // runs of steps: [FP64 heating kick][three_d]; 256 threads x 3 blocks per
-  // SM (64-register and 128-thread builds measured the same within 2 % on
-  // 1e7 ions, the latter 20 % slower on batches of uneven tubes)
+  // runs of steps: [FP64 heating kick][three_d].  64 registers (32 warps per
+  // SM; 8 B of spills, 100 B with the FP64 kick) against 79 (24 warps, 0 and
+  // 28 B), ms per 20 steps: 1e7 ions 2.78 / 2.81, FP64 kick 4.30 / 4.33, 1e8
+  // ions 26.6 / 27.0, 256 uneven tubes 15.16 / 15.40; 128-thread blocks are
+  // up to 30 % slower on the uneven tubes (twice the table set-ups)
   static const KFn k32run[2][2] = {
-      {k_push32<false, 256, 3, false, false, false, true>,
-       k_push32<true, 256, 3, false, false, false, true>},
-      {k_push32<false, 256, 3, false, false, true, true>,
-       k_push32<true, 256, 3, false, false, true, true>}};
+      {k_push32<false, 256, 4, false, false, false, true>,
+       k_push32<true, 256, 4, false, false, false, true>},
+      {k_push32<false, 256, 4, false, false, true, true>,
+       k_push32<true, 256, 4, false, false, true, true>}};
   const KFn fn = run ? (h->mixed ? k32run[h->kick64][h->three_d] : k64run[h->three_d])
                      : (h->mixed ? k32[h->kick64][ms][h->three_d][rs][ps] : k64[h->three_d][ps]);
   if (smem > 48 * 1024)
@@ -1364,6 +1379,7 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
     host_rho_z(T.qGC[0], T.pG, &d.rhoLB, &d.zLB);
     host_rho_z(T.qGC[T.nq - 1], T.pG, &d.rhoUB, &d.zUB);
     h->th.push_back(d);
+    note_heating(h, T);
     auto app = [&](std::vector<double> &v, const double *src, double dflt) {
       for (int k = 0; k < T.nq; ++k) v.push_back(src ? src[k] : dflt);
     };
@@ -1484,7 +1500,8 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
   };
   for (int m = 0; m < NCHUNKS; ++m)
     if ((rc = work_map(h->wmap[m], CHUNKS[m]))) return rc;
-  if ((rc = work_map(h->rmap, run_chunk(h)))) return rc;
+  h->rmap = h->wmap[0];
+  if (h->rmap.chunk != run_chunk(h) && (rc = work_map(h->rmap, run_chunk(h)))) return rc;
   if ((rc = dalloc(h, &h->d_nlive, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_nlive_new, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_next_id, ntubes))) return rc;
@@ -1824,6 +1841,7 @@ int kaos_update_tube(kaos_handle *h, int32_t tube, const kaos_tube_c *T) {
   host_rho_z(T->qGC[0], T->pG, &pt.d.rhoLB, &pt.d.zLB);
   host_rho_z(T->qGC[T->nq - 1], T->pG, &pt.d.rhoUB, &pt.d.zUB);
   pt.tables = tube_tables(*T, pt.d, h->P);
+  note_heating(h, *T);
   for (auto &q : h->pending)
     if (q.tube == tube) {
       q = std::move(pt);

@@ -33,6 +33,9 @@ struct PushArgs {
   uint32_t step;
   ForceFlags ff;
   int icr, icrcoh;
+  // whether any cell of any tube has lambdaPerp != 0 / ChiPerp1 != ChiPerp2
+  // (uniform: the mixed kick skips what no cell needs)
+  int heat_lam, heat_chi;
   int bin;        // accumulate start-of-step counts (master step)
   int prologue;   // re-interpolate the cached fields at qk4 first
   int write_qind; // store Qindk1 (needed by the next boundary/collision pass)
@@ -529,13 +532,13 @@ __device__ __forceinline__ void heat32(const PushArgs &a, uint32_t step,
   const float4 h0 = *(const float4 *)hk, h1 = *(const float4 *)(hk + 4);
   const float LOm = lg2f(Om);
   float b = 0.25f * lg2f(y);
-  if (h1.y != 0.0f) {  // lambda != 0
+  if (a.heat_lam && h1.y != 0.0f) {  // lambda != 0
     const float ls = fmaf(0.5f, lg2f(vp2), h1.z) - LOm;
     if (ls >= 0.0f) b -= 1.5f * ls;
   }
   const float lx = LOm + h1.x;
   const float e1 = ex2f(fmaf(-h0.z, lx, b));
-  const float e2 = (h0.w == h0.z) ? e1 : ex2f(fmaf(-h0.w, lx, b));
+  const float e2 = (!a.heat_chi || h0.w == h0.z) ? e1 : ex2f(fmaf(-h0.w, lx, b));
   float G1, G2;
   gauss2_mix(a.rk, id, step, G1, G2);
   dv1 = h0.x * e1 * G1;
@@ -691,13 +694,13 @@ __device__ __forceinline__ void load_vgrid_smem(const T *e1, const T *e2,
 // Load this block's tube and its oriented cell edges / centres into smem.
 __device__ __forceinline__ void load_tube_smem(const PushArgs &a, int t,
                                                TubeD &T, double *E,
-                                               double *Cc) {
+                                               double *Cc, bool centres = true) {
   T = a.tubes[t];
   const double *qGL = a.ct.qGL + T.coff, *qGH = a.ct.qGH + T.coff,
                *qGC = a.ct.qGC + T.coff;
   for (int k = threadIdx.x; k <= T.nq; k += blockDim.x) {
     E[k] = (k < T.nq) ? T.sgn * qGL[k] : T.sgn * qGH[T.nq - 1];
-    if (k < T.nq) Cc[k] = T.sgn * qGC[k];
+    if (centres && k < T.nq) Cc[k] = T.sgn * qGC[k];
   }
 }
 
@@ -935,6 +938,13 @@ __device__ __forceinline__ void start_bins(const PushArgs &a, const Ions &I,
   }
 }
 
+// Whether an offset lies in (2^-29, 1 - 2^-21), well inside (0, 1): its cell
+// then needs no edge search (the FP64 rounding of an offset is far below the
+// margins).  One integer comparison of the high word.
+__device__ __forceinline__ bool well_inside(double o) {
+  return (unsigned)(__double2hiint(o) - 0x3e200000) < 0x3fefffffu - 0x3e200000u;
+}
+
 // What the mixed push reads of an ion's cell, in shared memory: one record of
 // 16-byte loads from one address (the arrays per quantity it replaces took a
 // load and an address each; 80 bytes a record keeps neighbouring cells'
@@ -988,12 +998,13 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   const int nqmax = a.nqs;
   CellS *CS = (CellS *)sm;
   double *E = (double *)(CS + nqmax), *Cc = E + nqmax + 1;
-  // the cell fields (EAmag, EG) of the field re-interpolation
+  // the cell fields (EAmag, EG) of the field re-interpolation; the selection
+  // counts (runs hold neither these nor the cell centres)
   float2 *FE = (float2 *)(Cc + nqmax);
   unsigned *HC = (unsigned *)(FE + nqmax);
   const float h = (float)a.h, hh = 0.5f * h, h6 = h / 6.0f, hsq2 = 0.5f * h * h;
   const float hh6 = h * h6;
-  const double hd = a.h;
+  const double hd = a.h, hmre = -a.h / RE;
   const uint32_t step0 = a.dstep ? *a.dstep : a.step;
   const unsigned nsub = RUN ? a.nsub : 1u;
   if (a.dstep_w && blockIdx.x == 0 && threadIdx.x == 0) *a.dstep_w = step0 + nsub - 1u;
@@ -1009,9 +1020,8 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   // (offset arithmetic from the shared array itself: a pointer rebuilt from
   // an integer would lose its address space and the searches would issue
   // generic loads)
-  const size_t ve_off =
-      ((size_t)((const char *)(HC + nqmax + bin_win_size()) - (const char *)sm) + 15) &
-      ~(size_t)15;
+  const char *tail = RUN ? (const char *)Cc : (const char *)(HC + nqmax + bin_win_size());
+  const size_t ve_off = ((size_t)(tail - (const char *)sm) + 15) & ~(size_t)15;
   double *VE1 = (double *)((char *)sm + ve_off);
   double *VE2 = VE1 + (MAXV + 1), *VEP = VE2 + (MAXV + 1);
   VBinTab *VTS = (VBinTab *)(VEP + (MAXV + 1));
@@ -1033,7 +1043,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   const int64_t end = min(beg + (int64_t)a.chunk, nl);
   __syncthreads();  // the previous item is done with the shared tables
   if (t != tcur) {
-    load_tube_smem(a, t, T, E, Cc);
+    load_tube_smem(a, t, T, E, Cc, !RUN);
     for (int k = threadIdx.x; k < T.nq; k += blockDim.x) {
       const int64_t g = T.coff + k;
       const double ql = a.ct.qGL[g], qh = a.ct.qGH[g];
@@ -1136,6 +1146,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     // bins of the last value inside
     double l_vp = 0.0, l_s = 0.0;
     bool in_vp = false, in_s = false;
+    bool ins = well_inside(x0 - c0d);
 #pragma unroll 1
     for (unsigned m = 0;;) {
     const uint32_t step = step0 + m;
@@ -1150,47 +1161,27 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     const double u = quartic_newton_chord(
         q0, ipG, fma(o0, fma(1.0 - o0, cc.x, cu.y), cu.x));
     const double s2 = u * ipG;  // sin^2(theta)
-    // sqrt(s2): FP32 seed and one FP64 Newton step (relative error ~1e-14)
     const float s2f = (float)s2;
-    const float ysf = rsq(s2f);
-    double ys = (double)ysf;
-    ys = ys * fma(-0.5 * s2 * ys, ys, 1.5);
-    const double st = s2 * ys;
-    const double ct = q0 * u * u;
-    const double r = u * RE;
-    const double rho0 = r * st, z0 = r * ct;
-    // an offset strictly inside (0, 1) puts q0 inside cell c0 (its FP64
-    // rounding is far below the margin): no edge search
-    const int qi = (o0 > 1e-9 && o0 < 1.0 - 1e-9)
-                       ? c0 : cell_search_from(E, T.nq, T.sgn * q0, c0);
-    // ---- k1 geometry in FP32, from FP32 values (cos = q u^2, sin = s2
-    // rsqrt(s2)): two FP64->FP32 conversions fewer on the busy XU pipe, for
-    // a few FP32 roundings in forces that carry FP32 rounding anyway -------
+    // (a run knows from the step before; the search would find c0 too)
+    const int qi = ins ? c0 : cell_search_from(E, T.nq, T.sgn * q0, c0);
+    // ---- k1 geometry in FP32, from FP32 values (cos = q u^2): two
+    // FP64->FP32 conversions fewer on the busy XU pipe, for a few FP32
+    // roundings in forces that carry FP32 rounding anyway ------------------
     Geo<float> g1;
     g1.q = (float)q0;
     const float uf = (float)u;
     g1.ct = g1.q * uf * uf;
-    g1.st = s2f * ysf;
     const float rfl = uf * fRE;  // r in FP32
     g1.ir = rcpa(rfl);
     g1.ell = 1.0f + 3.0f * g1.ct * g1.ct;
     g1.isl = rsq(g1.ell);
-    g1.er = 3.0f * g1.ct * g1.st * g1.isl;
-    g1.ez = (3.0f * g1.ct * g1.ct - 1.0f) * g1.isl;
     const float vparf = (float)vpar, v1f = (float)v1, v2f = (float)v2;
     const float vp2 = v1f * v1f + v2f * v2f;
-    // the FP32 meridian point (used for the k2/k4 hemisphere signs and the
-    // turn of the field direction) from values already in FP32
-    const float rf = g1.st * rfl, zf = g1.ct * rfl;
-    // ---- the dominant displacement term h V|| e1 in FP64 (the direction
-    // from the FP64 cos/sin, 1/sqrt(ell) from the FP32 value and one FP64
-    // Newton step), taken now so that only its end point stays live --------
-    const double ell64 = fma(3.0 * ct, ct, 1.0);
+    // sqrt(ell) in FP64, ell = 1 + 3 cos^2 = 4 - 3 sin^2 on the field line:
+    // 1/sqrt from the FP32 value and one FP64 Newton step
+    const double ell64 = fma(-3.0, s2, 4.0);
     double yl = (double)g1.isl;
     yl = yl * fma(-0.5 * ell64 * yl, yl, 1.5);
-    const double hv = hd * vpar * yl;
-    const double xr0 = fma(hv, 3.0 * ct * st, rho0);
-    const double xz0 = fma(hv, fma(3.0 * ct, ct, -1.0), z0);
     if (bin_only) {
       int b1, b2, bp;
       start_bins<THREE_D>(a, I, j, VE1, VE2, VEP, VT1, VT2, VTP, vpar, v1, v2, b1, b2, bp);
@@ -1202,7 +1193,6 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     // (the FP64 kick of K64 runs after the position and V|| stores below:
     // nothing before them reads the kicked pair)
     if (!K64 && a.icr && qi >= 0) {
-      const float rr = (float)r;
       const float sl = g1.ell * g1.isl;
       const float ir3 = g1.ir * g1.ir * g1.ir;
       const float Om = qs_ms * (float)MDIP * sl * ir3;
@@ -1213,6 +1203,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
         v1n = v1 + (double)dv1;
         v2n = v2 + (double)dv2;
       } else {
+        const float rr = (float)(u * RE);
         const float invOm = c_invOm * (rr * rr * rr) * g1.isl;
         const HeatC<float> hc{hk[0], hk[1], hk[2], hk[3], hk[4], hk[5]};
         float w1 = v1f, w2 = v2f;
@@ -1235,7 +1226,8 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     // dF/ds = [s^2 c^2 (8 + 9 s^2/ell)/ell - (1 + c^2)(2 + s^2/ell)] / (ell r^2)
     // (dr/ds = 2c/sqrt(ell), dtheta/ds = s/(r sqrt(ell)) along the dipole e).
     const float il = g1.isl * g1.isl;  // 1/ell
-    const float sn2 = g1.st * g1.st, cs2 = g1.ct * g1.ct;
+    const float stf = s2f * rsq(s2f);  // sin(theta)
+    const float sn2 = stf * stf, cs2 = g1.ct * g1.ct;
     const float G2 = fmaf(sn2, il, 2.0f);
     const float hm = fc.cm * 1.5f * vp2 * g1.ir;
     const float M1 = hm * g1.ct * G2 * g1.isl;
@@ -1243,63 +1235,100 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
                      fmaf(sn2 * cs2 * il, fmaf(9.0f * sn2, il, 8.0f), -(1.0f + cs2) * G2);
     const float C0 = fc.ce2 * fabsf(aea) - fc.cg * fabsf(ag);
     const float Ce = fc.ce1 * aea;
-    const float a1 = M1 + (g1.ct <= 0.0f ? -C0 : C0) + Ce;
-    const float VRr = vparf * g1.er, VRz = vparf * g1.ez;
-    const float ds2 = hh * vparf, ds4 = fmaf(hsq2, a1, h * vparf);
-    const float z2 = fmaf(ds2, g1.ez, zf), z4 = fmaf(ds4, g1.ez, zf);
-    const float a2 = fmaf(dM, ds2, M1) + (z2 <= 0.0f ? -C0 : C0) + Ce;
-    const float a4 = fmaf(dM, ds4, M1) + (z4 <= 0.0f ? -C0 : C0) + Ce;
+    const float C1 = g1.ct <= 0.0f ? -C0 : C0;
+    const float a1 = M1 + C1 + Ce;
+    const float hvf = h * vparf, ds2 = hh * vparf, ds4 = fmaf(hsq2, a1, hvf);
     // q at the k4 point: dq/ds = -RE^2 sqrt(ell) / r^3 along e1
     if (last && a.write_qk4)
       QK[k] = fmaf(-(float)(RE * RE) * (g1.ell * g1.isl) * (g1.ir * g1.ir * g1.ir), ds4, g1.q);
-    // ---- displacement h/6 (V_R + 4 (V_R + h/2 A1) + (V_R + h A2)) ---------
-    // = h V|| e1 (FP64, above) + h^2/6 (2 a1 + a2) e1 (FP32; the k2 point's
-    // direction differs from e1 by ~1e-6 rad, ~1e-10 m here)
-    const float ac = hh6 * (2.0f * a1 + a2);
-    const float ddr = ac * g1.er, ddz = ac * g1.ez;
-    // ---- renormalisation in FP64: q of the new point --------------------
-    const double xr = xr0 + (double)ddr, xz = xz0 + (double)ddz;
-    const double r2 = xr * xr + xz * xz;
-    double y = (double)rsq((float)r2);
-    y = y * fma(-0.5 * r2 * y, y, 1.5);
-    const double qN = (RE * RE) * xz * (y * y * y);
-    // the new cell: most ions stay in the cell they started the step in,
-    // and an offset strictly inside (0, 1) there decides it without the
-    // edge search; escaped ions keep the end cell and an offset outside
-    const int cs = qi >= 0 ? qi : c0;
-    double cql = cq.x, cidq = cc.y;
-    if (cs != c0) {
-      cql = CS[cs].ql;
-      cidq = CS[cs].idq;
-    }
-    // (the product rounded on its own on every path: no fused multiply-add
-    // with the cell number)
-    double od = __dmul_rn(qN - cql, cidq);
-    double xN;
-    if (od > 1e-9 && od < 1.0 - 1e-9) {
-      // (a run: qi = c0 has been the cell of x0 all along unless the start
-      // lay next to an edge; the sum stays strictly inside the cell)
-      if (RUN) {
-        if (cs != c0) { c0 = cs; c0d = (double)cs; }
-        xN = c0d + od;
-      } else {
-        xN = (double)cs + od;
-      }
+    // ---- RK combination and renormalisation -------------------------------
+    // displacement h/6 (V_R + 4 (V_R + h/2 A1) + (V_R + h A2)) = (h V|| + h^2/6
+    // (2 a1 + a2)) e1 (the k2 point's direction differs from e1 by ~1e-6 rad,
+    // ~1e-10 m here): D along e1, dl = D / r.  q of the new point is q =
+    // RE^2 z / r^3 along the line x1 + D e1: with k = RE^2 / r^2, rho = e1 .
+    // x1 / r = 2 cos / sqrt(ell) and e_z the z component of e1,
+    //   q + k [-sqrt(ell) dl + c2 dl^2 + c3 dl^3 + O(dl^4)],
+    //   c2 = cos (15/2 rho^2 - 3/2) - 3 rho e_z,
+    //   c3 = (15/2 rho^2 - 3/2) e_z + cos rho (15/2 - 35/2 rho^2).
+    // The first-order term of h V|| is taken in FP64 (k / r = (1/u)^3 / RE
+    // with 1/u = 1/p + q^2 u^3 from the quartic), the rest, smaller by dl or
+    // by ac / (h V||), in FP32.  For |dl| <= 1e-4 (700 m at 1000 km altitude)
+    // the terms left out are below 1e-15 of q and the FP32 rounding below
+    // 4e-15; off the equator by more than that every stage has the
+    // hemisphere sign of the start.  The general expressions serve the rest.
+    // (Every multiply-add written out: the same rounding in every variant of
+    // the kernel.)
+    // (All through the meridian point in FP64, as the general ones are: 367
+    // instructions per ion and step where this takes 319, 3.05 ms per 20
+    // steps of 1e7 ions where this takes 2.83, and an error of q some 20
+    // times larger after 100 steps, from the refinements' ~1e-14 a step.)
+    double qN, dq = 0.0, od;
+    float a2 = fmaf(dM, ds2, M1), a4 = fmaf(dM, ds4, M1), dal;
+    const float pl = 3.0f * fmaf(g1.ct, g1.ct, 1.0f) * il;
+    const bool near = fmaxf(fabsf(hvf), fabsf(ds4)) * g1.ir <= 1e-4f && fabsf(g1.ct) > 2e-4f;
+    if (near) {
+      a2 = a2 + C1 + Ce;
+      a4 = a4 + C1 + Ce;
+      const float at = fmaf(2.0f, a1, a2), ac = hh6 * at;
+      const float dl = fmaf(hh6, at, hvf) * g1.ir;
+      const double qu = q0 * u;
+      const double iu = fma(qu * qu, u, ipG);  // 1/u
+      const double g = (ell64 * yl) * iu * (iu * iu);
+      const float xl = cs2 * il, nz = g1.ell - 2.0f;  // e_z sqrt(ell)
+      const float kk = fmaf(30.0f, xl, -1.5f);
+      const float c2 = g1.ct * fmaf(-6.0f * nz, il, kk);
+      const float c3 = g1.isl * fmaf(kk, nz, 2.0f * cs2 * fmaf(-70.0f, xl, 7.5f));
+      const float dq2 = (float)(RE * RE) * (g1.ir * g1.ir) *
+                        fmaf(dl * dl, fmaf(dl, c3, c2), -(g1.ell * g1.isl) * (ac * g1.ir));
+      dq = fma(hmre * vpar, g, (double)dq2);
+      od = fma(dq, cc.y, o0);
+      dal = pl * dl * (stf * g1.isl);
     } else {
-      const int cN = cell_search_from(E, T.nq, T.sgn * qN, cs);
+      const float ez = (g1.ell - 2.0f) * g1.isl, zf = g1.ct * rfl;
+      const float z2 = fmaf(ds2, ez, zf), z4 = fmaf(ds4, ez, zf);
+      a2 = a2 + (z2 <= 0.0f ? -C0 : C0) + Ce;
+      a4 = a4 + (z4 <= 0.0f ? -C0 : C0) + Ce;
+      const float ac = hh6 * (2.0f * a1 + a2);
+      // cos, sin and the meridian point in FP64 (sin from an FP32 seed and
+      // one FP64 Newton step)
+      double ys = (double)rsq(s2f);
+      ys = ys * fma(-0.5 * s2 * ys, ys, 1.5);
+      const double st = s2 * ys, ct = q0 * u * u, r = u * RE;
+      const double hv = hd * vpar * yl;
+      const double xr = fma(hv, 3.0 * ct * st, r * st) +
+                        (double)(ac * (3.0f * g1.ct * stf * g1.isl));
+      const double xz = fma(hv, fma(3.0 * ct, ct, -1.0), r * ct) + (double)(ac * ez);
+      const double r2 = xr * xr + xz * xz;
+      double y = (double)rsq((float)r2);
+      y = y * fma(-0.5 * r2 * y, y, 1.5);
+      qN = (RE * RE) * xz * (y * y * y);
+      od = __dmul_rn(qN - cq.x, cc.y);
+      dal = pl * ((hvf + ac) * g1.ir) * (stf * g1.isl);
+    }
+    // V|| along the new field direction: the turn of the direction over the
+    // step, dal = 3 (1 + cos^2) / ell dtheta, dtheta = D / r sin / sqrt(ell)
+    const float dv = fmaf(h6, a1 + 4.0f * a2 + a4, -0.5f * vparf * dal * dal);
+    const double vparN = vpar + (double)dv;
+    // the new cell: most ions stay well inside the cell they started the
+    // step in; else the edge search (escaped ions keep the end cell and an
+    // offset outside).  Products rounded on their own: no fused multiply-add
+    // with the cell number.
+    double xN;
+    ins = ins && well_inside(od);
+    if (ins) {
+      xN = c0d + od;
+    } else {
+      if (near) qN = q0 + dq;
+      const int cN = cell_search_from(E, T.nq, T.sgn * qN, qi >= 0 ? qi : c0);
       const int cpos = cN >= 0 ? cN : (cN == BELOW ? 0 : T.nq - 1);
       od = __dmul_rn(qN - CS[cpos].ql, CS[cpos].idq);
       xN = (double)cpos + od;
       if (RUN) {  // the cell as the next step reads it from the coordinate
         c0 = x_cell(xN, T.nq);
         c0d = (double)c0;
+        ins = well_inside(xN - c0d);
       }
     }
-    // ---- V|| along the new field direction ------------------------------
-    const float dth = (zf * fmaf(h, VRr, ddr) - rf * fmaf(h, VRz, ddz)) * (g1.ir * g1.ir);
-    const float dal = 3.0f * fmaf(g1.ct, g1.ct, 1.0f) * (g1.isl * g1.isl) * dth;
-    const float dv = fmaf(h6, a1 + 4.0f * a2 + a4, -0.5f * vparf * dal * dal);
-    const double vparN = vpar + (double)dv;
     if (RUN && !THREE_D) {
       if (vpar >= VEP[0] && vpar <= VEP[c_vg.npar]) { l_vp = vpar; in_vp = true; }
       if (m == 0u || a.icr) {  // (the speed changes only by the kicks)
@@ -1325,6 +1354,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
         // / r^3 and 1/Omega from the FP64 radius and 1/sqrt(ell) (yl), 1/r
         // from the FP32 reciprocal and one FP64 Newton step (relative error
         // ~1e-14); the RK above used the pre-kick Vperp, as heat() does
+        const double r = u * RE;
         double ir = (double)rcpa((float)r);
         ir = ir * fma(-r, ir, 2.0);
         const double Om = qs_ms64 * MDIP * (ell64 * yl) * (ir * ir * ir);
