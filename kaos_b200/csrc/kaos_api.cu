@@ -31,6 +31,7 @@ constexpr int BC_THREADS = 256;
 // arrays are compacted (order-preserving) every BC_COMPACT_EVERY master
 // steps, or earlier when an injection could overflow a tube's capacity.
 constexpr int BC_COMPACT_EVERY = 8;
+constexpr int64_t COUNT_STAGE = 64 * 1024;  // counters per staging buffer
 // cells per tube: the per-cell tables of a tube live in shared memory (the
 // mixed push holds 92 bytes per cell, the collision-count kernel 64)
 constexpr int MAX_CELLS = 2048;
@@ -104,6 +105,16 @@ struct kaos_handle {
   // the charge exchange, join before anything that follows the pushes)
   cudaStream_t s2 = nullptr;
   cudaEvent_t efork = nullptr, ejoin = nullptr;
+  // Per-tube counts in one device block [NSTAT][ntubes], the status word
+  // behind it; kaos_step copies the block to stat_host as its last work, so
+  // the getters of counts and boundary fluxes need no copy.  (Pageable: a
+  // pinned block saves ~5 us a step call and costs 1 ms at creation.)
+  enum { ST_LIVE, ST_DEAD, ST_ENA, ST_LB_OUT, ST_UB_OUT, ST_LB_IN, ST_UB_IN, ST_LBE, ST_UBE, NSTAT };
+  int64_t *d_stat = nullptr, *stat_host = nullptr, *d_ndead = nullptr;
+  std::vector<int64_t> stat_store;
+  size_t stat_bytes = 0;
+  unsigned *cnt_stage = nullptr;  // kaos_get_counts: 2 x COUNT_STAGE, pinned
+  int stat_ok = 0;  // stat_host holds the device's values
   // device
   TubeD *d_tubes = nullptr;
   int *d_blk_tube = nullptr;
@@ -147,7 +158,7 @@ struct kaos_handle {
   TubeD *d_conv_td = nullptr;
   int *d_conv_tube = nullptr;
   struct ConvHost {
-    double *stage = nullptr;  // pinned: [move][table][nqmax]
+    double *stage = nullptr;  // pinned: [move][raw table][nqmax]
     std::vector<double> pnew;
     std::vector<TubeD> td;
     std::vector<int> tube;
@@ -186,12 +197,11 @@ struct kaos_handle {
   int rank = 0, nranks = 1;          // share of the charge-exchange counts
   std::vector<uint64_t> id_base;     // first ion id per tube
   // tube moves (kaos_update_tube) applied at the next master step
-  struct PendingTube {
+  struct PendingTube {  // entry k's tables: row block k of conv_host.stage
     int tube;
     TubeD d;
-    std::vector<std::vector<double>> tables;  // in CONV_TABLES order
   };
-  std::vector<PendingTube> pending, applied;
+  std::vector<PendingTube> pending;
   // push work items: (tube, chunk of ions) maps, one per candidate chunk
   struct WorkMap {
     int chunk = 0, n = 0;
@@ -460,38 +470,22 @@ int zero_accum(kaos_handle *h) {
   return KAOS_OK;
 }
 
-// The per-cell tables of one tube, in the order of CellTables' pointers
-// listed by conv_table_ptr (the same values kaos_create builds).
-constexpr int CONV_TABLES = 28;
-std::vector<std::vector<double>> tube_tables(const kaos_tube_c &T, const TubeD &d,
-                                             const kaos_params_c &p) {
-  std::vector<std::vector<double>> v(CONV_TABLES);
-  auto app = [&](int k, const double *src, double dflt) {
-    for (int c = 0; c < T.nq; ++c) v[k].push_back(src ? src[c] : dflt);
-  };
-  app(0, T.qGL, 0); app(1, T.qGH, 0); app(2, T.qGC, 0); app(3, T.hqC, 0);
-  app(4, T.dqC, 0); app(5, T.d3xC, 1); app(6, T.rGC, 0); app(7, T.thetaGC, 0);
-  app(8, T.ellGC, 1); app(9, T.TeG, 0); app(10, T.TsG, 0); app(11, T.nsnormCNeut, 0);
-  app(12, T.lambdaPerp, 0); app(13, T.EtaLH, 0); app(14, T.XiPerp1, 0);
-  app(15, T.XiPerp2, 0); app(16, T.S0, 0); app(17, T.OmegaG0, 1);
-  app(18, T.ChiPerp1, 0); app(19, T.ChiPerp2, 0);
-  for (int c = 0; c < T.nq; ++c) {
-    v[20].push_back(host_quartic_u(T.qGL[c], T.pG));
-    v[21].push_back(host_quartic_u(T.qGH[c], T.pG));
-    const double pre = (d.qs * d.qs / (2.0 * d.ms * d.ms)) *
-                       (T.S0 ? T.S0[c] : 0.0) * (T.EtaLH ? T.EtaLH[c] : 0.0);
-    v[22].push_back(p.h * std::sqrt(pre * (T.XiPerp1 ? T.XiPerp1[c] : 0.0) / PI));
-    v[23].push_back(p.h * std::sqrt(pre * (T.XiPerp2 ? T.XiPerp2[c] : 0.0) / PI));
-    v[24].push_back(0.5 * (T.ChiPerp1 ? T.ChiPerp1[c] : 0.0));
-    v[25].push_back(0.5 * (T.ChiPerp2 ? T.ChiPerp2[c] : 0.0));
-    v[26].push_back(T.OmegaG0 && T.OmegaG0[c] != 0.0 ? 1.0 / T.OmegaG0[c] : 0.0);
-    v[27].push_back(host_quartic_u(0.5 * (T.qGL[c] + T.qGH[c]), T.pG));
-  }
-  return v;
+// The tables a caller gives for one tube, in the order of CellTables'
+// pointers listed by conv_table_ptr, into rows of nqm doubles (the derived
+// ones follow on the device, k_apply_tables).
+void tube_tables(const kaos_tube_c &T, double *out, int nqm) {
+  const struct { const double *src; double dflt; } in[CONV_RAW] = {
+      {T.qGL, 0}, {T.qGH, 0}, {T.qGC, 0}, {T.hqC, 0}, {T.dqC, 0}, {T.d3xC, 1}, {T.rGC, 0},
+      {T.thetaGC, 0}, {T.ellGC, 1}, {T.TeG, 0}, {T.TsG, 0}, {T.nsnormCNeut, 0},
+      {T.lambdaPerp, 0}, {T.EtaLH, 0}, {T.XiPerp1, 0}, {T.XiPerp2, 0}, {T.S0, 0},
+      {T.OmegaG0, 1}, {T.ChiPerp1, 0}, {T.ChiPerp2, 0}};
+  for (int k = 0; k < CONV_RAW; ++k, out += nqm)
+    if (in[k].src) memcpy(out, in[k].src, (size_t)T.nq * sizeof(double));
+    else std::fill(out, out + T.nq, in[k].dflt);
 }
 
 const double *conv_table_ptr(const CellTables &c, int k) {
-  const double *p[CONV_TABLES] = {c.qGL, c.qGH, c.qGC, c.hqC, c.dqC, c.d3xC, c.rGC,
+  const double *p[CONV_NTAB] = {c.qGL, c.qGH, c.qGC, c.hqC, c.dqC, c.d3xC, c.rGC,
                                   c.thetaGC, c.ellGC, c.TeG, c.TsG, c.nsnormCNeut,
                                   c.lambdaPerp, c.EtaLH, c.XiPerp1, c.XiPerp2, c.S0,
                                   c.OmegaG0, c.ChiPerp1, c.ChiPerp2, c.uL, c.uH,
@@ -505,24 +499,28 @@ const double *conv_table_ptr(const CellTables &c, int k) {
 // copy.
 static int sm_count(kaos_handle *h);
 
+// Staging of the moves of one master step: room for every entry at once.
+int conv_staging(kaos_handle *h) {
+  if (h->conv_host.stage) return KAOS_OK;
+  int rc;
+  const size_t len = (size_t)h->ntubes * CONV_RAW * max_nq(h);
+  if ((rc = dalloc(h, &h->d_conv_stage, len)) ||
+      (rc = dalloc(h, &h->d_conv_td, (size_t)h->ntubes)) ||
+      (rc = dalloc(h, &h->d_conv_tube, (size_t)h->ntubes)) ||
+      (rc = dalloc(h, &h->d_conv_pnew, (size_t)h->ntubes)))
+    return rc;
+  CK(cudaDeviceSynchronize());  // dalloc's clearing, before the copies on h->s
+  CK(cudaMallocHost((void **)&h->conv_host.stage, len * sizeof(double)));
+  return KAOS_OK;
+}
+
 int apply_pending_tubes(kaos_handle *h) {
-  static_assert(CONV_TABLES == CONV_NTAB, "table count");
   const int np = (int)h->pending.size();
   if (!np) return KAOS_OK;
   const int nqm = max_nq(h);
-  int rc;
-  const size_t stage_len = (size_t)h->ntubes * CONV_TABLES * nqm;
-  if (!h->d_conv_stage) {  // staging for every entry moving at once
-    if ((rc = dalloc(h, &h->d_conv_stage, stage_len)) ||
-        (rc = dalloc(h, &h->d_conv_td, (size_t)h->ntubes)) ||
-        (rc = dalloc(h, &h->d_conv_tube, (size_t)h->ntubes)) ||
-        (rc = dalloc(h, &h->d_conv_pnew, (size_t)h->ntubes)))
-      return rc;
-    CK(cudaMallocHost((void **)&h->conv_host.stage, stage_len * sizeof(double)));
-  }
-  // the moves, their new descriptors and tables in host staging (the tables
-  // in pinned memory, copied asynchronously; the staging is next written at
-  // the next move, after the step that applied this one has finished)
+  // the moves' descriptors; their tables lie in the pinned staging since
+  // kaos_update_tube, which runs between calls of kaos_step, so never while
+  // this copy is under way
   auto &S = h->conv_host;
   S.td.resize(np);
   S.tube.resize(np);
@@ -532,11 +530,8 @@ int apply_pending_tubes(kaos_handle *h) {
     S.td[p] = pt.d;
     S.tube[p] = pt.tube;
     S.pnew[p] = pt.d.pG;
-    for (int k = 0; k < CONV_TABLES; ++k)
-      std::copy(pt.tables[k].begin(), pt.tables[k].end(),
-                S.stage + ((size_t)p * CONV_TABLES + k) * nqm);
   }
-  CK(cudaMemcpyAsync(h->d_conv_stage, S.stage, (size_t)np * CONV_TABLES * nqm * sizeof(double),
+  CK(cudaMemcpyAsync(h->d_conv_stage, S.stage, (size_t)np * CONV_RAW * nqm * sizeof(double),
                      cudaMemcpyHostToDevice, h->s));
   CK(cudaMemcpyAsync(h->d_conv_td, S.td.data(), np * sizeof(TubeD), cudaMemcpyHostToDevice, h->s));
   CK(cudaMemcpyAsync(h->d_conv_tube, S.tube.data(), np * sizeof(int), cudaMemcpyHostToDevice, h->s));
@@ -552,13 +547,14 @@ int apply_pending_tubes(kaos_handle *h) {
   ca.mixed = h->mixed;
   k_convect_many<<<dim3(std::max(1, sm_count(h) * 16 / np), np), 256, 0, h->s>>>(ca);
   TableApplyArgs ta{};
-  for (int k = 0; k < CONV_TABLES; ++k) ta.dst[k] = (double *)conv_table_ptr(h->ct, k);
+  for (int k = 0; k < CONV_NTAB; ++k) ta.dst[k] = (double *)conv_table_ptr(h->ct, k);
   ta.stage = h->d_conv_stage;
   ta.td = h->d_conv_td;
   ta.tube = h->d_conv_tube;
   ta.tubes = h->d_tubes;
   ta.nqmax = nqm;
-  k_apply_tables<<<dim3(CONV_TABLES, np), 256, 0, h->s>>>(ta);
+  ta.h = h->P.h;
+  k_apply_tables<<<dim3(CONV_RAW + 1, np), 256, 0, h->s>>>(ta);
   h->launches += 2;
   CK(cudaGetLastError());
   for (const auto &pt : h->pending) h->th[pt.tube] = pt.d;
@@ -724,10 +720,8 @@ int launch_boundary(kaos_handle *h, int compact) {
     b.ub_out = h->d_ub_out;
     b.qind_w = h->ion[h->cur].qind;
     b.x_w = h->mixed ? h->ion[h->cur].x : nullptr;
-    CK(cudaMemsetAsync(h->d_lb_out, 0, h->ntubes * sizeof(unsigned long long), h->s));
-    CK(cudaMemsetAsync(h->d_ub_out, 0, h->ntubes * sizeof(unsigned long long), h->s));
-    CK(cudaMemsetAsync(h->d_lb_in, 0, h->ntubes * sizeof(unsigned long long), h->s));
-    CK(cudaMemsetAsync(h->d_ub_in, 0, h->ntubes * sizeof(unsigned long long), h->s));
+    b.ndead = h->d_ndead;
+    CK(cudaMemsetAsync(h->d_lb_out, 0, 4 * h->ntubes * sizeof(int64_t), h->s));  // all four
     k_bc_mark<<<h->nblk, BC_THREADS, 0, h->s>>>(b);
     h->launches++;
     CK(cudaGetLastError());
@@ -746,10 +740,8 @@ int launch_boundary(kaos_handle *h, int compact) {
   b.lb_out = h->d_lb_out;
   b.ub_out = h->d_ub_out;
   b.fields = ion_fields(h, h->cur, 1 - h->cur);
-  CK(cudaMemsetAsync(h->d_lb_out, 0, h->ntubes * sizeof(unsigned long long), h->s));
-  CK(cudaMemsetAsync(h->d_ub_out, 0, h->ntubes * sizeof(unsigned long long), h->s));
-  CK(cudaMemsetAsync(h->d_lb_in, 0, h->ntubes * sizeof(unsigned long long), h->s));
-  CK(cudaMemsetAsync(h->d_ub_in, 0, h->ntubes * sizeof(unsigned long long), h->s));
+  b.ndead = h->d_ndead;
+  CK(cudaMemsetAsync(h->d_lb_out, 0, 4 * h->ntubes * sizeof(int64_t), h->s));  // all four
   BcArgs bc = b;
   bc.nlive = h->d_nlive;  // count reads the live counts
   k_bc_count<<<h->nblk, BC_THREADS, 0, h->s>>>(bc);
@@ -821,6 +813,7 @@ CxArgs cx_args(kaos_handle *h) {
   a.chunk_list = h->d_cx_chunks;
   a.nchunk = h->d_cx_nchunk;
   a.tube_active = h->d_tube_active;
+  a.ndead = h->d_ndead;
   a.rank = h->rank;
   a.nranks = h->nranks;
   a.nqmax = max_nq(h);
@@ -922,8 +915,7 @@ int launch_boundary_ena(kaos_handle *h) {
   F.f[F.n++] = Field{A.qind, B.qind, 4}; F.f[F.n++] = Field{A.vb, B.vb, 4};
   F.f[F.n++] = Field{A.id, B.id, 8};
   b.fields = F;
-  CK(cudaMemsetAsync(h->d_lbe_out, 0, h->ntubes * sizeof(unsigned long long), h->s));
-  CK(cudaMemsetAsync(h->d_ube_out, 0, h->ntubes * sizeof(unsigned long long), h->s));
+  CK(cudaMemsetAsync(h->d_lbe_out, 0, 2 * h->ntubes * sizeof(int64_t), h->s));  // both
   BcArgs bc = b;
   bc.nlive = h->d_nena;
   k_bc_count<<<h->neblk, BC_THREADS, 0, h->s>>>(bc);
@@ -1043,7 +1035,6 @@ int step_once(kaos_handle *h) {
   // ConvectionSub runs first on a master step (_8_KineticSolver.f90:62)
   if (master && !h->pending.empty()) {
     if ((rc = apply_pending_tubes(h))) return rc;
-    for (auto &pt : h->pending) h->applied.push_back(std::move(pt));
     h->pending.clear();
   }
   // an idle interval converts nothing: no selection; its master step still
@@ -1265,6 +1256,23 @@ int graph_steps(kaos_handle *h, int g) {
 }
 
 constexpr int GRAPH_RUN = 8;  // ordinary steps per replayed graph
+
+// The per-tube counts as of the last call: what kaos_step brought back, or
+// read from the device (before the first step, after an error).
+int tube_stat(kaos_handle *h, const int64_t **st) {
+  if (!h->stat_host) return fail(h, KAOS_ERR_STATE, "the handle was not created");
+  if (!h->stat_ok) {
+    CK(cudaStreamSynchronize(h->s));
+    CK(cudaMemcpy(h->stat_host, h->d_stat, h->stat_bytes, cudaMemcpyDeviceToHost));
+    h->stat_ok = 1;
+  }
+  *st = h->stat_host;
+  return KAOS_OK;
+}
+int64_t live_ions(const kaos_handle *h, const int64_t *st, int tube) {
+  return st[(size_t)kaos_handle::ST_LIVE * h->ntubes + tube] -
+         st[(size_t)kaos_handle::ST_DEAD * h->ntubes + tube];
+}
 
 }  // namespace
 
@@ -1502,16 +1510,30 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
     if ((rc = work_map(h->wmap[m], CHUNKS[m]))) return rc;
   h->rmap = h->wmap[0];
   if (h->rmap.chunk != run_chunk(h) && (rc = work_map(h->rmap, run_chunk(h)))) return rc;
-  if ((rc = dalloc(h, &h->d_nlive, ntubes))) return rc;
+  {
+    const size_t n = (size_t)kaos_handle::NSTAT * ntubes;
+    h->stat_bytes = (n + 1) * sizeof(int64_t);
+    if ((rc = dalloc(h, &h->d_stat, n + 1))) return rc;
+    h->stat_store.assign(n + 1, 0);
+    h->stat_host = h->stat_store.data();
+    auto row = [&](int k) { return h->d_stat + (size_t)k * ntubes; };
+    h->d_nlive = row(kaos_handle::ST_LIVE);
+    h->d_ndead = row(kaos_handle::ST_DEAD);
+    h->d_lb_out = (unsigned long long *)row(kaos_handle::ST_LB_OUT);
+    h->d_ub_out = (unsigned long long *)row(kaos_handle::ST_UB_OUT);
+    h->d_lb_in = (unsigned long long *)row(kaos_handle::ST_LB_IN);
+    h->d_ub_in = (unsigned long long *)row(kaos_handle::ST_UB_IN);
+    if (p->QEXCHANGEflag == 1) {
+      h->d_nena = row(kaos_handle::ST_ENA);
+      h->d_lbe_out = (unsigned long long *)row(kaos_handle::ST_LBE);
+      h->d_ube_out = (unsigned long long *)row(kaos_handle::ST_UBE);
+    }
+    h->d_status = (uint32_t *)(h->d_stat + n);
+  }
   if ((rc = dalloc(h, &h->d_nlive_new, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_next_id, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_blkcnt, bt.size()))) return rc;
   if ((rc = dalloc(h, &h->d_blkoff, bt.size()))) return rc;
-  if ((rc = dalloc(h, &h->d_lb_out, ntubes))) return rc;
-  if ((rc = dalloc(h, &h->d_ub_out, ntubes))) return rc;
-  if ((rc = dalloc(h, &h->d_lb_in, ntubes))) return rc;
-  if ((rc = dalloc(h, &h->d_ub_in, ntubes))) return rc;
-  if ((rc = dalloc(h, &h->d_status, 1))) return rc;
   if ((rc = dalloc(h, &h->d_step, 1))) return rc;
   // particle arrays (two buffer sets for the order-preserving compaction)
   const int64_t cap = poff;
@@ -1599,9 +1621,8 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
         (rc = up_i(&h->d_tube_eblk0, te0)) || (rc = up_i(&h->d_cx_tube, cxt)) ||
         (rc = up_l(&h->d_cx_start, cxs)) || (rc = up_i(&h->d_tube_cx0, tc0)))
       return rc;
-    if ((rc = dalloc(h, &h->d_nena, ntubes)) || (rc = dalloc(h, &h->d_nena_new, ntubes)) ||
+    if ((rc = dalloc(h, &h->d_nena_new, ntubes)) ||
         (rc = dalloc(h, &h->d_eblkcnt, ebt.size())) || (rc = dalloc(h, &h->d_eblkoff, ebt.size())) ||
-        (rc = dalloc(h, &h->d_lbe_out, ntubes)) || (rc = dalloc(h, &h->d_ube_out, ntubes)) ||
         (rc = dalloc(h, &h->d_cxconv, cxt.size())) ||
         (rc = dalloc(h, &h->d_cxbase, cxt.size())) ||
         (rc = dalloc(h, &h->d_cxend, (size_t)h->ncell)) ||
@@ -1682,7 +1703,9 @@ int kaos_load_particles(kaos_handle *h, int32_t tube, const double *q,
   int64_t nl = n;
   uint64_t nid = h->id_base[tube] + (uint64_t)n;
   h->bc_bound[tube] = n;
+  h->stat_ok = 0;
   CK(cudaMemcpy(h->d_nlive + tube, &nl, sizeof(int64_t), cudaMemcpyHostToDevice));
+  CK(cudaMemset(h->d_ndead + tube, 0, sizeof(int64_t)));
   CK(cudaMemcpy(h->d_next_id + tube, &nid, sizeof(uint64_t), cudaMemcpyHostToDevice));
   if (h->d_cxc)  // the first push starts the selection counts from zero
     CK(cudaMemset(h->d_cxc, 0, (size_t)h->ncx * max_nq(h) * sizeof(unsigned)));
@@ -1738,7 +1761,9 @@ int kaos_init_particles(kaos_handle *h, int32_t tube, const kaos_init_c *in) {
   int64_t nl = n;
   uint64_t nid = h->id_base[tube] + (uint64_t)n;
   h->bc_bound[tube] = n;
+  h->stat_ok = 0;
   CK(cudaMemcpy(h->d_nlive + tube, &nl, sizeof(int64_t), cudaMemcpyHostToDevice));
+  CK(cudaMemset(h->d_ndead + tube, 0, sizeof(int64_t)));
   CK(cudaMemcpy(h->d_next_id + tube, &nid, sizeof(uint64_t), cudaMemcpyHostToDevice));
   if (h->d_cxc)  // the first push starts the selection counts from zero
     CK(cudaMemset(h->d_cxc, 0, (size_t)h->ncx * max_nq(h) * sizeof(unsigned)));
@@ -1765,6 +1790,7 @@ int kaos_set_export(kaos_handle *h, int32_t on) {
   if (on && !h->acc.hist) {
     int rc = dalloc(h, &h->acc.hist, (size_t)h->ncell * h->nv);
     if (rc) return rc;
+    CK(cudaMallocHost((void **)&h->cnt_stage, 2 * COUNT_STAGE * sizeof(unsigned)));
   }
   h->export_on = on ? 1 : 0;
   return KAOS_OK;
@@ -1840,14 +1866,15 @@ int kaos_update_tube(kaos_handle *h, int32_t tube, const kaos_tube_c *T) {
   pt.d.sumdsICR = T->sumdsICR;
   host_rho_z(T->qGC[0], T->pG, &pt.d.rhoLB, &pt.d.zLB);
   host_rho_z(T->qGC[T->nq - 1], T->pG, &pt.d.rhoUB, &pt.d.zUB);
-  pt.tables = tube_tables(*T, pt.d, h->P);
+  const int rc = conv_staging(h);
+  if (rc) return rc;
   note_heating(h, *T);
-  for (auto &q : h->pending)
-    if (q.tube == tube) {
-      q = std::move(pt);
-      return KAOS_OK;
-    }
-  h->pending.push_back(std::move(pt));
+  size_t k = 0;
+  while (k < h->pending.size() && h->pending[k].tube != tube) ++k;
+  if (k == h->pending.size()) h->pending.push_back(pt);
+  else h->pending[k] = pt;
+  const int nqm = max_nq(h);
+  tube_tables(*T, h->conv_host.stage + k * CONV_RAW * nqm, nqm);
   return KAOS_OK;
 }
 
@@ -1893,6 +1920,7 @@ int kaos_step(kaos_handle *h, int64_t nsteps) {
   }
   h->launches = 0;
   h->npev = 0;
+  h->stat_ok = 0;
   CK(cudaEventRecord(h->e0, h->s));
   for (int64_t k = 0; k < nsteps;) {
     const int64_t n = h->n + 1;
@@ -1921,8 +1949,9 @@ int kaos_step(kaos_handle *h, int64_t nsteps) {
     k += g;
   }
   CK(cudaEventRecord(h->e1, h->s));
-  CK(cudaEventSynchronize(h->e1));
-  h->applied.clear();  // their host tables have been copied
+  CK(cudaMemcpyAsync(h->stat_host, h->d_stat, h->stat_bytes, cudaMemcpyDeviceToHost, h->s));
+  CK(cudaStreamSynchronize(h->s));
+  h->stat_ok = 1;
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, h->e0, h->e1));
   h->last_ms = ms;
@@ -1932,8 +1961,7 @@ int kaos_step(kaos_handle *h, int64_t nsteps) {
     CK(cudaEventElapsedTime(&m, h->pev[2 * k], h->pev[2 * k + 1]));
     h->push_ms += m;
   }
-  uint32_t st = 0;
-  CK(cudaMemcpy(&st, h->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+  const uint32_t st = *(const uint32_t *)(h->stat_host + (size_t)kaos_handle::NSTAT * h->ntubes);
   if (st & ST_NAN) return fail(h, KAOS_ERR_NAN, "non-finite particle state on the device");
   if (st & ST_CAP) return fail(h, KAOS_ERR_CAPACITY, "tube capacity exceeded during injection");
   return KAOS_OK;
@@ -1953,36 +1981,14 @@ int kaos_get_status(kaos_handle *h, uint32_t *status) {
 
 int kaos_get_count(kaos_handle *h, int32_t tube, int64_t *nion, int64_t *nena) {
   if (!h || tube < 0 || tube >= h->ntubes) return KAOS_ERR_PARAM;
-  CK(cudaStreamSynchronize(h->s));
-  int64_t nl = 0;
-  CK(cudaMemcpy(&nl, h->d_nlive + tube, sizeof(int64_t), cudaMemcpyDeviceToHost));
-  // slots converted to ENAs or marked at a removal (DEAD) are not ions:
-  // the live slots are counted on the device (the export's count and scan)
-  int64_t live = 0;
-  if (nl) {
-    ExportArgs a{};
-    a.ion = h->ion[h->cur];
-    a.off = h->th[tube].off;
-    a.nl = nl;
-    a.nb = (int)ceil_div(nl, (int64_t)EXP_THREADS * EXP_ITEMS);
-    a.blkoff = (unsigned long long *)h->d_blkoff;
-    a.blkcnt = (unsigned *)h->d_blkcnt;
-    a.total = (unsigned long long *)(h->d_nlive_new + tube);
-    k_exp_count<<<a.nb, EXP_THREADS, 0, h->s>>>(a);
-    k_exp_scan<<<1, 1024, 0, h->s>>>(a);
-    CK(cudaGetLastError());
-    unsigned long long t = 0;
-    CK(cudaMemcpyAsync(&t, a.total, sizeof(t), cudaMemcpyDeviceToHost, h->s));
-    CK(cudaStreamSynchronize(h->s));
-    live = (int64_t)t;
-  }
-  if (nion) *nion = live;
-  int64_t ne = 0;
-  if (h->d_nena) {
-    CK(cudaMemcpy(&ne, h->d_nena + tube, sizeof(int64_t), cudaMemcpyDeviceToHost));
-    ne = std::min(ne, h->th[tube].ecap);
-  }
-  if (nena) *nena = ne;
+  const int64_t *st = nullptr;
+  const int rc = tube_stat(h, &st);
+  if (rc) return rc;
+  // slots converted to ENAs or marked at a removal (DEAD) are not ions
+  if (nion) *nion = live_ions(h, st, tube);
+  if (nena)
+    *nena = h->d_nena ? std::min(st[(size_t)kaos_handle::ST_ENA * h->ntubes + tube],
+                                 h->th[tube].ecap) : 0;
   return KAOS_OK;
 }
 
@@ -1992,20 +1998,17 @@ int kaos_get_moments(kaos_handle *h, int32_t tube, int32_t which, double *out,
       which >= KAOS_NMOMENTS)
     return KAOS_ERR_PARAM;
   if (nq != h->th[tube].nq) return fail(h, KAOS_ERR_PARAM, "nq mismatch");
+  CK(cudaMemcpyAsync(out, mom_row(h->ct, h->th[tube], which), nq * sizeof(double),
+                     cudaMemcpyDeviceToHost, h->s));
   CK(cudaStreamSynchronize(h->s));
-  CK(cudaMemcpy(out, h->ct.mom + which * h->ncell + h->th[tube].coff,
-                nq * sizeof(double), cudaMemcpyDeviceToHost));
   return KAOS_OK;
 }
 
 int kaos_get_moments_all(kaos_handle *h, int32_t tube, double *out, int32_t nq) {
   if (!h || !out || tube < 0 || tube >= h->ntubes) return KAOS_ERR_PARAM;
   if (nq != h->th[tube].nq) return fail(h, KAOS_ERR_PARAM, "nq mismatch");
-  // rows of the [KAOS_NMOMENTS][ncell] block, the tube's nq cells of each
-  CK(cudaMemcpy2DAsync(out, (size_t)nq * sizeof(double),
-                       h->ct.mom + h->th[tube].coff, (size_t)h->ncell * sizeof(double),
-                       (size_t)nq * sizeof(double), KAOS_NMOMENTS,
-                       cudaMemcpyDeviceToHost, h->s));
+  CK(cudaMemcpyAsync(out, mom_row(h->ct, h->th[tube], 0),
+                     (size_t)KAOS_NMOMENTS * nq * sizeof(double), cudaMemcpyDeviceToHost, h->s));
   CK(cudaStreamSynchronize(h->s));
   return KAOS_OK;
 }
@@ -2013,19 +2016,39 @@ int kaos_get_moments_all(kaos_handle *h, int32_t tube, double *out, int32_t nq) 
 int kaos_get_counts(kaos_handle *h, int32_t tube, int64_t *out, int64_t nbins) {
   if (!h || !out || tube < 0 || tube >= h->ntubes) return KAOS_ERR_PARAM;
   const TubeD &T = h->th[tube];
-  CK(cudaStreamSynchronize(h->s));
+  const unsigned *src = h->acc.cnt + T.coff;
+  if (nbins != T.nq) {
+    if (nbins != (int64_t)T.nq * h->nv) return fail(h, KAOS_ERR_PARAM, "nbins must be nq or nq*nv");
+    if (!h->acc.hist) return fail(h, KAOS_ERR_STATE, "full histogram needs kaos_set_export(h, 1)");
+    src = h->acc.hist + T.hoff;
+  }
   if (nbins == T.nq) {
-    std::vector<unsigned> v(T.nq);
-    CK(cudaMemcpy(v.data(), h->acc.cnt + T.coff, T.nq * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    unsigned v[MAX_CELLS];
+    CK(cudaMemcpyAsync(v, src, nbins * sizeof(unsigned), cudaMemcpyDeviceToHost, h->s));
+    CK(cudaStreamSynchronize(h->s));
     for (int k = 0; k < T.nq; ++k) out[k] = v[k];
     return KAOS_OK;
   }
-  if (nbins != (int64_t)T.nq * h->nv) return fail(h, KAOS_ERR_PARAM, "nbins must be nq or nq*nv");
-  if (!h->acc.hist) return fail(h, KAOS_ERR_STATE, "full histogram needs kaos_set_export(h, 1)");
-  std::vector<unsigned> v(nbins);
-  CK(cudaMemcpy(v.data(), h->acc.hist + T.hoff, nbins * sizeof(unsigned), cudaMemcpyDeviceToHost));
-  for (int64_t k = 0; k < nbins; ++k) out[k] = v[k];
-  return KAOS_OK;
+  // the 32-bit counters come through two pinned buffers in turn, one being
+  // widened into the caller's array while the other fills
+  int64_t at[2] = {0, 0}, len[2] = {0, 0};
+  auto fetch = [&](int b, int64_t k0) -> int {
+    at[b] = k0;
+    len[b] = std::min<int64_t>(COUNT_STAGE, nbins - k0);
+    if (len[b] <= 0) return KAOS_OK;
+    CK(cudaMemcpyAsync(h->cnt_stage + b * COUNT_STAGE, src + k0, len[b] * sizeof(unsigned),
+                       cudaMemcpyDeviceToHost, h->s));
+    CK(cudaEventRecord(b ? h->ejoin : h->efork, h->s));
+    return KAOS_OK;
+  };
+  int rc = fetch(0, 0);
+  for (int b = 0; rc == KAOS_OK && len[b] > 0; b ^= 1) {
+    if ((rc = fetch(b ^ 1, at[b] + len[b]))) break;
+    CK(cudaEventSynchronize(b ? h->ejoin : h->efork));
+    const unsigned *v = h->cnt_stage + b * COUNT_STAGE;
+    for (int64_t k = 0; k < len[b]; ++k) out[at[b] + k] = v[k];
+  }
+  return rc;
 }
 
 int kaos_get_particles(kaos_handle *h, int32_t tube, double *q, double *vpar,
@@ -2033,17 +2056,19 @@ int kaos_get_particles(kaos_handle *h, int32_t tube, double *q, double *vpar,
                        int64_t n) {
   if (!h || tube < 0 || tube >= h->ntubes) return KAOS_ERR_PARAM;
   const TubeD &T = h->th[tube];
-  CK(cudaStreamSynchronize(h->s));
-  int64_t nl = 0;
-  CK(cudaMemcpy(&nl, h->d_nlive + tube, sizeof(int64_t), cudaMemcpyDeviceToHost));
-  if (nl == 0) {
-    if (n != 0) return fail(h, KAOS_ERR_PARAM, "n (%lld) must equal the ion count (0)", (long long)n);
-    return KAOS_OK;
-  }
+  const int64_t *st = nullptr;
+  int rc = tube_stat(h, &st);
+  if (rc) return rc;
+  const int64_t nl = st[(size_t)kaos_handle::ST_LIVE * h->ntubes + tube];
+  const int64_t live = live_ions(h, st, tube);
+  if (live != n)
+    return fail(h, KAOS_ERR_PARAM, "n (%lld) must equal the ion count (%lld)", (long long)n, (long long)live);
+  if (n == 0) return KAOS_OK;
   // the export runs on the device into the spare buffer set (no
   // allocation): q, V||, Vperp1, Vperp2 (FP64) and Qindk1 of the live ions
   // in particle order; the block counts and offsets use the packing's
-  // per-block arrays, the total the packing's new-count slot of the tube
+  // per-block arrays, the total the packing's new-count slot of the tube.
+  // Without a DEAD slot the count and the scan are left out.
   ExportArgs a{};
   a.ion = h->ion[h->cur];
   a.off = T.off;
@@ -2061,23 +2086,19 @@ int kaos_get_particles(kaos_handle *h, int32_t tube, double *q, double *vpar,
   a.v1 = vperp1 ? dq[2] : nullptr;
   a.v2 = vperp2 ? dq[3] : nullptr;
   a.qind = qind ? dqi : nullptr;
-  a.blkoff = (unsigned long long *)h->d_blkoff;
-  a.blkcnt = (unsigned *)h->d_blkcnt;
-  a.total = (unsigned long long *)(h->d_nlive_new + tube);
-  k_exp_count<<<a.nb, EXP_THREADS, 0, h->s>>>(a);
-  k_exp_scan<<<1, 1024, 0, h->s>>>(a);
+  if (live != nl) {
+    a.blkoff = (unsigned long long *)h->d_blkoff;
+    a.blkcnt = (unsigned *)h->d_blkcnt;
+    a.total = (unsigned long long *)(h->d_nlive_new + tube);
+    k_exp_count<<<a.nb, EXP_THREADS, 0, h->s>>>(a);
+    k_exp_scan<<<1, 1024, 0, h->s>>>(a);
+  }
   k_exp_write<<<a.nb, EXP_THREADS, 0, h->s>>>(a);
-  unsigned long long live = 0;
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&live, a.total, sizeof(live), cudaMemcpyDeviceToHost, h->s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->s);
-  if (e == cudaSuccess && (int64_t)live != n)
-    return fail(h, KAOS_ERR_PARAM, "n (%lld) must equal the ion count (%lld)", (long long)n, (long long)live);
   double *dst[4] = {q, vpar, vperp1, vperp2};
   for (int k = 0; k < 4 && e == cudaSuccess; ++k)
-    if (dst[k] && n) e = cudaMemcpyAsync(dst[k], dq[k], n * sizeof(double), cudaMemcpyDeviceToHost, h->s);
-  if (e == cudaSuccess && qind && n)
+    if (dst[k]) e = cudaMemcpyAsync(dst[k], dq[k], n * sizeof(double), cudaMemcpyDeviceToHost, h->s);
+  if (e == cudaSuccess && qind)
     e = cudaMemcpyAsync(qind, dqi, n * sizeof(int32_t), cudaMemcpyDeviceToHost, h->s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->s);
   if (e != cudaSuccess) return fail(h, KAOS_ERR_CUDA, "get_particles: %s", cudaGetErrorString(e));
@@ -2142,30 +2163,26 @@ int kaos_get_enas(kaos_handle *h, int32_t tube, double *x, double *y, double *z,
 int kaos_get_boundary(kaos_handle *h, int32_t tube, int64_t *lb_out,
                       int64_t *ub_out, int64_t *lb_in, int64_t *ub_in) {
   if (!h || tube < 0 || tube >= h->ntubes) return KAOS_ERR_PARAM;
-  CK(cudaStreamSynchronize(h->s));
-  unsigned long long v[4] = {0, 0, 0, 0};
-  CK(cudaMemcpy(&v[0], h->d_lb_out + tube, 8, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(&v[1], h->d_ub_out + tube, 8, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(&v[2], h->d_lb_in + tube, 8, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(&v[3], h->d_ub_in + tube, 8, cudaMemcpyDeviceToHost));
-  if (lb_out) *lb_out = (int64_t)v[0];
-  if (ub_out) *ub_out = (int64_t)v[1];
-  if (lb_in) *lb_in = (int64_t)v[2];
-  if (ub_in) *ub_in = (int64_t)v[3];
+  const int64_t *st = nullptr;
+  const int rc = tube_stat(h, &st);
+  if (rc) return rc;
+  const size_t n = h->ntubes;
+  if (lb_out) *lb_out = st[kaos_handle::ST_LB_OUT * n + tube];
+  if (ub_out) *ub_out = st[kaos_handle::ST_UB_OUT * n + tube];
+  if (lb_in) *lb_in = st[kaos_handle::ST_LB_IN * n + tube];
+  if (ub_in) *ub_in = st[kaos_handle::ST_UB_IN * n + tube];
   return KAOS_OK;
 }
 
 int kaos_get_boundary_ena(kaos_handle *h, int32_t tube, int64_t *lb_out,
                           int64_t *ub_out) {
   if (!h || tube < 0 || tube >= h->ntubes) return KAOS_ERR_PARAM;
-  unsigned long long v[2] = {0, 0};
-  if (h->d_lbe_out) {
-    CK(cudaStreamSynchronize(h->s));
-    CK(cudaMemcpy(&v[0], h->d_lbe_out + tube, 8, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&v[1], h->d_ube_out + tube, 8, cudaMemcpyDeviceToHost));
-  }
-  if (lb_out) *lb_out = (int64_t)v[0];
-  if (ub_out) *ub_out = (int64_t)v[1];
+  const int64_t *st = nullptr;
+  const int rc = tube_stat(h, &st);
+  if (rc) return rc;
+  const size_t n = h->ntubes;
+  if (lb_out) *lb_out = st[kaos_handle::ST_LBE * n + tube];
+  if (ub_out) *ub_out = st[kaos_handle::ST_UBE * n + tube];
   return KAOS_OK;
 }
 
@@ -2226,6 +2243,7 @@ void kaos_destroy(kaos_handle *h) {
   if (h->e1) cudaEventDestroy(h->e1);
   if (h->conv_host.stage) cudaFreeHost(h->conv_host.stage);
   if (h->cx_stat) cudaFreeHost(h->cx_stat);
+  if (h->cnt_stage) cudaFreeHost(h->cnt_stage);
   if (h->efork) cudaEventDestroy(h->efork);
   if (h->ejoin) cudaEventDestroy(h->ejoin);
   if (h->s2) cudaStreamDestroy(h->s2);

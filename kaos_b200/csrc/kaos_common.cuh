@@ -68,9 +68,16 @@ struct CellTables {
   const double *uM;       // ... and at the cell's midpoint in q
   const double *hK1, *hK2, *hc1, *hc2, *hiom0;  // wave-heating constants
   double *Te, *EAmag, *EG, *M0prev, *nuPoi;
-  double *mom;            // [KAOS_NMOMENTS][ncell_total]
+  double *mom;            // per tube [KAOS_NMOMENTS][nq], tubes one after another
   int64_t ncell_total;
 };
+
+// Row `which` of a tube's moment block (one contiguous block per tube, read
+// back by one plain copy).
+__host__ __device__ __forceinline__ double *mom_row(const CellTables &c, const TubeD &T,
+                                                    int which) {
+  return c.mom + (int64_t)T.coff * KAOS_NMOMENTS + (int64_t)which * T.nq;
+}
 
 // Ion particle arrays.  vpar (V||, FP64) serves both modes; FP64 mode adds
 // rho, z, v1, v2, aea, ag, qk4, mixed mode x, v12, ffl, fqk4.

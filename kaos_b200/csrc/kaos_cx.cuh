@@ -46,6 +46,7 @@ struct CxArgs {
   int *tube_active;          // per tube: listed cells
   int nqmax, mixed;
   int ncx;                   // selection chunks (all tubes)
+  int64_t *ndead;            // per tube: ion slots marked DEAD
   int rank, nranks;          // this rank's share of a split tube's conversions
   uint32_t *status;
 };
@@ -406,6 +407,7 @@ __device__ __forceinline__ void cx_convert_chunk(const CxArgs &a, int c, int t) 
   __syncthreads();
   unsigned tot = 0;
   for (int v = 0; v < CX_WARPS; ++v) tot += wconv[v];
+  if (threadIdx.x == 0 && tot) add64(a.ndead + t, tot);
   const int64_t slot0 = a.cxbase[c];
   for (int m = threadIdx.x; m < (int)tot; m += blockDim.x) {
     int v = 0;
@@ -650,8 +652,8 @@ __global__ void __launch_bounds__(256) k_ena_moments(const TubeD *tubes,
   for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < NC; g += nw) {
     const unsigned ne = acc.ecnt[g];
     double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // the rows KAOS_ENA_NQ ..
+    const TubeD &T = tubes[cell_tube[g]];
     if (ne) {
-      const TubeD &T = tubes[cell_tube[g]];
       const double ms = T.ms, w = T.nsnormfac / c.d3xC[g];
       M[0] = (double)ne * w;
       unsigned mp[VLANE], mq[VLANE], mph[VLANE], n = 0;
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(256) k_ena_moments(const TubeD *tubes,
       }
     }
     const double v = lane_value(M, lane);
-    if (lane < 9) c.mom[(KAOS_ENA_NQ + lane) * NC + g] = v;
+    if (lane < 9) mom_row(c, T, KAOS_ENA_NQ + lane)[g - T.coff] = v;
   }
 }
 

@@ -92,13 +92,13 @@ __global__ void k_fields(TubeArgs a) {
   // 363-536); k_cell_moments copies the same values at later master steps
   for (int Q = threadIdx.x; Q < nq; Q += blockDim.x) {
     const int64_t g = T.coff + Q;
-    c.mom[KAOS_EGMAG * c.ncell_total + g] = c.EG[g];
-    if (a.have_import || !a.eamb) c.mom[KAOS_EAMAG * c.ncell_total + g] = c.EAmag[g];
+    mom_row(c, T, KAOS_EGMAG)[Q] = c.EG[g];
+    if (a.have_import || !a.eamb) mom_row(c, T, KAOS_EAMAG)[Q] = c.EAmag[g];
   }
   if (a.have_import || !a.eamb) return;  // imported EAmag kept as is
   for (int Q = threadIdx.x; Q < nq; Q += blockDim.x) {
     M0f[Q] = a.momfilter ? filter_cell(M0p, nq, Q, a.fpM0) : M0p[Q];
-    c.mom[KAOS_M0FILT * c.ncell_total + T.coff + Q] = M0f[Q];  // M0FiltAvrgRT
+    mom_row(c, T, KAOS_M0FILT)[Q] = M0f[Q];  // M0FiltAvrgRT
   }
   __syncthreads();
   const double S = T.sgn;  // qGL(1) <= 0 ? +1 : -1
@@ -135,7 +135,7 @@ __global__ void k_fields(TubeArgs a) {
     double v = EP[Q];
     if (a.eambself && Q <= 2 && nq > 3 && M0p[Q] != 0.0 && a.eapressure) v = EP[3];
     c.EAmag[T.coff + Q] = 0.0 + v;  // EAInertial = 0 (EAINERTIALflag = 0)
-    c.mom[KAOS_EAMAG * c.ncell_total + T.coff + Q] = 0.0 + v;
+    mom_row(c, T, KAOS_EAMAG)[Q] = 0.0 + v;
   }
 }
 
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) k_cell_moments(TubeArgs a, const int *cel
     M[13] = M[KAOS_M0];  // M0prev, not a row (KAOS_M0FILT is the field kernel's)
     static_assert(KAOS_NQ == 10 && KAOS_EAMAG == 11 && KAOS_EGMAG == 12, "row order");
     const double v = lane_value(M, lane);
-    if (lane < 13) c.mom[lane * NC + g] = v;
+    if (lane < 13) mom_row(c, T, lane)[g - T.coff] = v;
     else if (lane == 13) c.M0prev[g] = v;
   }
 }
@@ -338,18 +338,15 @@ __global__ void k_collision_counts(TubeArgs a) {
   const TubeD T = a.tubes[blockIdx.x];
   const int nq = T.nq;
   const CellTables &c = a.ct;
-  const int64_t NC = c.ncell_total;
-  double *mom = c.mom;
   const uint32_t nn = a.dstep ? *a.dstep / (uint32_t)a.ndatfac + 1u : a.nn;
   double *f1p = sm, *f11 = sm + nq, *f12 = sm + 2 * nq, *f2p = sm + 3 * nq;
   double *s1p = sm + 4 * nq, *s11 = sm + 5 * nq, *s12 = sm + 6 * nq, *s2p = sm + 7 * nq;
   const int m1i = a.three_d ? KAOS_M1PERP1 : KAOS_M1PERP;
   for (int Q = threadIdx.x; Q < nq; Q += blockDim.x) {
-    const int64_t g = T.coff + Q;
-    s1p[Q] = mom[KAOS_M1PAR * NC + g];
-    s11[Q] = mom[m1i * NC + g];
-    s12[Q] = a.three_d ? mom[KAOS_M1PERP2 * NC + g] : 0.0;
-    s2p[Q] = mom[KAOS_M2PAR * NC + g];
+    s1p[Q] = mom_row(c, T, KAOS_M1PAR)[Q];
+    s11[Q] = mom_row(c, T, m1i)[Q];
+    s12[Q] = a.three_d ? mom_row(c, T, KAOS_M1PERP2)[Q] : 0.0;
+    s2p[Q] = mom_row(c, T, KAOS_M2PAR)[Q];
   }
   __syncthreads();
   for (int Q = threadIdx.x; Q < nq; Q += blockDim.x) {
@@ -361,7 +358,7 @@ __global__ void k_collision_counts(TubeArgs a) {
   __syncthreads();
   for (int Q = threadIdx.x; Q < nq; Q += blockDim.x) {
     const int64_t g = T.coff + Q;
-    const double M0 = mom[KAOS_M0 * NC + g];
+    const double M0 = mom_row(c, T, KAOS_M0)[Q];
     double sigma = 0.0, nu = 0.0;
     if (M0 != 0.0 && f2p[Q] != 0.0) {
       double E = (6.242e18) * (1e-3) * f2p[Q];
@@ -389,7 +386,7 @@ __global__ void k_collision_counts(TubeArgs a) {
       }
     }
     c.nuPoi[g] = nu;
-    mom[KAOS_NUPOI * NC + g] = nu;
+    mom_row(c, T, KAOS_NUPOI)[Q] = nu;
   }
 }
 
@@ -422,7 +419,13 @@ struct BcArgs {
   // k_bc_mark: the slot arrays marked DEAD (x: mixed precision only)
   int32_t *qind_w;
   double *x_w;
+  int64_t *ndead;  // per tube: ion slots marked DEAD (null: ENAs)
 };
+
+// Adds to an int64 counter.
+__device__ __forceinline__ void add64(int64_t *p, int64_t v) {
+  atomicAdd((unsigned long long *)p, (unsigned long long)v);
+}
 
 __device__ __forceinline__ bool keep_slot(int q) {
   return q != BELOW && q != ABOVE && q != DEAD;
@@ -505,6 +508,7 @@ __global__ void k_bc_mark(BcArgs a) {
     for (int k = 0; k < (int)(blockDim.x >> 5); ++k) { L += sl[k]; U += su[k]; }
     if (L) atomicAdd(a.lb_out + t, (unsigned long long)L);
     if (U) atomicAdd(a.ub_out + t, (unsigned long long)U);
+    if (L + U) add64(a.ndead + t, L + U);
   }
 }
 
@@ -535,7 +539,10 @@ __global__ void k_bc_scan(BcArgs a) {
     if (threadIdx.x == 0) base += tot;
     __syncthreads();
   }
-  if (threadIdx.x == 0) a.nlive[t] = base;
+  if (threadIdx.x == 0) {
+    a.nlive[t] = base;
+    if (a.ndead) a.ndead[t] = 0;
+  }
 }
 
 __global__ void k_bc_scatter(BcArgs a, const int64_t *nlive_old) {
@@ -951,23 +958,61 @@ __global__ void k_convect_many(ConvManyArgs m) {
 }
 
 // The new per-cell tables and descriptors of the moved entries, from one
-// staging copy: blockIdx.y = the move, blockIdx.x = the table.
-constexpr int CONV_NTAB = 28;
+// staging copy: blockIdx.y = the move, blockIdx.x = the table; one more block
+// per move derives the tables that kaos_create derives on the host (wave-
+// heating constants, quartic roots at the cell edges and midpoint).
+constexpr int CONV_RAW = 20;   // tables the caller gives
+constexpr int CONV_NTAB = 28;  // ... and the derived ones
 struct TableApplyArgs {
   double *dst[CONV_NTAB];  // the per-cell tables (concatenated over entries)
-  const double *stage;     // [move][table][nqmax]
+  const double *stage;     // [move][raw table][nqmax]
   const TubeD *td;         // per move: the new descriptor
   const int *tube;         // per move: the entry
   TubeD *tubes;
   int nqmax;
+  double h;                // time step
 };
+
+// Positive root u of q^2 u^4 + u/p - 1 = 0 by Newton from u = p, where the
+// (convex, increasing) function is not negative: monotone to the root.
+__device__ inline double quartic_root(double q, double p) {
+  double u = p;
+  for (int k = 0; k < 200; ++k) {
+    const double q2u3 = q * q * (u * u * u);
+    const double du = (fma(q2u3, u, u / p) - 1.0) / fma(4.0, q2u3, 1.0 / p);
+    u -= du;
+    if (!(fabs(du) > 1e-15 * u)) break;
+  }
+  return u;
+}
 
 __global__ void k_apply_tables(TableApplyArgs a) {
   const int p = blockIdx.y, k = blockIdx.x;
   const TubeD &T = a.td[p];
-  const double *src = a.stage + ((int64_t)p * CONV_NTAB + k) * a.nqmax;
-  for (int i = threadIdx.x; i < T.nq; i += blockDim.x) a.dst[k][T.coff + i] = src[i];
-  if (k == 0 && threadIdx.x == 0) a.tubes[a.tube[p]] = T;
+  const double *raw = a.stage + (int64_t)p * CONV_RAW * a.nqmax;
+  if (k < CONV_RAW) {
+    const double *src = raw + (int64_t)k * a.nqmax;
+    for (int i = threadIdx.x; i < T.nq; i += blockDim.x) a.dst[k][T.coff + i] = src[i];
+    if (k == 0 && threadIdx.x == 0) a.tubes[a.tube[p]] = T;
+    return;
+  }
+  auto in = [&](int table, int i) { return raw[(int64_t)table * a.nqmax + i]; };
+  for (int i = threadIdx.x; i < T.nq; i += blockDim.x) {
+    // (tables: 0 qGL, 1 qGH, 13 EtaLH, 14 XiPerp1, 15 XiPerp2, 16 S0, 17
+    // OmegaG0, 18 ChiPerp1, 19 ChiPerp2; derived 20 uL, 21 uH, 22 K1, 23 K2,
+    // 24 c1, 25 c2, 26 1/OmegaG0, 27 uM)
+    const int64_t g = T.coff + i;
+    const double ql = in(0, i), qh = in(1, i);
+    a.dst[20][g] = quartic_root(ql, T.pG);
+    a.dst[21][g] = quartic_root(qh, T.pG);
+    a.dst[27][g] = quartic_root(0.5 * (ql + qh), T.pG);
+    const double pre = (T.qs * T.qs / (2.0 * T.ms * T.ms)) * in(16, i) * in(13, i);
+    a.dst[22][g] = a.h * sqrt(pre * in(14, i) / PI);
+    a.dst[23][g] = a.h * sqrt(pre * in(15, i) / PI);
+    a.dst[24][g] = 0.5 * in(18, i);
+    a.dst[25][g] = 0.5 * in(19, i);
+    a.dst[26][g] = in(17, i) != 0.0 ? 1.0 / in(17, i) : 0.0;
+  }
 }
 
 }  // namespace kaos
@@ -1042,7 +1087,8 @@ __global__ void __launch_bounds__(EXP_THREADS) k_exp_write(ExportArgs a) {
   const int64_t beg = (int64_t)blockIdx.x * EXP_THREADS * EXP_ITEMS;
   __shared__ unsigned ws[EXP_THREADS / 32];
   const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned long long done = a.blkoff[blockIdx.x];
+  // no slot DEAD (blkoff null): every slot is written where it lies
+  unsigned long long done = a.blkoff ? a.blkoff[blockIdx.x] : (unsigned long long)beg;
   for (int k = 0; k < EXP_ITEMS; ++k) {
     const int64_t i = beg + k * EXP_THREADS + threadIdx.x;
     const int64_t j = a.off + i;
