@@ -91,6 +91,7 @@ struct kaos_handle {
   int ntubes = 0;
   int mixed = 0;
   int kick64 = 0;  // mixed push with the FP64 heating kick
+  double *d_kf = nullptr;  // PushArgs::kf
   int heat_lam = 0, heat_chi = 0;  // PushArgs: seen in any tube's tables so far
   int three_d = 1;
   int nv = 0;
@@ -330,6 +331,7 @@ PushArgs push_args(kaos_handle *h, bool run = false) {
   a.ff.eambsign = h->P.EAMBSIGNflag == 1;
   a.icr = h->P.ICRflag == 1;
   a.icrcoh = h->P.ICRCOHERENCEflag == 1;
+  a.kf = h->d_kf;
   a.heat_lam = h->heat_lam;
   a.heat_chi = h->heat_chi;
   a.status = h->d_status;
@@ -425,10 +427,13 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
   static const KFn k64[2][2] = {
       {k_push64<false, 256, 2, false, false>, k_push64<false, 256, 2, true, false>},
       {k_push64<true, 256, 2, false, false>, k_push64<true, 256, 2, true, false>}};
-  // FP64 runs: 80 registers (24 warps per SM) spill 32 B; the 124-register
-  // build (16 warps) spills nothing and is 5 % slower on 1e7 ions, 13 % on 1e5
-  static const KFn k64run[2] = {k_push64<false, 256, 3, false, true>,
-                                k_push64<true, 256, 3, false, true>};
+  // FP64 runs, [many items][three_d]: 64 registers (32 warps per SM, 120-150
+  // B of spills) where there are several waves of blocks, else 80 (24 warps,
+  // 60-80 B): ms per 20 steps 1e7 ions 6.20 / 6.35, 1e5 ions 0.143 / 0.127
+  // (124 registers, 16 warps, no spills: 6.75, 0.137)
+  static const KFn k64run[2][2] = {
+      {k_push64<false, 256, 3, false, true>, k_push64<true, 256, 3, false, true>},
+      {k_push64<false, 256, 4, false, true>, k_push64<true, 256, 4, false, true>}};
   // runs of steps: [FP64 heating kick][three_d].  64 registers (32 warps per
   // SM; 8 B of spills, 100 B with the FP64 kick) against 79 (24 warps, 0 and
   // 28 B), ms per 20 steps: 1e7 ions 2.78 / 2.81, FP64 kick 4.30 / 4.33, 1e8
@@ -439,7 +444,7 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
        k_push32<true, 256, 4, false, false, false, true>},
       {k_push32<false, 256, 4, false, false, true, true>,
        k_push32<true, 256, 4, false, false, true, true>}};
-  const KFn fn = run ? (h->mixed ? k32run[h->kick64][h->three_d] : k64run[h->three_d])
+  const KFn fn = run ? (h->mixed ? k32run[h->kick64][h->three_d] : k64run[a.chunk > 256][h->three_d])
                      : (h->mixed ? k32[h->kick64][ms][h->three_d][rs][ps] : k64[h->three_d][ps]);
   if (smem > 48 * 1024)
     CK(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -947,7 +952,8 @@ int sample_width(int kind) {
 
 __global__ void k_sample_rng(SampleArgs a) {
   double *kt = kf_tables();
-  if (a.kind == KAOS_SAMPLE_GAUSS64T) kf_tables_fill(kt);
+  if (a.kind == KAOS_SAMPLE_GAUSS64T)
+    for (int i = threadIdx.x; i <= KF_N; i += blockDim.x) kf_tables_make(kt, i);
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -1563,6 +1569,11 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
     if ((rc = dalloc(h, &I.qind, cap))) return rc;
     if (!h->three_d && (rc = dalloc(h, &I.vb, cap))) return rc;
     if ((rc = dalloc(h, &I.id, cap))) return rc;
+  }
+  if (p->ICRflag == 1 && (!h->mixed || h->kick64)) {  // the FP64 kick's tables
+    if ((rc = dalloc(h, &h->d_kf, 3 * (KF_N + 1)))) return rc;
+    k_kf_tables<<<1, 160>>>(h->d_kf);
+    CK(cudaGetLastError());
   }
   // global cell -> (tube, cell) map
   {

@@ -172,7 +172,27 @@ template <typename T> struct Geo {
   T ct, st, ir, q, isl, ell, er, ez;  // cos, sin, 1/r, q, 1/sqrt(ell), ell, e
 };
 
-__device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
+// FP64: FP32 seed (one MUFU) and one third-order step, e = 1 - x y^2,
+// y (1 + e/2 + 3 e^2/8): the seed's ~1e-7 leaves ~1e-21.  rsq_near forms e
+// with the rounding of x y (about 1 ulp); rsq carries that rounding along and
+// comes within ~0.5 ulp, closer than the library's rsqrt.  Both without the
+// library's range checks: for x well inside the FP32 range (squared radii in
+// m^2, ell in [1, 4], sin^2); not finite for x = 0 or inf.
+__device__ __forceinline__ double rsq_seed(double x) {
+  float s;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"((float)x));
+  return (double)s;
+}
+__device__ __forceinline__ double rsq_near(double x) {
+  const double y = rsq_seed(x);
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double rsq(double x) {
+  const double y = rsq_seed(x), t = x * y;
+  const double e = fma(-fma(x, y, -t), y, fma(-t, y, 1.0));
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
 // FP32: one MUFU operation, denormals flushed (the FP32 geometry of the
 // mixed push never comes near the denormal range).
 __device__ __forceinline__ float rsq(float x) {
@@ -181,17 +201,19 @@ __device__ __forceinline__ float rsq(float x) {
   return r;
 }
 
-template <typename T>
+// NEAR: the square roots by rsq_near (the k2 and k4 points, whose forces are
+// a small part of the step).
+template <bool NEAR = false, typename T>
 __device__ __forceinline__ Geo<T> geo(T rho, T z) {
   Geo<T> g;
   T r2 = rho * rho + z * z;
-  T ir = rsq(r2);
+  T ir = NEAR ? rsq_near(r2) : rsq(r2);
   g.ir = ir;
   g.ct = z * ir;
   g.st = rho * ir;
   g.q = T(RE * RE) * g.ct * (ir * ir);
   g.ell = T(1) + T(3) * g.ct * g.ct;
-  g.isl = rsq(g.ell);
+  g.isl = NEAR ? rsq_near(g.ell) : rsq(g.ell);
   g.er = T(3) * g.ct * g.st * g.isl;
   g.ez = (T(3) * g.ct * g.ct - T(1)) * g.isl;
   return g;

@@ -57,6 +57,7 @@ struct PushArgs {
   uint32_t *dstep_w;
   // Philox key schedule of the seed: key words of round r at rk[2r], rk[2r+1]
   uint32_t rk[20];
+  const double *kf;  // the FP64 kick's tables (heating, FP64 and K64 modes)
 };
 
 // Flush a block's per-cell Qindk1 counts into its selection-chunk row.
@@ -552,14 +553,19 @@ __device__ __forceinline__ double *kf_tables() {
   __shared__ double t[3 * (KF_N + 1)];
   return t;
 }
-__device__ __forceinline__ void kf_tables_fill(double *t) {
-  for (int i = threadIdx.x; i <= KF_N; i += blockDim.x) {
-    double sn, cs;
-    t[i] = exp2((double)i / KF_N);
-    sincospi((double)i / (KF_N / 2), &sn, &cs);
-    t[KF_N + 1 + 2 * i] = cs;
-    t[KF_N + 2 + 2 * i] = sn;
-  }
+__device__ __forceinline__ void kf_tables_make(double *t, int i) {
+  double sn, cs;
+  t[i] = exp2((double)i / KF_N);
+  sincospi((double)i / (KF_N / 2), &sn, &cs);
+  t[KF_N + 1 + 2 * i] = cs;
+  t[KF_N + 2 + 2 * i] = sn;
+}
+// ... from the handle's copy, made once (k_kf_tables)
+__device__ __forceinline__ void kf_tables_fill(double *t, const double *src) {
+  for (int i = threadIdx.x; i < 3 * (KF_N + 1); i += blockDim.x) t[i] = src[i];
+}
+__global__ void k_kf_tables(double *t) {
+  for (int i = threadIdx.x; i <= KF_N; i += blockDim.x) kf_tables_make(t, i);
 }
 
 // gauss2_64's Gaussian pair (the same Philox words, 53-bit uniforms) through
@@ -592,25 +598,31 @@ __device__ __forceinline__ void gauss2_64t(const uint32_t (&rk)[20], const doubl
 __device__ __forceinline__ void heat64t(const PushArgs &a, uint32_t step,
                                         const double *kt, const CellTables &ct,
                                         int64_t g, uint64_t id, double invsumds,
-                                        double ylim, double Om, double invOm,
-                                        double vabs, double &v1, double &v2) {
+                                        double ylim, double Om, double vabs, double &v1,
+                                        double &v2) {
   double arg = Om * vabs * invsumds;  // y
   if (!(arg <= ylim)) return;         // beyond the stochastic regime
-  const double lam = ct.lambdaPerp[g];
-  if (lam != 0.0) {
-    const double sk = (2.0 * PI) * invOm / lam;
-    const double S2 = sk * sk * fma(v1, v1, v2 * v2);  // Sig^2
-    if (S2 >= 1.0) arg = arg / (S2 * S2 * S2);
+  if (a.heat_lam) {
+    const double lam = ct.lambdaPerp[g];
+    if (lam != 0.0) {
+      const double sk = (2.0 * PI) / (Om * lam);
+      const double S2 = sk * sk * fma(v1, v1, v2 * v2);  // Sig^2
+      if (S2 >= 1.0) arg = arg / (S2 * S2 * S2);
+    }
   }
   if (!(arg > 1e-300)) return;
   double G1, G2;
   gauss2_64t(a.rk, kt, id, step, G1, G2);
   const double *p2 = kt;
-  const double c1 = ct.hc1[g], c2 = ct.hc2[g];
+  const double c1 = ct.hc1[g];
   const double lx = kf_log2(p2, Om * ct.hiom0[g]);
   const double b = 0.25 * kf_log2(p2, arg);
   const double e1 = kf_exp2(p2, fma(-c1, lx, b));
-  const double e2 = (c2 == c1) ? e1 : kf_exp2(p2, fma(-c2, lx, b));
+  double e2 = e1;
+  if (a.heat_chi) {
+    const double c2 = ct.hc2[g];
+    if (c2 != c1) e2 = kf_exp2(p2, fma(-c2, lx, b));
+  }
   v1 = fma(ct.hK1[g] * e1, G1, v1);
   v2 = fma(ct.hK2[g] * e2, G2, v2);
 }
@@ -736,6 +748,8 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
   // velocity-cell edges for the bin searches: shared memory serves the
   // threads' different addresses in parallel (constant memory serialises)
   __shared__ double VE1[MAXV + 1], VE2[MAXV + 1], VEP[MAXV + 1];
+  const bool kick = a.icr && !a.icrcoh;  // ordered by the item loop's barrier
+  if (kick) kf_tables_fill(kf_tables(), a.kf);
   if (bin || !THREE_D) load_vgrid_smem(c_vg.e1, c_vg.e2, c_vg.epar, VE1, VE2, VEP);
   // one work item per block, or a persistent grid striding over the items
   for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
@@ -758,6 +772,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
   const double ipG = 1.0 / T.pG, invsumds = 1.0 / T.sumdsICR;
   const double qs_ms = T.qs / T.ms;
   const double c_invOm = T.ms / (T.qs * MDIP);
+  const double ylim = (2.0 * PI / a.h) * (2.0 * PI / a.h);
   for (int64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
     const int64_t j = T.off + i;
     int qprev = I.qind[j];
@@ -813,18 +828,23 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     if (a.icr && qi >= 0) {
       const double sl = g1.ell * g1.isl;
       const double Om = qs_ms * MDIP * sl * (g1.ir * g1.ir * g1.ir);
-      const double r = 1.0 / g1.ir;
-      const double invOm = c_invOm * (r * r * r) * g1.isl;
-      const HeatC<double> hc = heat_consts<double>(a.ct, (int64_t)T.coff + qi);
-      heat<double>(a, step, hc, pid, invsumds, Om, invOm, fabs(vpar), v1n, v2n);
+      if (kick) {
+        heat64t(a, step, kf_tables(), a.ct, (int64_t)T.coff + qi, pid, invsumds, ylim, Om,
+                fabs(vpar), v1n, v2n);
+      } else {
+        const double r = 1.0 / g1.ir;
+        const double invOm = c_invOm * (r * r * r) * g1.isl;
+        const HeatC<double> hc = heat_consts<double>(a.ct, (int64_t)T.coff + qi);
+        heat<double>(a, step, hc, pid, invsumds, Om, invOm, fabs(vpar), v1n, v2n);
+      }
     }
     // ---- k2: half step along V_R (KineticUpdateB) -----------------------
     const double VRr = vpar * g1.er, VRz = vpar * g1.ez;
-    const Geo<double> g2 = geo(fma(hh, VRr, rho), fma(hh, VRz, z));
+    const Geo<double> g2 = geo<true>(fma(hh, VRr, rho), fma(hh, VRz, z));
     const double a2 = apar(g2, vp2, aea, ag, a.ff);
     // ---- k4: x + h V_R + h^2/2 A1 (KineticUpdateC) ----------------------
     const double A1r = a1 * g1.er, A1z = a1 * g1.ez;
-    const Geo<double> g4 = geo(rho + h * VRr + hsq2 * A1r, z + h * VRz + hsq2 * A1z);
+    const Geo<double> g4 = geo<true>(rho + h * VRr + hsq2 * A1r, z + h * VRz + hsq2 * A1z);
     const double a4 = apar(g4, vp2, aea, ag, a.ff);
     if (last && a.write_qk4) {
       I.qk4[j] = g4.q;
@@ -844,18 +864,18 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     const double xz = z + h6 * (VRz + 2.0 * Vk2z + 2.0 * Vk2z + Vk4z);
     // ---- re-projection onto the tube: q of the RK point, p reset to pG --
     const double r2 = xr * xr + xz * xz;
-    const double ir = rsqrt(r2);
+    const double ir = rsq(r2);
     const double qN = (RE * RE) * (xz * ir) * (ir * ir);
     const double u = quartic_newton(qN, ipG, r2 * ir * (1.0 / RE), 2);
     const double s2 = u * ipG;                 // sin^2(theta)
-    const double st = s2 * rsqrt(s2);
+    const double st = s2 * rsq(s2);
     const double ctn = qN * u * u;
     const double rr = u * RE;
     double rhoN = rr * st, zN = rr * ctn;
     if (fabs(rhoN) < 1e-6) rhoN = 0.0;
     if (fabs(zN) < 1e-6) zN = 0.0;
     // ---- V|| along the new field direction ------------------------------
-    const double isl = rsqrt(1.0 + 3.0 * ctn * ctn);
+    const double isl = rsq(1.0 + 3.0 * ctn * ctn);
     const double vparN = (3.0 * ctn * st * isl) * VNr + ((3.0 * ctn * ctn - 1.0) * isl) * VNz;
     if (RUN && !last) {
       rho = rhoN;
@@ -1026,7 +1046,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   double *VE2 = VE1 + (MAXV + 1), *VEP = VE2 + (MAXV + 1);
   VBinTab *VTS = (VBinTab *)(VEP + (MAXV + 1));
   VBinTab &VT1 = VTS[0], &VT2 = VTS[1], &VTP = VTS[2];
-  if (K64) kf_tables_fill(kf_tables());  // ordered by the item loop's barrier
+  if (K64 && a.icr) kf_tables_fill(kf_tables(), a.kf);  // ordered by the item loop's barrier
   if (bin || !THREE_D) {
     load_vgrid_smem(c_vg.e1, c_vg.e2, c_vg.epar, VE1, VE2, VEP);
     build_vbin_tab(VTP, c_vg.epar, c_vg.npar);
@@ -1358,11 +1378,11 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
         double ir = (double)rcpa((float)r);
         ir = ir * fma(-r, ir, 2.0);
         const double Om = qs_ms64 * MDIP * (ell64 * yl) * (ir * ir * ir);
-        const double invOm = c_invOm64 * (r * r * r) * yl;
         if (!a.icrcoh) {
           heat64t(a, step, kf_tables(), a.ct, (int64_t)T.coff + qi, pid, invsumds64,
-                  ylim64, Om, invOm, fabs(vpar), v1n, v2n);
-        } else {  // coherent branch: the FP64 path's own code
+                  ylim64, Om, fabs(vpar), v1n, v2n);
+        } else {  // coherent branch: the general form
+          const double invOm = c_invOm64 * (r * r * r) * yl;
           const HeatC<double> hc = heat_consts<double>(a.ct, (int64_t)T.coff + qi);
           heat<double>(a, step, hc, pid, invsumds64, Om, invOm, fabs(vpar), v1n, v2n);
         }
