@@ -233,7 +233,8 @@ __device__ __forceinline__ T apar(const Geo<T> &g, T vperp2, T aea, T ag,
   bool south = (g.ct <= T(0));  // the sign of q = RE^2 cos(theta) / r^2
   if (f.mirror) {
     // |mu dBds/ms| = Vperp^2/2 * 3 ct/r (2 + st^2/ell)/sqrt(ell)
-    T m = T(1.5) * vperp2 * fabs(g.ct) * g.ir * (T(2) + g.st * g.st * g.isl * g.isl) * g.isl;
+    const T sl = g.st * g.isl;
+    T m = T(1.5) * vperp2 * fabs(g.ct) * (g.ir * g.isl) * (T(2) + sl * sl);
     a += south ? -m : m;
   }
   if (f.grav) a += south ? fabs(ag) : -fabs(ag);

@@ -737,7 +737,8 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
   const int nqmax = a.nqs;
   double *E = sm, *Cc = sm + nqmax + 1;
   unsigned *HC = (unsigned *)(Cc + nqmax);
-  const double h = a.h, hh = 0.5 * a.h, h6 = a.h / 6.0, hsq2 = 0.5 * a.h * a.h;
+  const double h = a.h, hh = 0.5 * a.h, h6 = a.h / 6.0, hsq2 = 0.5 * a.h * a.h,
+               hh6 = a.h * h6;
   const uint32_t step0 = a.dstep ? *a.dstep : a.step;
   const unsigned nsub = RUN ? a.nsub : 1u;
   if (a.dstep_w && blockIdx.x == 0 && threadIdx.x == 0) *a.dstep_w = step0 + nsub - 1u;
@@ -856,17 +857,19 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     const double A2r = a2 * g2.er, A2z = a2 * g2.ez;
     const double A4r = a4 * g4.er, A4z = a4 * g4.ez;
     // ---- RK combination (k3 = k2) ---------------------------------------
-    const double VNr = VRr + h6 * (A1r + 2.0 * A2r + 2.0 * A2r + A4r);
-    const double VNz = VRz + h6 * (A1z + 2.0 * A2z + 2.0 * A2z + A4z);
-    const double Vk2r = VRr + hh * A1r, Vk2z = VRz + hh * A1z;
-    const double Vk4r = VRr + h * A2r, Vk4z = VRz + h * A2z;
-    const double xr = rho + h6 * (VRr + 2.0 * Vk2r + 2.0 * Vk2r + Vk4r);
-    const double xz = z + h6 * (VRz + 2.0 * Vk2z + 2.0 * Vk2z + Vk4z);
+    const double VNr = fma(h6, fma(4.0, A2r, A1r) + A4r, VRr);
+    const double VNz = fma(h6, fma(4.0, A2z, A1z) + A4z, VRz);
+    // h/6 (V_R + 4 (V_R + h/2 A1) + (V_R + h A2)) = h V_R + h^2/6 (2 A1 + A2),
+    // summed before it meets the position (one rounding there)
+    const double xr = rho + fma(h, VRr, hh6 * fma(2.0, A1r, A2r));
+    const double xz = z + fma(h, VRz, hh6 * fma(2.0, A1z, A2z));
     // ---- re-projection onto the tube: q of the RK point, p reset to pG --
-    const double r2 = xr * xr + xz * xz;
+    const double r2 = fma(xr, xr, xz * xz);
     const double ir = rsq(r2);
     const double qN = (RE * RE) * (xz * ir) * (ir * ir);
-    const double u = quartic_newton(qN, ipG, r2 * ir * (1.0 / RE), 2);
+    // (the Runge-Kutta point leaves the field line by the square of the step
+    // over the radius, 1e-12 for 10 m: the chord step only settles rounding)
+    const double u = quartic_newton_chord(qN, ipG, r2 * ir * (1.0 / RE));
     const double s2 = u * ipG;                 // sin^2(theta)
     const double st = s2 * rsq(s2);
     const double ctn = qN * u * u;
