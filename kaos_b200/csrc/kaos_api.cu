@@ -110,10 +110,12 @@ struct kaos_handle {
   // behind it; kaos_step copies the block to stat_host as its last work, so
   // the getters of counts and boundary fluxes need no copy.  (Pageable: a
   // pinned block saves ~5 us a step call and costs 1 ms at creation.)
-  enum { ST_LIVE, ST_DEAD, ST_ENA, ST_LB_OUT, ST_UB_OUT, ST_LB_IN, ST_UB_IN, ST_LBE, ST_UBE, NSTAT };
+  // The first ST_ZEROED rows start every master step from zero.
+  enum { ST_LB_OUT, ST_UB_OUT, ST_LB_IN, ST_UB_IN, ST_LBE, ST_UBE, ST_ZEROED,
+         ST_LIVE = ST_ZEROED, ST_DEAD, ST_ENA, NSTAT };
   int64_t *d_stat = nullptr, *stat_host = nullptr, *d_ndead = nullptr;
   std::vector<int64_t> stat_store;
-  size_t stat_bytes = 0;
+  size_t stat_bytes = 0, zero_bytes = 0;
   unsigned *cnt_stage = nullptr;  // kaos_get_counts: 2 x COUNT_STAGE, pinned
   int stat_ok = 0;  // stat_host holds the device's values
   // device
@@ -469,7 +471,7 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
 
 int zero_accum(kaos_handle *h) {
   const int64_t nc = h->ncell;
-  CK(cudaMemsetAsync(h->acc_base, 0, (size_t)h->acc_len * sizeof(unsigned), h->s));
+  CK(cudaMemsetAsync(h->acc_base, 0, h->zero_bytes, h->s));
   if (h->export_on && h->acc.hist)
     CK(cudaMemsetAsync(h->acc.hist, 0, nc * (int64_t)h->nv * sizeof(unsigned), h->s));
   return KAOS_OK;
@@ -577,6 +579,7 @@ int reduce_accum(kaos_handle *h) {
 }
 
 CxArgs cx_args(kaos_handle *h);
+InjArgs inject_args(kaos_handle *h, int ub);
 
 // Blocks of the per-cell moment kernels: a warp per cell, eight per block, at
 // most four resident blocks per SM striding over the cells (each block builds
@@ -585,16 +588,17 @@ int moment_grid(kaos_handle *h) {
   return (int)std::min<int64_t>(ceil_div(h->ncell, 8), 4 * (int64_t)sm_count(h));
 }
 
-int launch_moments(kaos_handle *h, uint32_t nn) {
+// commit: 0, or 1 / 2 to commit the lower / upper boundary's injection too.
+int launch_moments(kaos_handle *h, uint32_t nn, int commit = 0) {
   TubeArgs ta = tube_args(h, nn);
-  k_cell_moments<<<moment_grid(h), 256, 0, h->s>>>(ta, h->d_cell_tube);
+  k_cell_moments<<<moment_grid(h), 256, 0, h->s>>>(ta, h->d_cell_tube,
+                                                   inject_args(h, commit == 2), commit);
   h->launches++;
   if (ta.qexchange) {
     size_t smem = (size_t)8 * max_nq(h) * sizeof(double);
     k_collision_counts<<<h->ntubes, 256, smem, h->s>>>(ta);
     // the cells that will convert ions until the next master step
-    CK(cudaMemsetAsync(h->d_cx_nlist, 0, sizeof(int), h->s));
-    CK(cudaMemsetAsync(h->d_tube_active, 0, h->ntubes * sizeof(int), h->s));
+    CK(cudaMemsetAsync(h->d_cx_nlist, 0, (1 + h->ntubes) * sizeof(int), h->s));
     k_cx_list<<<(int)((h->ncell + 255) / 256), 256, 0, h->s>>>(cx_args(h), h->d_cell_tube,
                                                              h->ncell);
     h->launches += 2;
@@ -603,7 +607,9 @@ int launch_moments(kaos_handle *h, uint32_t nn) {
     CK(cudaMemcpyAsync(h->cx_stat + 1, h->d_nena, h->ntubes * sizeof(int64_t),
                        cudaMemcpyDeviceToHost, h->s));
     h->cx_stat_pending = 1;
-    if (nn > 1) {  // ENA statistics from the second master step on
+    // ENA statistics from the second master step on (an idle interval has no
+    // ENA, its last master step had none either: the rows are zero already)
+    if (nn > 1 && !h->cx_idle) {
       k_ena_moments<<<moment_grid(h), 256, 0, h->s>>>(h->d_tubes, h->d_cell_tube, h->ct, h->acc);
       h->launches++;
     }
@@ -612,12 +618,13 @@ int launch_moments(kaos_handle *h, uint32_t nn) {
   return KAOS_OK;
 }
 
-int launch_fields(kaos_handle *h, int te_update) {
+// The first step's fields: from the first moments, or gravity only beside an
+// imported EAmag.
+int launch_first_fields(kaos_handle *h) {
   TubeArgs ta = tube_args(h, 0);
-  ta.te_update = te_update;
-  ta.have_import = 0;
-  size_t smem = (size_t)3 * max_nq(h) * sizeof(double);
-  k_fields<<<h->ntubes, 256, smem, h->s>>>(ta);
+  ta.have_import = h->have_import;
+  k_master_begin<<<h->ntubes, 256, (size_t)3 * max_nq(h) * sizeof(double), h->s>>>(ta, BcArgs{},
+                                                                                 nullptr);
   h->launches++;
   CK(cudaGetLastError());
   return KAOS_OK;
@@ -713,25 +720,33 @@ void bc_after(kaos_handle *h, int compact) {
   for (int t = 0; t < h->ntubes; ++t) h->bc_bound[t] += inject_max(h, t);
 }
 
-int launch_boundary(kaos_handle *h, int compact) {
-  if (!compact) {
-    BcArgs b{};
-    b.tubes = h->d_tubes;
-    b.blk_tube = h->d_blk_tube;
-    b.blk_start = h->d_blk_start;
-    b.chunk = PUSH_THREADS * PUSH_ITEMS;
-    b.nlive = h->d_nlive;
-    b.lb_out = h->d_lb_out;
-    b.ub_out = h->d_ub_out;
-    b.qind_w = h->ion[h->cur].qind;
-    b.x_w = h->mixed ? h->ion[h->cur].x : nullptr;
-    b.ndead = h->d_ndead;
-    CK(cudaMemsetAsync(h->d_lb_out, 0, 4 * h->ntubes * sizeof(int64_t), h->s));  // all four
-    k_bc_mark<<<h->nblk, BC_THREADS, 0, h->s>>>(b);
-    h->launches++;
-    CK(cudaGetLastError());
-    return KAOS_OK;
-  }
+// The fields of a master step (and, unless it packs, its removal) in one
+// launch; the step number of a replayed graph advances here.
+int launch_master_begin(kaos_handle *h, int compact) {
+  TubeArgs ta = tube_args(h, 0);
+  ta.te_update = 1;
+  ta.have_import = 0;
+  BcArgs b{};
+  b.tubes = h->d_tubes;
+  b.blk_tube = h->d_blk_tube;
+  b.blk_start = h->d_blk_start;
+  b.chunk = PUSH_THREADS * PUSH_ITEMS;
+  b.nlive = h->d_nlive;
+  b.lb_out = h->d_lb_out;
+  b.ub_out = h->d_ub_out;
+  b.ndead = h->d_ndead;
+  b.qind_w = h->ion[h->cur].qind;
+  b.x_w = h->mixed ? h->ion[h->cur].x : nullptr;
+  const size_t smem = (size_t)3 * max_nq(h) * sizeof(double);
+  k_master_begin<<<h->ntubes + (compact ? 0 : h->nblk), 256, smem, h->s>>>(
+      ta, b, h->capturing ? h->d_step : nullptr);
+  h->launches++;
+  CK(cudaGetLastError());
+  return KAOS_OK;
+}
+
+// The order-preserving packing of the ion arrays.
+int launch_pack(kaos_handle *h) {
   BcArgs b{};
   b.tubes = h->d_tubes;
   b.blk_tube = h->d_blk_tube;
@@ -746,7 +761,6 @@ int launch_boundary(kaos_handle *h, int compact) {
   b.ub_out = h->d_ub_out;
   b.fields = ion_fields(h, h->cur, 1 - h->cur);
   b.ndead = h->d_ndead;
-  CK(cudaMemsetAsync(h->d_lb_out, 0, 4 * h->ntubes * sizeof(int64_t), h->s));  // all four
   BcArgs bc = b;
   bc.nlive = h->d_nlive;  // count reads the live counts
   k_bc_count<<<h->nblk, BC_THREADS, 0, h->s>>>(bc);
@@ -759,7 +773,7 @@ int launch_boundary(kaos_handle *h, int compact) {
   return KAOS_OK;  // the caller swaps the buffer sets (bc_after)
 }
 
-int launch_inject(kaos_handle *h, int ub) {
+InjArgs inject_args(kaos_handle *h, int ub) {
   InjArgs a{};
   a.tubes = h->d_tubes;
   a.ct = h->ct;
@@ -784,14 +798,23 @@ int launch_inject(kaos_handle *h, int ub) {
     a.cx_stride = max_nq(h);
     a.cx_chunk = CX_CHUNK;
   }
+  return a;
+}
+
+int launch_inject(kaos_handle *h, int ub, cudaStream_t s) {
   // blocks per tube: enough for the largest injection, at most 64
   int64_t kmax = 0;
   for (const TubeD &T : h->th)
     kmax = std::max(kmax, (int64_t)std::llrint(ub ? T.nsnormCUB : T.nsnormCLB));
   const int bx = (int)std::min<int64_t>(64, std::max<int64_t>(1, (kmax + 255) / 256));
-  k_inject<<<dim3(bx, h->ntubes), 256, 0, h->s>>>(a);
-  k_inject_commit<<<(h->ntubes + 127) / 128, 128, 0, h->s>>>(a, h->ntubes);
-  h->launches += 2;
+  k_inject<<<dim3(bx, h->ntubes), 256, 0, s>>>(inject_args(h, ub));
+  h->launches++;
+  CK(cudaGetLastError());
+  return KAOS_OK;
+}
+int commit_inject(kaos_handle *h, int ub) {
+  k_inject_commit<<<(h->ntubes + 127) / 128, 128, 0, h->s>>>(inject_args(h, ub), h->ntubes);
+  h->launches++;
   CK(cudaGetLastError());
   return KAOS_OK;
 }
@@ -861,11 +884,8 @@ int launch_cx(kaos_handle *h) {
   return KAOS_OK;
 }
 
-// The ENA push on the side stream, forked from the main stream here; the
-// caller joins it (join_push_ena) after the ion push.
+// The ENA push, on the side stream.
 int launch_push_ena(kaos_handle *h, int bin) {
-  CK(cudaEventRecord(h->efork, h->s));
-  CK(cudaStreamWaitEvent(h->s2, h->efork, 0));
   EnaArgs a{};
   a.acc = h->acc;
   a.bin = bin;
@@ -888,11 +908,18 @@ int launch_push_ena(kaos_handle *h, int bin) {
                ena_push_smem(max_nq(h), h->ntubes), h->s2>>>(a);
   h->launches++;
   CK(cudaGetLastError());
-  CK(cudaEventRecord(h->ejoin, h->s2));
   return KAOS_OK;
 }
 
-int join_push_ena(kaos_handle *h) {
+// Work on the side stream, beside the ion push: everything launched on the
+// main stream so far comes before it, what follows the join comes after it.
+int side_fork(kaos_handle *h) {
+  CK(cudaEventRecord(h->efork, h->s));
+  CK(cudaStreamWaitEvent(h->s2, h->efork, 0));
+  return KAOS_OK;
+}
+int side_join(kaos_handle *h) {
+  CK(cudaEventRecord(h->ejoin, h->s2));
   CK(cudaStreamWaitEvent(h->s, h->ejoin, 0));
   return KAOS_OK;
 }
@@ -920,7 +947,6 @@ int launch_boundary_ena(kaos_handle *h) {
   F.f[F.n++] = Field{A.qind, B.qind, 4}; F.f[F.n++] = Field{A.vb, B.vb, 4};
   F.f[F.n++] = Field{A.id, B.id, 8};
   b.fields = F;
-  CK(cudaMemsetAsync(h->d_lbe_out, 0, 2 * h->ntubes * sizeof(int64_t), h->s));  // both
   BcArgs bc = b;
   bc.nlive = h->d_nena;
   k_bc_count<<<h->neblk, BC_THREADS, 0, h->s>>>(bc);
@@ -1004,7 +1030,9 @@ int step_once(kaos_handle *h) {
   const bool next_master = is_master(h, n + 1);
   const bool qx = h->P.QEXCHANGEflag == 1;
   int rc;
-  if (h->capturing) {  // d_step: n - 1 -> n for the kernels of this step
+  // d_step: n - 1 -> n for the kernels of this step (a master step advances
+  // it in its first kernel)
+  if (h->capturing && !is_master(h, n)) {
     k_next_step<<<1, 1, 0, h->s>>>(h->d_step);
     h->launches++;
   }
@@ -1018,14 +1046,7 @@ int step_once(kaos_handle *h) {
     a.write_qind = 1;
     if ((rc = launch_push(h, a))) return rc;
     if ((rc = reduce_accum(h)) || (rc = launch_moments(h, 1))) return rc;
-    if (!h->have_import) {
-      if ((rc = launch_fields(h, 0))) return rc;
-    } else {
-      TubeArgs ta = tube_args(h, 0);
-      ta.have_import = 1;  // gravity only, EAmag kept
-      k_fields<<<h->ntubes, 256, (size_t)3 * max_nq(h) * sizeof(double), h->s>>>(ta);
-      h->launches++;
-    }
+    if ((rc = launch_first_fields(h))) return rc;
     PushArgs p = push_args(h);
     p.step = (uint32_t)n;
     p.prologue = 1;  // interpolate at q0 (qk4 holds q0 after loading)
@@ -1049,13 +1070,18 @@ int step_once(kaos_handle *h) {
   if (cx_on && (rc = launch_cx(h))) return rc;
   if (qx && !cx_on && master)
     CK(cudaMemsetAsync(h->d_cxc, 0, (size_t)h->ncx * max_nq(h) * sizeof(unsigned), h->s));
+  // the injection of one boundary runs beside the push (it fills slots behind
+  // the live ions, whose count advances after both); with both boundaries
+  // open the second needs the first's count, so they follow the push
+  const bool lb = master && h->P.LBCONDITIONflag == 1, ub = master && h->P.UBCONDITIONflag == 1;
+  const bool beside = lb != ub;
   if (master) {
-    const int compact = bc_decide(h, n);
-    if ((rc = launch_boundary(h, compact))) return rc;
-    bc_after(h, compact);
-    if (qx && (rc = launch_boundary_ena(h))) return rc;
-    if ((rc = launch_fields(h, 1))) return rc;
     if ((rc = zero_accum(h))) return rc;
+    const int compact = bc_decide(h, n);
+    if (compact && (rc = launch_pack(h))) return rc;
+    if ((rc = launch_master_begin(h, compact))) return rc;
+    bc_after(h, compact);
+    if (cx_on && (rc = launch_boundary_ena(h))) return rc;
   }
   PushArgs p = push_args(h);
   p.step = (uint32_t)n;
@@ -1066,13 +1092,18 @@ int step_once(kaos_handle *h) {
   p.write_qk4 = next_master || cx_rec;
   if (cx_rec) p.cxc = h->d_cxc;
   // the ENA push (independent of the ions) runs beside the ion push
+  if ((cx_on || beside) && (rc = side_fork(h))) return rc;
   if (cx_on && (rc = launch_push_ena(h, master))) return rc;
+  if (beside && (rc = launch_inject(h, ub, h->s2))) return rc;
   if ((rc = launch_push(h, p))) return rc;
-  if (cx_on && (rc = join_push_ena(h))) return rc;
+  if ((cx_on || beside) && (rc = side_join(h))) return rc;
   if (master) {
-    if (h->P.LBCONDITIONflag == 1 && (rc = launch_inject(h, 0))) return rc;
-    if (h->P.UBCONDITIONflag == 1 && (rc = launch_inject(h, 1))) return rc;
-    if ((rc = reduce_accum(h)) || (rc = launch_moments(h, nn))) return rc;
+    if (lb && ub)
+      for (int k = 0; k < 2; ++k)
+        if ((rc = launch_inject(h, k, h->s)) || (rc = commit_inject(h, k))) return rc;
+    if ((rc = reduce_accum(h)) ||
+        (rc = launch_moments(h, nn, beside ? 1 + (int)ub : 0)))
+      return rc;
   }
   h->n = n;
   return KAOS_OK;
@@ -1228,7 +1259,7 @@ int graph_steps(kaos_handle *h, int g) {
       if (is_master(h, m)) {  // launch_boundary / launch_boundary_ena swaps
         bc_after(h, bc_decide(h, m));
         if (h->P.QEXCHANGEflag == 1) {
-          h->ecur = 1 - h->ecur;
+          if (!h->cx_idle) h->ecur = 1 - h->ecur;
           h->cx_stat_pending = 1;  // the graph copied the next interval's stat
         }
       }
@@ -1455,13 +1486,16 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
   if ((rc = dalloc(h, &c.mom, coff * KAOS_NMOMENTS))) return rc;
   h->host_cells = {qGL, qGH, qGC};
   // binning accumulators, ions then ENAs, in one block (one reduction
-  // covers them all when a tube is split across ranks)
+  // covers them all when a tube is split across ranks), behind them the
+  // per-tube counts: one memset clears what a master step starts from zero
   {
     const size_t nc = (size_t)coff;
     const size_t ion_n = nc * (1 + vg.npar + vg.n1 + std::max(vg.n2, 1));
     const size_t ena_n = p->QEXCHANGEflag == 1 ? nc * (1 + 3 * (size_t)MAXV) : 0;
+    const size_t acc_n = (ion_n + ena_n + 1) & ~(size_t)1;  // the counts 8-byte aligned
+    const size_t n = (size_t)kaos_handle::NSTAT * ntubes;
     unsigned *base = nullptr;
-    if ((rc = dalloc(h, &base, ion_n + ena_n))) return rc;
+    if ((rc = dalloc(h, &base, acc_n + 2 * (n + 1)))) return rc;
     h->acc_base = base;
     h->acc_len = (int64_t)(ion_n + ena_n);
     h->acc.cnt = base;
@@ -1474,6 +1508,24 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
       h->acc.emq = h->acc.emp + nc * MAXV;
       h->acc.emph = h->acc.emq + nc * MAXV;
     }
+    h->d_stat = (int64_t *)(base + acc_n);
+    h->zero_bytes = acc_n * sizeof(unsigned) + (size_t)kaos_handle::ST_ZEROED * ntubes * sizeof(int64_t);
+    h->stat_bytes = (n + 1) * sizeof(int64_t);
+    h->stat_store.assign(n + 1, 0);
+    h->stat_host = h->stat_store.data();
+    auto row = [&](int k) { return h->d_stat + (size_t)k * ntubes; };
+    h->d_nlive = row(kaos_handle::ST_LIVE);
+    h->d_ndead = row(kaos_handle::ST_DEAD);
+    h->d_lb_out = (unsigned long long *)row(kaos_handle::ST_LB_OUT);
+    h->d_ub_out = (unsigned long long *)row(kaos_handle::ST_UB_OUT);
+    h->d_lb_in = (unsigned long long *)row(kaos_handle::ST_LB_IN);
+    h->d_ub_in = (unsigned long long *)row(kaos_handle::ST_UB_IN);
+    if (p->QEXCHANGEflag == 1) {
+      h->d_nena = row(kaos_handle::ST_ENA);
+      h->d_lbe_out = (unsigned long long *)row(kaos_handle::ST_LBE);
+      h->d_ube_out = (unsigned long long *)row(kaos_handle::ST_UBE);
+    }
+    h->d_status = (uint32_t *)(h->d_stat + n);
   }
   // tube descriptors and the static block -> (tube, chunk) map
   std::vector<int> bt;
@@ -1516,26 +1568,6 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
     if ((rc = work_map(h->wmap[m], CHUNKS[m]))) return rc;
   h->rmap = h->wmap[0];
   if (h->rmap.chunk != run_chunk(h) && (rc = work_map(h->rmap, run_chunk(h)))) return rc;
-  {
-    const size_t n = (size_t)kaos_handle::NSTAT * ntubes;
-    h->stat_bytes = (n + 1) * sizeof(int64_t);
-    if ((rc = dalloc(h, &h->d_stat, n + 1))) return rc;
-    h->stat_store.assign(n + 1, 0);
-    h->stat_host = h->stat_store.data();
-    auto row = [&](int k) { return h->d_stat + (size_t)k * ntubes; };
-    h->d_nlive = row(kaos_handle::ST_LIVE);
-    h->d_ndead = row(kaos_handle::ST_DEAD);
-    h->d_lb_out = (unsigned long long *)row(kaos_handle::ST_LB_OUT);
-    h->d_ub_out = (unsigned long long *)row(kaos_handle::ST_UB_OUT);
-    h->d_lb_in = (unsigned long long *)row(kaos_handle::ST_LB_IN);
-    h->d_ub_in = (unsigned long long *)row(kaos_handle::ST_UB_IN);
-    if (p->QEXCHANGEflag == 1) {
-      h->d_nena = row(kaos_handle::ST_ENA);
-      h->d_lbe_out = (unsigned long long *)row(kaos_handle::ST_LBE);
-      h->d_ube_out = (unsigned long long *)row(kaos_handle::ST_UBE);
-    }
-    h->d_status = (uint32_t *)(h->d_stat + n);
-  }
   if ((rc = dalloc(h, &h->d_nlive_new, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_next_id, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_blkcnt, bt.size()))) return rc;
@@ -1639,13 +1671,13 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
         (rc = dalloc(h, &h->d_cxend, (size_t)h->ncell)) ||
         (rc = dalloc(h, &h->d_tube_done, (size_t)ntubes)) ||
         (rc = dalloc(h, &h->d_cx_list, (size_t)h->ncell)) ||
-        (rc = dalloc(h, &h->d_cx_nlist, 1)) ||
+        (rc = dalloc(h, &h->d_cx_nlist, 1 + (size_t)ntubes)) ||
         (rc = dalloc(h, &h->d_cx_chunks, cxt.size())) ||
         (rc = dalloc(h, &h->d_cx_nchunk, 2)) ||
-        (rc = dalloc(h, &h->d_tube_active, (size_t)ntubes)) ||
         (rc = dalloc(h, &h->d_cxc, cxt.size() * (size_t)max_nq(h))) ||
         (rc = dalloc(h, &h->d_cxo, cxt.size() * (size_t)max_nq(h))))
       return rc;
+    h->d_tube_active = h->d_cx_nlist + 1;
     CK(cudaMallocHost((void **)&h->cx_stat, (size_t)(ntubes + 1) * sizeof(int64_t)));
     memset(h->cx_stat, 0, (size_t)(ntubes + 1) * sizeof(int64_t));
   }
@@ -1655,11 +1687,11 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
     const std::pair<const void *, size_t> big[] = {
         {(const void *)k_collision_counts, 8 * nq * sizeof(double)},
         {(const void *)k_cx_convert, cx_convert_smem((int)nq)},
-        {(const void *)k_fields, 3 * nq * sizeof(double)},
+        {(const void *)k_master_begin, 3 * nq * sizeof(double)},
         {(const void *)k_push_ena, ena_push_smem((int)nq, ntubes)},
         {(const void *)k_load, (nq + 1) * sizeof(double)}};
-    for (const auto &b : big)
-      if (b.second > 48 * 1024)
+    for (const auto &b : big)  // (static shared memory counts towards the 48 KB)
+      if (b.second > 44 * 1024)
         CK(cudaFuncSetAttribute(b.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.second));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cx_convert, 256,

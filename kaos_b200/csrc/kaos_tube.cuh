@@ -67,10 +67,10 @@ __device__ double filter_cell(const double *in, int nq, int Q, int Pt) {
 // ---------------------------------------------------------------------------
 // AmbipolarEfieldSub pressure term (_8_7_AmbipolarEfield.f90:611-1299),
 // GravfieldSub (_8_7_2_Gravfield.f90:57-65) and the Te update of
-// KineticSolverSub (_8_KineticSolver.f90:69-89).  One block per tube.
-__global__ void k_fields(TubeArgs a) {
+// KineticSolverSub (_8_KineticSolver.f90:69-89).  One block per tube t.
+__device__ __forceinline__ void tube_fields(const TubeArgs &a, int t) {
   extern __shared__ double sm[];
-  const TubeD T = a.tubes[blockIdx.x];
+  const TubeD T = a.tubes[t];
   const int nq = T.nq;
   double *M0p = sm, *M0f = sm + nq, *EP = sm + 2 * nq;
   const CellTables &c = a.ct;
@@ -281,10 +281,62 @@ __device__ __forceinline__ double lane_value(const double (&M)[N], int lane) {
 }
 
 // ---------------------------------------------------------------------------
-// Moments of one master step, a grid striding over the cells.
-__global__ void __launch_bounds__(256) k_cell_moments(TubeArgs a, const int *cell_tube) {
+// Lower / upper boundary injection on a master step (BoundaryConditionsSub
+// :743-809, KineticSolverBSub _8_0_0_2_KineticSolverB.f90:195-793,
+// MBVelocityDistributionSub _6_1_MBVelocityDistribution.f90:29-120).
+struct InjArgs {
+  const TubeD *tubes;
+  CellTables ct;
+  Accum acc;
+  Ions ion;
+  int64_t *nlive;
+  uint64_t *next_id;
+  unsigned long long *n_in;  // per tube injected count (LB, UB)
+  int mixed, ub, bin, exporting;
+  int flux, stat;  // FLUXINJECTIONflag, STATICINJECTIONflag
+  double ms, qs;
+  uint64_t seed;
+  uint32_t *status;
+  unsigned *cxc;             // charge exchange on: selection-chunk counts
+  const int *tube_cx0;
+  int cx_stride, cx_chunk;
+};
+
+// Ions injected by one tube at this master step (capacity-clamped).
+__device__ __forceinline__ int64_t inject_count(const InjArgs &a, const TubeD &T,
+                                                int64_t nl) {
+  const int64_t k = (int64_t)llrint(a.ub ? T.nsnormCUB : T.nsnormCLB);
+  if (k <= 0) return 0;
+  return nl + k > T.cap ? max(T.cap - nl, (int64_t)0) : k;
+}
+
+// After k_inject: advance the live counts and ids (one thread per tube) and
+// flag a capacity clamp.
+__device__ __forceinline__ void inject_commit(const InjArgs &a, int t) {
+  const TubeD &T = a.tubes[t];
+  const int64_t nl = a.nlive[t];
+  const int64_t want = (int64_t)llrint(a.ub ? T.nsnormCUB : T.nsnormCLB);
+  const int64_t k = inject_count(a, T, nl);
+  if (want > 0 && k < want) atomicOr(a.status, ST_CAP);
+  a.nlive[t] = nl + k;
+  a.next_id[t] += (uint64_t)k;
+  a.n_in[t] = (unsigned long long)k;
+}
+
+__global__ void k_inject_commit(InjArgs a, int ntubes) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < ntubes) inject_commit(a, t);
+}
+
+// ---------------------------------------------------------------------------
+// Moments of one master step, a grid striding over the cells; the first block
+// also commits the step's injection (nothing here reads the live counts).
+__global__ void __launch_bounds__(256) k_cell_moments(TubeArgs a, const int *cell_tube,
+                                                      InjArgs inj, int commit) {
   __shared__ BinCentres C;
   load_centres(C, c_vg);
+  if (commit && blockIdx.x == 0)
+    for (int t = threadIdx.x; t < a.ntubes; t += blockDim.x) inject_commit(inj, t);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const CellTables &c = a.ct;
@@ -416,7 +468,7 @@ struct BcArgs {
   unsigned long long *lb_out, *ub_out;  // per tube escape counts
   Fields fields;
   int ena;  // 1: operate on the ENA segments (tube.eoff) instead of ions
-  // k_bc_mark: the slot arrays marked DEAD (x: mixed precision only)
+  // mark_escaped: the slot arrays marked DEAD (x: mixed precision only)
   int32_t *qind_w;
   double *x_w;
   int64_t *ndead;  // per tube: ion slots marked DEAD (null: ENAs)
@@ -467,11 +519,11 @@ __global__ void k_bc_count(BcArgs a) {
 // counted and marked DEAD in place, as slots converted to ENAs are; the
 // live ions keep their order, and a later compaction removes every DEAD
 // slot at once.
-__global__ void k_bc_mark(BcArgs a) {
-  const int t = a.blk_tube[blockIdx.x];
+__device__ __forceinline__ void mark_escaped(const BcArgs &a, int blk) {
+  const int t = a.blk_tube[blk];
   const TubeD &T = a.tubes[t];
   const int64_t nl = a.nlive[t];
-  const int64_t beg = a.blk_start[blockIdx.x];
+  const int64_t beg = a.blk_start[blk];
   const int64_t end = min(beg + (int64_t)a.chunk, nl);
   int lb = 0, ub = 0;
   // the indices of a tile of MARK_IT slots per thread are loaded before any
@@ -509,6 +561,20 @@ __global__ void k_bc_mark(BcArgs a) {
     if (L) atomicAdd(a.lb_out + t, (unsigned long long)L);
     if (U) atomicAdd(a.ub_out + t, (unsigned long long)U);
     if (L + U) add64(a.ndead + t, L + U);
+  }
+}
+
+// The start of a master step in one launch: the first ntubes blocks compute
+// the fields of their tube (from the moments of the last master step), the
+// others mark the escaped ions (none when the step packs instead).  The two
+// touch different data and each is a few microseconds of latency: together
+// they cost the longer one.  step: advanced by one (graph replay).
+__global__ void __launch_bounds__(256) k_master_begin(TubeArgs f, BcArgs b, uint32_t *step) {
+  if ((int)blockIdx.x < f.ntubes) {
+    if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1u;
+    tube_fields(f, blockIdx.x);
+  } else {
+    mark_escaped(b, blockIdx.x - f.ntubes);
   }
 }
 
@@ -586,35 +652,7 @@ __global__ void k_bc_scatter(BcArgs a, const int64_t *nlive_old) {
 }
 
 // ---------------------------------------------------------------------------
-// Lower / upper boundary injection on a master step (BoundaryConditionsSub
-// :743-809, KineticSolverBSub _8_0_0_2_KineticSolverB.f90:195-793,
-// MBVelocityDistributionSub _6_1_MBVelocityDistribution.f90:29-120).
-struct InjArgs {
-  const TubeD *tubes;
-  CellTables ct;
-  Accum acc;
-  Ions ion;
-  int64_t *nlive;
-  uint64_t *next_id;
-  unsigned long long *n_in;  // per tube injected count (LB, UB)
-  int mixed, ub, bin, exporting;
-  int flux, stat;  // FLUXINJECTIONflag, STATICINJECTIONflag
-  double ms, qs;
-  uint64_t seed;
-  uint32_t *status;
-  unsigned *cxc;             // charge exchange on: selection-chunk counts
-  const int *tube_cx0;
-  int cx_stride, cx_chunk;
-};
-
-// Ions injected by one tube at this master step (capacity-clamped).
-__device__ __forceinline__ int64_t inject_count(const InjArgs &a, const TubeD &T,
-                                                int64_t nl) {
-  const int64_t k = (int64_t)llrint(a.ub ? T.nsnormCUB : T.nsnormCLB);
-  if (k <= 0) return 0;
-  return nl + k > T.cap ? max(T.cap - nl, (int64_t)0) : k;
-}
-
+// Injection (InjArgs above).
 // grid (blocks per tube, tubes): every block of a tube reads the same live
 // count; k_inject_commit advances it afterwards
 __global__ void k_inject(InjArgs a) {
@@ -683,21 +721,6 @@ __global__ void k_inject(InjArgs a) {
       agg_inc(a.cxc, (int64_t)(a.tube_cx0[t] + (int)((nl + i) / a.cx_chunk)) * a.cx_stride + Q);
     if (a.bin) accumulate(a.acc, T, Q, b1, d3 ? b2 : 0, bp, a.exporting);
   }
-}
-
-// After k_inject: advance the live counts and ids (one thread per tube) and
-// flag a capacity clamp.
-__global__ void k_inject_commit(InjArgs a, int ntubes) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntubes) return;
-  const TubeD &T = a.tubes[t];
-  const int64_t nl = a.nlive[t];
-  const int64_t want = (int64_t)llrint(a.ub ? T.nsnormCUB : T.nsnormCLB);
-  const int64_t k = inject_count(a, T, nl);
-  if (want > 0 && k < want) atomicOr(a.status, ST_CAP);
-  a.nlive[t] = nl + k;
-  a.next_id[t] += (uint64_t)k;
-  a.n_in[t] = (unsigned long long)k;
 }
 
 // ---------------------------------------------------------------------------
