@@ -365,8 +365,9 @@ int kaos_set_graph(kaos_handle *h, int32_t on);
  * autotuner, which is on by default: before the first step after step 1 it
  * times the push of every candidate on a copy of the ion state and keeps
  * the fastest, then the master-step variant's budget alone.  Runs of steps
- * (kaos_step) have a shape of their own.  Results do not depend on the
- * shape.  No reference counterpart (the reference has one MPI rank per core,
+ * (kaos_step) have a shape of their own, and a handle of fewer than 2^21
+ * slots takes items of 256 ions while no shape is set here (reported as 1024,
+ * the smallest that can be set).  Results do not depend on the shape.  No reference counterpart (the reference has one MPI rank per core,
  * _8_KineticSolver.f90:43-44). */
 int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode);
 

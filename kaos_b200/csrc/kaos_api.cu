@@ -92,6 +92,7 @@ struct kaos_handle {
   int mixed = 0;
   int kick64 = 0;  // mixed push with the FP64 heating kick
   double *d_kf = nullptr;  // PushArgs::kf
+  VBins *d_vbins = nullptr;  // PushArgs::vbins
   int heat_lam = 0, heat_chi = 0;  // PushArgs: seen in any tube's tables so far
   int three_d = 1;
   int nv = 0;
@@ -216,6 +217,7 @@ struct kaos_handle {
   int wsel = 1;          // chosen map (CHUNKS[wsel] ions per item)
   int persistent = 0;    // persistent grid striding over the items
   int tune_pending = 1;  // autotune before the next step
+  int forced = 0;        // shape given by kaos_set_launch
   int regsel = 0;        // mixed push register budget: 0 = 64, 1 = 80, 2 = 72
   int regsel_master = 0; // the same for the master-step variant of the push
   int nsm = 0;
@@ -313,7 +315,11 @@ void note_heating(kaos_handle *h, const kaos_tube_c &T) {
 PushArgs push_args(kaos_handle *h, bool run = false) {
   PushArgs a{};
   a.tubes = h->d_tubes;
-  const kaos_handle::WorkMap &M = run ? h->rmap : h->wmap[h->wsel];
+  // a small handle's single steps are latency, not throughput: one ion per
+  // thread in items of 256 unless the caller chose a shape (3e5 ions, every
+  // step a master step: push 28 us with items of 1024, 15 with 256)
+  const bool fine = run || (h->rmap.chunk == 256 && !h->forced);
+  const kaos_handle::WorkMap &M = fine ? h->rmap : h->wmap[h->wsel];
   a.blk_tube = M.d_tube;
   a.blk_start = M.d_start;
   a.nitems = M.n;
@@ -334,6 +340,7 @@ PushArgs push_args(kaos_handle *h, bool run = false) {
   a.icr = h->P.ICRflag == 1;
   a.icrcoh = h->P.ICRCOHERENCEflag == 1;
   a.kf = h->d_kf;
+  a.vbins = h->d_vbins;
   a.heat_lam = h->heat_lam;
   a.heat_chi = h->heat_chi;
   a.status = h->d_status;
@@ -1155,8 +1162,10 @@ int autotune(kaos_handle *h) {
   CK(cudaEventCreate(&e1));
   float best = 1e30f;
   int bw = h->wsel, bp = h->persistent, br = h->regsel;
-  for (int m = 0; m < NCHUNKS; ++m)
-    for (int pm = 0; pm < 2; ++pm)
+  // (items of 256 ions, push_args: only the register budget is left to choose)
+  const bool fine = h->rmap.chunk == 256 && !h->forced;
+  for (int m = 0; m < (fine ? 1 : NCHUNKS); ++m)
+    for (int pm = 0; pm < (fine ? 1 : 2); ++pm)
     for (int rs = 0; rs < (h->mixed ? 3 : 1); ++rs) {
       h->wsel = m;
       h->persistent = pm;
@@ -1602,6 +1611,9 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
     if (!h->three_d && (rc = dalloc(h, &I.vb, cap))) return rc;
     if ((rc = dalloc(h, &I.id, cap))) return rc;
   }
+  if ((rc = dalloc(h, &h->d_vbins, 1))) return rc;
+  k_vbins<<<1, 256>>>(h->d_vbins, h->vg);
+  CK(cudaGetLastError());
   if (p->ICRflag == 1 && (!h->mixed || h->kick64)) {  // the FP64 kick's tables
     if ((rc = dalloc(h, &h->d_kf, 3 * (KF_N + 1)))) return rc;
     k_kf_tables<<<1, 160>>>(h->d_kf);
@@ -1849,6 +1861,7 @@ int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode) {
   if (!h) return KAOS_ERR_PARAM;
   if (chunk == 0 || mode < 0) {
     h->tune_pending = 1;
+    h->forced = 0;
     return KAOS_OK;
   }
   int m = -1;
@@ -1857,6 +1870,7 @@ int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode) {
   if (m < 0 || mode > 31 || ((mode >> 1) & 3) == 3)
     return fail(h, KAOS_ERR_PARAM, "launch: chunk must be 1024, 2048 or 4096; mode bits "
                 "1-2 in 0..2, bits 3-4 in 0..3");
+  h->forced = 1;
   h->wsel = m;
   h->persistent = mode & 1;
   h->regsel = (mode >> 1) & 3;

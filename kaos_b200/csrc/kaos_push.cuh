@@ -17,6 +17,8 @@ namespace kaos {
 
 __constant__ VGridC c_vg;
 
+struct VBins;  // the velocity-bin tables, below
+
 struct PushArgs {
   const TubeD *tubes;
   const int *blk_tube;       // work item -> tube
@@ -57,6 +59,7 @@ struct PushArgs {
   uint32_t *dstep_w;
   // Philox key schedule of the seed: key words of round r at rk[2r], rk[2r+1]
   uint32_t rk[20];
+  const VBins *vbins;  // the ion grid's edges and bin tables
   const double *kf;  // the FP64 kick's tables (heating, FP64 and K64 modes)
 };
 
@@ -193,12 +196,14 @@ __device__ __forceinline__ void bin_win_flush(const Accum &acc, const TubeD &T,
 // field values).
 __device__ __forceinline__ int centre_segment(const double *E, const double *C,
                                               int nq, double s, int guess) {
-  if (s < E[0] || s > E[nq]) return -1;
-  if (s <= C[0]) return 0;
-  if (s >= C[nq - 1]) return nq;
   int k = min(max(guess, 1), nq - 1);
   while (k > 1 && s <= C[k - 1]) --k;
   while (k < nq - 1 && s > C[k]) ++k;
+  // between inner centres nothing is left to check: C[0] < s < C[nq - 1]
+  if (k > 1 && k < nq - 1) return k;
+  if (s < E[0] || s > E[nq]) return -1;
+  if (s <= C[0]) return 0;
+  if (s >= C[nq - 1]) return nq;
   return k;
 }
 
@@ -410,7 +415,8 @@ __device__ __forceinline__ void field_prologue32(const ForceFlags &ff,
                                                  float qk, int guess, float qm,
                                                  float &aea, float &ag) {
   const int nq = T.nq;
-  const int k = centre_segment(E, C, nq, T.sgn * (double)qk, guess);
+  const double s = T.sgn * (double)qk;
+  const int k = centre_segment(E, C, nq, s, guess);
   if (k < 0) return;
   float2 f;
   if (k == 0) {
@@ -418,8 +424,9 @@ __device__ __forceinline__ void field_prologue32(const ForceFlags &ff,
   } else if (k == nq) {
     f = FE[nq - 1];
   } else {
-    const double x1 = T.sgn * C[k - 1], x2 = T.sgn * C[k];
-    const float frac = (float)((double)qk - x1) * rcpa((float)(x2 - x1));
+    // (the orientation's sign cancels: the differences are exact negatives)
+    const double x1 = C[k - 1];
+    const float frac = (float)(s - x1) * rcpa((float)(C[k] - x1));
     const float2 y1 = FE[k - 1], y2 = FE[k];
     f.x = fmaf(frac, y2.x - y1.x, y1.x);
     f.y = fmaf(frac, y2.y - y1.y, y1.y);
@@ -435,31 +442,53 @@ __device__ __forceinline__ void field_prologue32(const ForceFlags &ff,
 }
 
 // Velocity-bin search of the mixed push from a lookup table: VTAB uniform
-// slots over the axis hold the bin of each slot's left end, and a short walk
-// over the FP64 edges finishes the search.
-// The walk establishes both edge conditions of vbin (v <= e[b+1], and
-// v > e[b] unless b = 0) in FP64, so the result equals vbin's on the FP64
-// edges whatever the table holds.
+// slots over the axis hold a bin at or below every value of the slot, and a
+// short walk up the FP64 edges finishes the search with vbin's result (v <=
+// e[b+1], and v > e[b] unless b = 0).
 constexpr int VTAB = 256;
 struct VBinTab {
   double e0, iw;             // first edge, VTAB / (last edge - first edge)
-  unsigned char t[VTAB];     // bin at each slot's left end (n <= 128)
+  unsigned char t[VTAB];     // a bin at or below every value of the slot (n <= 128)
 };
-// Dynamic shared memory of the mixed push's bin searches: alignment slack,
-// three FP64 edge arrays and three lookup tables.
-constexpr size_t BINS_SMEM_BYTES = 16 + 3 * (MAXV + 1) * sizeof(double) + 3 * sizeof(VBinTab);
+// The three axes' FP64 edges and tables, made once per handle (k_vbins) and
+// copied to shared memory by the kernels that search.
+struct VBins {
+  double e1[MAXV + 1], e2[MAXV + 1], ep[MAXV + 1];
+  VBinTab t1, t2, tp;
+  double pad;                // a multiple of 16 bytes
+};
+static_assert(sizeof(VBins) % 16 == 0, "copied 16 bytes at a time");
+// Dynamic shared memory of the mixed push's bin searches (with alignment
+// slack).
+constexpr size_t BINS_SMEM_BYTES = 16 + sizeof(VBins);
 
-// All threads of the block; edges e[0..n] in shared memory already visible,
-// and the caller synchronises before the table is used.
-__device__ __forceinline__ void build_vbin_tab(VBinTab &T, const double *e, int n) {
-  if (threadIdx.x == 0) {
+// Slot k of the table over edges e[0..n], and its scale: the bin of a point a
+// millionth of a slot left of the slot's left end, so that the rounding of a
+// value's slot never puts it below.
+__device__ __forceinline__ void make_vbin_slot(VBinTab &T, const double *e, int n, int k) {
+  if (k == 0) {
     T.e0 = e[0];
     T.iw = (double)VTAB / (e[n] - e[0]);
   }
-  for (int k = threadIdx.x; k < VTAB; k += blockDim.x) {
-    const double v = e[0] + (e[n] - e[0]) * ((double)k / (double)VTAB);
-    T.t[k] = (unsigned char)max(vbin(e, n, v), 0);
+  const double v = e[0] + (e[n] - e[0]) * (((double)k - 1e-6) / (double)VTAB);
+  T.t[k] = (unsigned char)max(vbin(e, n, v), 0);
+}
+// All threads of the block; edges in shared memory already visible, and the
+// caller synchronises before the table is used.
+__device__ __forceinline__ void build_vbin_tab(VBinTab &T, const double *e, int n) {
+  for (int k = threadIdx.x; k < VTAB; k += blockDim.x) make_vbin_slot(T, e, n, k);
+}
+
+__global__ void k_vbins(VBins *B, VGridC vg) {
+  for (int k = threadIdx.x; k <= MAXV; k += blockDim.x) {
+    B->e1[k] = vg.e1[k];
+    B->e2[k] = vg.e2[k];
+    B->ep[k] = vg.epar[k];
   }
+  __syncthreads();
+  build_vbin_tab(B->tp, B->ep, vg.npar);
+  build_vbin_tab(B->t1, B->e1, vg.n1);
+  if (vg.three_d) build_vbin_tab(B->t2, B->e2, vg.n2);
 }
 
 __device__ __forceinline__ int vbin_tab(const VBinTab &T, const double *e, int n,
@@ -468,15 +497,10 @@ __device__ __forceinline__ int vbin_tab(const VBinTab &T, const double *e, int n
   // slot floor((v - e0) iw): round-to-nearest of (v - e0) iw - 1/2 read from
   // the low word of its sum with 1.5 * 2^52 (no conversion instruction)
   const double sl = fma(v - T.e0, T.iw, -0.5) + 6755399441055744.0;
-  const int s = min(max((int)__double2loint(sl), 0), VTAB - 1);
-  int b = T.t[s];
-  // one predicated step up settles almost every value (the table gives the
-  // bin of the slot's left end); the loops finish the rare rest exactly
-  b += (b < n - 1 && v > e[b + 1]) ? 1 : 0;
-  if (__builtin_expect((b > 0 && v <= e[b]) || (b < n - 1 && v > e[b + 1]), 0)) {
-    while (b > 0 && v <= e[b]) --b;
-    while (b < n - 1 && v > e[b + 1]) ++b;
-  }
+  int b = T.t[min(max((int)__double2loint(sl), 0), VTAB - 1)];
+  // up to the bin that holds v: v <= e[b + 1], and v > e[b] unless b = 0
+  // (the table's bin is at or below; one step settles almost every value)
+  while (b < n - 1 && v > e[b + 1]) ++b;
   return b;
 }
 
@@ -746,12 +770,15 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
   Ions I = a.ion;
   TubeD T;
   int tcur = -1;
-  // velocity-cell edges for the bin searches: shared memory serves the
-  // threads' different addresses in parallel (constant memory serialises)
-  __shared__ double VE1[MAXV + 1], VE2[MAXV + 1], VEP[MAXV + 1];
+  // velocity-cell edges and tables for the bin searches (ordered by the item
+  // loop's first barrier)
+  __shared__ __align__(16) VBins VB;
+  if (bin || !THREE_D)
+    for (int k = threadIdx.x; k < (int)(sizeof(VBins) / 16); k += NT)
+      ((uint4 *)&VB)[k] = ((const uint4 *)a.vbins)[k];
+  const double *VE1 = VB.e1, *VEP = VB.ep;
   const bool kick = a.icr && !a.icrcoh;  // ordered by the item loop's barrier
   if (kick) kf_tables_fill(kf_tables(), a.kf);
-  if (bin || !THREE_D) load_vgrid_smem(c_vg.e1, c_vg.e2, c_vg.epar, VE1, VE2, VEP);
   // one work item per block, or a persistent grid striding over the items
   for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
   const int t = a.blk_tube[item];
@@ -805,14 +832,14 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
       }
     } else if (THREE_D) {
       if (bin) {
-        bp = vbin(VEP, c_vg.npar, vpar);
-        b1 = vbin(VE1, c_vg.n1, v1);
-        b2 = vbin(VE2, c_vg.n2, v2);
+        bp = vbin_tab(VB.tp, VB.ep, c_vg.npar, vpar);
+        b1 = vbin_tab(VB.t1, VB.e1, c_vg.n1, v1);
+        b2 = vbin_tab(VB.t2, VB.e2, c_vg.n2, v2);
       }
     } else {  // 2D grid: an out-of-grid speed keeps its previous bin
       const int old = I.vb[j];
-      const int np_ = vbin(VEP, c_vg.npar, vpar);
-      const int n1_ = vbin(VE1, c_vg.n1, sqrt(vp2));
+      const int np_ = vbin_tab(VB.tp, VB.ep, c_vg.npar, vpar);
+      const int n1_ = vbin_tab(VB.t1, VB.e1, c_vg.n1, sqrt(vp2));
       bp = np_ >= 0 ? np_ : (old & 0xffff) - 1;
       b1 = n1_ >= 0 ? n1_ : (old >> 16) - 1;
       const int nw = ((b1 + 1) << 16) | (bp + 1);
@@ -907,8 +934,8 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     if (!RUN && a.cxc && qi >= 0) atomicAdd(&HC[qi], 1u);
     if (RUN && !THREE_D) {
       const int old = I.vb[j];
-      bp = in_vp ? vbin(VEP, c_vg.npar, l_vp) : (old & 0xffff) - 1;
-      b1 = in_s ? vbin(VE1, c_vg.n1, l_s) : (old >> 16) - 1;
+      bp = in_vp ? vbin_tab(VB.tp, VB.ep, c_vg.npar, l_vp) : (old & 0xffff) - 1;
+      b1 = in_s ? vbin_tab(VB.t1, VB.e1, c_vg.n1, l_s) : (old >> 16) - 1;
       const int nw = ((b1 + 1) << 16) | (bp + 1);
       if (nw != old) I.vb[j] = nw;
     }
@@ -1045,18 +1072,13 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   // generic loads)
   const char *tail = RUN ? (const char *)Cc : (const char *)(HC + nqmax + bin_win_size());
   const size_t ve_off = ((size_t)(tail - (const char *)sm) + 15) & ~(size_t)15;
-  double *VE1 = (double *)((char *)sm + ve_off);
-  double *VE2 = VE1 + (MAXV + 1), *VEP = VE2 + (MAXV + 1);
-  VBinTab *VTS = (VBinTab *)(VEP + (MAXV + 1));
-  VBinTab &VT1 = VTS[0], &VT2 = VTS[1], &VTP = VTS[2];
+  VBins &VB = *(VBins *)((char *)sm + ve_off);
+  const double *VE1 = VB.e1, *VE2 = VB.e2, *VEP = VB.ep;
+  const VBinTab &VT1 = VB.t1, &VT2 = VB.t2, &VTP = VB.tp;
   if (K64 && a.icr) kf_tables_fill(kf_tables(), a.kf);  // ordered by the item loop's barrier
-  if (bin || !THREE_D) {
-    load_vgrid_smem(c_vg.e1, c_vg.e2, c_vg.epar, VE1, VE2, VEP);
-    build_vbin_tab(VTP, c_vg.epar, c_vg.npar);
-    build_vbin_tab(VT1, c_vg.e1, c_vg.n1);
-    if (THREE_D) build_vbin_tab(VT2, c_vg.e2, c_vg.n2);
-    // the first barrier of the item loop orders the tables before any use
-  }
+  if (bin || !THREE_D)  // the first barrier of the item loop orders them before any use
+    for (int k = threadIdx.x; k < (int)(sizeof(VBins) / 16); k += NT)
+      ((uint4 *)&VB)[k] = ((const uint4 *)a.vbins)[k];
   // one work item per block, or a persistent grid striding over the items
   for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
   const int t = a.blk_tube[item];
