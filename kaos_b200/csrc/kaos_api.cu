@@ -46,7 +46,7 @@ static size_t ena_push_smem(int nq, int ntubes) {
   return (size_t)(nq + 1) * sizeof(double) + (size_t)(ntubes + 1) * sizeof(int);
 }
 // k_cx_convert's shared memory: conversions still owed per cell, per-warp
-// per-cell counts (8 warps), the chunk's Qindk1
+// per-cell counts (CX_WARPS warps), the chunk's Qindk1
 static size_t cx_convert_smem(int nq) {
   return ((size_t)cx_qs_word(nq) + CX_CHUNK) * sizeof(unsigned);
 }
@@ -417,44 +417,53 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
   const bool run = a.nsub > 1;  // ordinary steps only, one item per block
   const int rs = h->mixed && !run ? (ms ? h->regsel_master : h->regsel) : 0;
   const int ps = run ? 0 : h->persistent;
-  // kernel variant: [master-step work][three_d][register budget][persistent];
-  // the budgets: 64 registers (4 blocks of 256 threads per SM), 80 (3
+  // the register budgets: 64 registers (4 blocks of 256 threads per SM), 80 (3
   // blocks of 256), 72 (7 blocks of 128)
   using KFn = void (*)(PushArgs);
-#define KAOS_K32(M, D, K)                                                     \
-  {{k_push32<D, 256, 4, false, M, K, false>, k_push32<D, 256, 4, true, M, K, false>}, \
-   {k_push32<D, 256, 3, false, M, K, false>, k_push32<D, 256, 3, true, M, K, false>}, \
-   {k_push32<D, 128, 7, false, M, K, false>, k_push32<D, 128, 7, true, M, K, false>}}
-  // [FP64 heating kick][master-step work][three_d][register budget][persistent]
-  static const KFn k32[2][2][2][3][2] = {
-      {{KAOS_K32(false, false, false), KAOS_K32(false, true, false)},
-       {KAOS_K32(true, false, false), KAOS_K32(true, true, false)}},
-      {{KAOS_K32(false, false, true), KAOS_K32(false, true, true)},
-       {KAOS_K32(true, false, true), KAOS_K32(true, true, true)}}};
+#define KAOS_K32(M, D, K, H)                                                  \
+  {{k_push32<D, 256, 4, false, M, K, false, H>, k_push32<D, 256, 4, true, M, K, false, H>}, \
+   {k_push32<D, 256, 3, false, M, K, false, H>, k_push32<D, 256, 3, true, M, K, false, H>}, \
+   {k_push32<D, 128, 7, false, M, K, false, H>, k_push32<D, 128, 7, true, M, K, false, H>}}
+#define KAOS_K32S(K, H)                                                       \
+  {{KAOS_K32(false, false, K, H), KAOS_K32(false, true, K, H)},               \
+   {KAOS_K32(true, false, K, H), KAOS_K32(true, true, K, H)}}
+  // [no heating, FP32 kick, FP64 kick][master-step work][three_d][register
+  // budget][persistent]
+  const int hk = h->P.ICRflag == 1 ? 1 + h->kick64 : 0;
+  static const KFn k32[3][2][2][3][2] = {KAOS_K32S(false, false), KAOS_K32S(false, true),
+                                         KAOS_K32S(true, true)};
+#undef KAOS_K32S
 #undef KAOS_K32
   const int nt = rs == 2 ? 128 : PUSH_THREADS;
-  static const KFn k64[2][2] = {
-      {k_push64<false, 256, 2, false, false>, k_push64<false, 256, 2, true, false>},
-      {k_push64<true, 256, 2, false, false>, k_push64<true, 256, 2, true, false>}};
-  // FP64 runs, [many items][three_d]: 64 registers (32 warps per SM, 120-150
-  // B of spills) where there are several waves of blocks, else 80 (24 warps,
-  // 60-80 B): ms per 20 steps 1e7 ions 6.20 / 6.35, 1e5 ions 0.143 / 0.127
-  // (124 registers, 16 warps, no spills: 6.75, 0.137)
-  static const KFn k64run[2][2] = {
-      {k_push64<false, 256, 3, false, true>, k_push64<true, 256, 3, false, true>},
-      {k_push64<false, 256, 4, false, true>, k_push64<true, 256, 4, false, true>}};
-  // runs of steps: [FP64 heating kick][three_d].  64 registers (32 warps per
-  // SM; 8 B of spills, 100 B with the FP64 kick) against 79 (24 warps, 0 and
-  // 28 B), ms per 20 steps: 1e7 ions 2.78 / 2.81, FP64 kick 4.30 / 4.33, 1e8
-  // ions 26.6 / 27.0, 256 uneven tubes 15.16 / 15.40; 128-thread blocks are
-  // up to 30 % slower on the uneven tubes (twice the table set-ups)
-  static const KFn k32run[2][2] = {
-      {k_push32<false, 256, 4, false, false, false, true>,
-       k_push32<true, 256, 4, false, false, false, true>},
-      {k_push32<false, 256, 4, false, false, true, true>,
-       k_push32<true, 256, 4, false, false, true, true>}};
-  const KFn fn = run ? (h->mixed ? k32run[h->kick64][h->three_d] : k64run[a.chunk > 256][h->three_d])
-                     : (h->mixed ? k32[h->kick64][ms][h->three_d][rs][ps] : k64[h->three_d][ps]);
+  const int ht = h->P.ICRflag == 1;
+  static const KFn k64[2][2][2] = {  // [heating][three_d][persistent]
+      {{k_push64<false, 256, 2, false, false, false>, k_push64<false, 256, 2, true, false, false>},
+       {k_push64<true, 256, 2, false, false, false>, k_push64<true, 256, 2, true, false, false>}},
+      {{k_push64<false, 256, 2, false, false, true>, k_push64<false, 256, 2, true, false, true>},
+       {k_push64<true, 256, 2, false, false, true>, k_push64<true, 256, 2, true, false, true>}}};
+  // FP64 runs, [many items][heating][three_d]: 64 registers (32 warps per SM,
+  // 120-150 B of spills) where there are several waves of blocks, else 80 (24
+  // warps, 60-80 B): ms per 20 steps 1e7 ions 6.20 / 6.35, 1e5 ions 0.143 /
+  // 0.127 (124 registers, 16 warps, no spills: 6.75, 0.137)
+  static const KFn k64run[2][2][2] = {
+      {{k_push64<false, 256, 3, false, true, false>, k_push64<true, 256, 3, false, true, false>},
+       {k_push64<false, 256, 3, false, true, true>, k_push64<true, 256, 3, false, true, true>}},
+      {{k_push64<false, 256, 4, false, true, false>, k_push64<true, 256, 4, false, true, false>},
+       {k_push64<false, 256, 4, false, true, true>, k_push64<true, 256, 4, false, true, true>}}};
+  // runs of steps: [no heating, FP32 kick, FP64 kick][three_d].  64 registers
+  // (32 warps per SM; 8 B of spills, 100 B with the FP64 kick) against 79 (24
+  // warps, 0 and 28 B), ms per 20 steps: 1e7 ions 2.78 / 2.81, FP64 kick 4.30
+  // / 4.33, 1e8 ions 26.6 / 27.0, 256 uneven tubes 15.16 / 15.40; 128-thread
+  // blocks are up to 30 % slower on the uneven tubes (twice the table set-ups)
+  static const KFn k32run[3][2] = {
+      {k_push32<false, 256, 4, false, false, false, true, false>,
+       k_push32<true, 256, 4, false, false, false, true, false>},
+      {k_push32<false, 256, 4, false, false, false, true, true>,
+       k_push32<true, 256, 4, false, false, false, true, true>},
+      {k_push32<false, 256, 4, false, false, true, true, true>,
+       k_push32<true, 256, 4, false, false, true, true, true>}};
+  const KFn fn = run ? (h->mixed ? k32run[hk][h->three_d] : k64run[a.chunk > 256][ht][h->three_d])
+                     : (h->mixed ? k32[hk][ms][h->three_d][rs][ps] : k64[ht][h->three_d][ps]);
   if (smem > 48 * 1024)
     CK(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int &occ = h->occ[h->mixed ? ms : 0][rs];
@@ -874,18 +883,20 @@ static int strided_grid(kaos_handle *h, int n) {
 }
 
 // charge exchange at the start of a step (_8_KineticSolver.f90:95-166)
-int launch_cx(kaos_handle *h) {
+int launch_cx(kaos_handle *h, bool master) {
   CxArgs a = cx_args(h);
   const int nq = max_nq(h);
   // the per-chunk Qindk1 counts were accumulated by the previous push
   // a block per listed cell (the list length is on the device: one
   // resident wave of 256-thread blocks, striding over the list)
+  // (an ordinary step's first kernel: it advances a replayed graph's step)
   k_cx_scan<<<(int)std::min<int64_t>(h->ncell, 8 * (int64_t)sm_count(h)), 256, 0, h->s>>>(
-      a, h->d_cell_tube, h->d_cell_q);
+      a, h->d_cell_tube, h->d_cell_q, h->capturing && !master ? h->d_step : nullptr);
   // the scan has read every count: cleared for the next push; then a block
   // per chunk with conversions
   CK(cudaMemsetAsync(h->d_cxc, 0, (size_t)h->ncx * nq * sizeof(unsigned), h->s));
-  k_cx_convert<<<std::max(1, std::min(h->ncx, h->cx_blocks)), 256, cx_convert_smem(nq), h->s>>>(a);
+  k_cx_convert<<<std::max(1, std::min(h->ncx, h->cx_blocks)), 32 * CX_WARPS,
+                 cx_convert_smem(nq), h->s>>>(a);
   h->launches += 2;
   CK(cudaGetLastError());
   return KAOS_OK;
@@ -1016,7 +1027,6 @@ __global__ void k_sample_rng(SampleArgs a) {
 }
 
 __global__ void k_set_step(uint32_t *d, uint32_t v) { *d = v; }
-__global__ void k_next_step(uint32_t *d) { *d += 1u; }
 
 // The charge-exchange activity of the master interval that starts at the
 // next step, from the list length and ENA counts the last master step
@@ -1037,12 +1047,8 @@ int step_once(kaos_handle *h) {
   const bool next_master = is_master(h, n + 1);
   const bool qx = h->P.QEXCHANGEflag == 1;
   int rc;
-  // d_step: n - 1 -> n for the kernels of this step (a master step advances
-  // it in its first kernel)
-  if (h->capturing && !is_master(h, n)) {
-    k_next_step<<<1, 1, 0, h->s>>>(h->d_step);
-    h->launches++;
-  }
+  // (captured: d_step goes from n - 1 to n in the step's first kernel -- the
+  // selection scan of an ordinary step, k_master_begin of a master step)
   if (n == 1) {
     // KineticSolverASub: statistics of the initial state, fields, push.
     if ((rc = zero_accum(h))) return rc;
@@ -1074,7 +1080,7 @@ int step_once(kaos_handle *h) {
   // an idle interval converts nothing: no selection; its master step still
   // counts Qindk1 for the next interval, into rows cleared here
   const bool cx_on = qx && !h->cx_idle;
-  if (cx_on && (rc = launch_cx(h))) return rc;
+  if (cx_on && (rc = launch_cx(h, master))) return rc;
   if (qx && !cx_on && master)
     CK(cudaMemsetAsync(h->d_cxc, 0, (size_t)h->ncx * max_nq(h) * sizeof(unsigned), h->s));
   // the injection of one boundary runs beside the push (it fills slots behind
@@ -1706,7 +1712,7 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
       if (b.second > 44 * 1024)
         CK(cudaFuncSetAttribute(b.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.second));
     int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cx_convert, 256,
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cx_convert, 32 * CX_WARPS,
                                                      cx_convert_smem((int)nq)));
     h->cx_blocks = std::max(1, per_sm) * sm_count(h);
   }

@@ -755,7 +755,7 @@ __device__ __forceinline__ HeatC<T> heat_consts(const CellTables &c, int64_t g) 
 // ---------------------------------------------------------------------------
 // FP64 kernel: ions stored as meridian-plane (rho, z) in FP64.  RUN: nsub
 // ordinary steps per launch with the ion's state in registers, as in k_push32.
-template <bool THREE_D, int NT, int MINB, bool PERSIST, bool RUN>
+template <bool THREE_D, int NT, int MINB, bool PERSIST, bool RUN, bool HEAT>
 __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
   extern __shared__ double sm[];
   const int nqmax = a.nqs;
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     for (int k = threadIdx.x; k < (int)(sizeof(VBins) / 16); k += NT)
       ((uint4 *)&VB)[k] = ((const uint4 *)a.vbins)[k];
   const double *VE1 = VB.e1, *VEP = VB.ep;
-  const bool kick = a.icr && !a.icrcoh;  // ordered by the item loop's barrier
+  const bool kick = HEAT && !a.icrcoh;  // ordered by the item loop's barrier
   if (kick) kf_tables_fill(kf_tables(), a.kf);
   // one work item per block, or a persistent grid striding over the items
   for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     double rho = I.rho[j], z = I.z[j], vpar = I.vpar[j];
     double v1 = I.v1[j], v2 = I.v2[j];
     double aea = I.aea[j], ag = I.ag[j];
-    const uint64_t pid = a.icr ? I.id[j] : 0;
+    const uint64_t pid = HEAT ? I.id[j] : 0;
     if (prologue) field_prologue(a, T, E, Cc, I.qk4[j], qprev, aea, ag);
     // (2D grid, a run: the last speeds inside the grid, as in k_push32)
     double l_vp = 0.0, l_s = 0.0;
@@ -826,7 +826,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     int b1 = -1, b2 = -1, bp = -1;
     if (RUN && !THREE_D) {
       if (vpar >= VEP[0] && vpar <= VEP[c_vg.npar]) { l_vp = vpar; in_vp = true; }
-      if (m == 0u || a.icr) {  // (the speed changes only by the kicks)
+      if (m == 0u || HEAT) {  // (the speed changes only by the kicks)
         const double sp = sqrt(vp2);
         if (sp >= VE1[0] && sp <= VE1[c_vg.n1]) { l_s = sp; in_s = true; }
       }
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     const double a1 = apar(g1, vp2, aea, ag, a.ff);
     // wave heating (the mirror force keeps the pre-kick Vperp)
     double v1n = v1, v2n = v2;
-    if (a.icr && qi >= 0) {
+    if (HEAT && qi >= 0) {
       const double sl = g1.ell * g1.isl;
       const double Om = qs_ms * MDIP * sl * (g1.ir * g1.ir * g1.ir);
       if (kick) {
@@ -922,7 +922,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     I.rho[j] = rhoN;
     I.z[j] = zN;
     I.vpar[j] = vparN;
-    if (a.icr) {
+    if (HEAT) {
       I.v1[j] = v1n;
       I.v2[j] = v2n;
     }
@@ -1037,9 +1037,14 @@ struct __align__(16) CellS {
 // it is loaded and stored once instead of once per step, and every step does
 // the arithmetic of the one-step variant in the same order (bit-identical
 // results however a run is cut, tests/test_gpu_runs.py).
-template <bool THREE_D, int NT, int MINB, bool PERSIST, bool MASTER, bool K64, bool RUN>
+//
+// HEAT false: runs without wave heating, whose push needs neither the kick's
+// code nor the registers it costs every variant (charge exchange of 2e7 ions,
+// ordinary step: 301 us with the kick's code behind a flag, 267 without).
+template <bool THREE_D, int NT, int MINB, bool PERSIST, bool MASTER, bool K64, bool RUN, bool HEAT>
 __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   static_assert(!(RUN && (MASTER || PERSIST)), "runs hold ordinary steps, one item per block");
+  static_assert(HEAT || !K64, "no kick, no FP64 kick");
   // master-step work (field re-interpolation, binning) only in the MASTER
   // variant: the ordinary step carries none of its code or registers
   const bool bin = MASTER && a.bin, prologue = MASTER && a.prologue,
@@ -1075,7 +1080,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
   VBins &VB = *(VBins *)((char *)sm + ve_off);
   const double *VE1 = VB.e1, *VE2 = VB.e2, *VEP = VB.ep;
   const VBinTab &VT1 = VB.t1, &VT2 = VB.t2, &VTP = VB.tp;
-  if (K64 && a.icr) kf_tables_fill(kf_tables(), a.kf);  // ordered by the item loop's barrier
+  if (K64) kf_tables_fill(kf_tables(), a.kf);  // ordered by the item loop's barrier
   if (bin || !THREE_D)  // the first barrier of the item loop orders them before any use
     for (int k = threadIdx.x; k < (int)(sizeof(VBins) / 16); k += NT)
       ((uint4 *)&VB)[k] = ((const uint4 *)a.vbins)[k];
@@ -1100,7 +1105,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       C.ud = a.ct.uH[g] - a.ct.uL[g];
       // quadratic in the offset through the edges and the midpoint
       C.uc = 4.0 * a.ct.uM[g] - 2.0 * (a.ct.uL[g] + a.ct.uH[g]);
-      if (a.icr) {
+      if (HEAT) {
         const double lam = a.ct.lambdaPerp[g];
         C.hk[0] = (float)a.ct.hK1[g];
         C.hk[1] = (float)a.ct.hK2[g];
@@ -1156,7 +1161,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     n_vp = VP[k];
     n_v = V12[k];
     n_f = FF[k];
-    if (a.icr) n_id = ID[k];
+    if (HEAT) n_id = ID[k];
     if (prologue) n_qk = QK[k];
   }
   for (unsigned k = threadIdx.x; k < (unsigned)nk; k += NT) {
@@ -1166,7 +1171,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       n_vp = VP[k];
       n_v = V12[k];
       n_f = FF[k];
-      if (a.icr) n_id = ID[k];
+      if (HEAT) n_id = ID[k];
     }
     double x0 = n_x;
     double vpar = n_vp;
@@ -1180,7 +1185,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       n_vp = VP[kn];
       n_v = V12[kn];
       n_f = FF[kn];
-      if (a.icr) n_id = ID[kn];
+      if (HEAT) n_id = ID[kn];
       if (prologue) n_qk = QK[kn];
     }
     if (x0 < XDEAD_LIM) continue;  // slot marked DEAD
@@ -1218,10 +1223,10 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     g1.ct = g1.q * uf * uf;
     const float rfl = uf * fRE;  // r in FP32
     g1.ir = rcpa(rfl);
-    g1.ell = 1.0f + 3.0f * g1.ct * g1.ct;
+    g1.ell = fmaf(3.0f * g1.ct, g1.ct, 1.0f);
     g1.isl = rsq(g1.ell);
     const float vparf = (float)vpar, v1f = (float)v1, v2f = (float)v2;
-    const float vp2 = v1f * v1f + v2f * v2f;
+    const float vp2 = fmaf(v1f, v1f, v2f * v2f);
     // sqrt(ell) in FP64, ell = 1 + 3 cos^2 = 4 - 3 sin^2 on the field line:
     // 1/sqrt from the FP32 value and one FP64 Newton step
     const double ell64 = fma(-3.0, s2, 4.0);
@@ -1237,7 +1242,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     double v1n = v1, v2n = v2;  // after the wave-heating kick
     // (the FP64 kick of K64 runs after the position and V|| stores below:
     // nothing before them reads the kicked pair)
-    if (!K64 && a.icr && qi >= 0) {
+    if (!K64 && HEAT && qi >= 0) {
       const float sl = g1.ell * g1.isl;
       const float ir3 = g1.ir * g1.ir * g1.ir;
       const float Om = qs_ms * (float)MDIP * sl * ir3;
@@ -1258,7 +1263,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       }
     }
     // stored at once: the kicked pair holds no registers through the RK
-    if (!RUN && !K64 && a.icr) V12[k] = make_double2(v1n, v2n);
+    if (!RUN && !K64 && HEAT) V12[k] = make_double2(v1n, v2n);
     // ---- the stage accelerations ----------------------------------------
     // a|| = M + s C0 + ce1 AEA with the signed mirror term M (cos(theta) in
     // place of s |cos|: smooth through the equator), the hemisphere sign s
@@ -1277,11 +1282,12 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     const float hm = fc.cm * 1.5f * vp2 * g1.ir;
     const float M1 = hm * g1.ct * G2 * g1.isl;
     const float dM = hm * g1.ir * il *
-                     fmaf(sn2 * cs2 * il, fmaf(9.0f * sn2, il, 8.0f), -(1.0f + cs2) * G2);
+                     fmaf(sn2 * cs2 * il, fmaf(9.0f * sn2, il, 8.0f),
+                          -__fadd_rn(1.0f, cs2) * G2);
     const float C0 = fc.ce2 * fabsf(aea) - fc.cg * fabsf(ag);
     const float Ce = fc.ce1 * aea;
     const float C1 = g1.ct <= 0.0f ? -C0 : C0;
-    const float a1 = M1 + C1 + Ce;
+    const float a1 = __fadd_rn(M1, C1) + Ce;
     const float hvf = h * vparf, ds2 = hh * vparf, ds4 = fmaf(hsq2, a1, hvf);
     // q at the k4 point: dq/ds = -RE^2 sqrt(ell) / r^3 along e1
     if (last && a.write_qk4)
@@ -1333,7 +1339,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       const float z2 = fmaf(ds2, ez, zf), z4 = fmaf(ds4, ez, zf);
       a2 = a2 + (z2 <= 0.0f ? -C0 : C0) + Ce;
       a4 = a4 + (z4 <= 0.0f ? -C0 : C0) + Ce;
-      const float ac = hh6 * (2.0f * a1 + a2);
+      const float at = fmaf(2.0f, a1, a2), ac = hh6 * at;
       // cos, sin and the meridian point in FP64 (sin from an FP32 seed and
       // one FP64 Newton step)
       double ys = (double)rsq(s2f);
@@ -1343,16 +1349,16 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       const double xr = fma(hv, 3.0 * ct * st, r * st) +
                         (double)(ac * (3.0f * g1.ct * stf * g1.isl));
       const double xz = fma(hv, fma(3.0 * ct, ct, -1.0), r * ct) + (double)(ac * ez);
-      const double r2 = xr * xr + xz * xz;
+      const double r2 = fma(xr, xr, xz * xz);
       double y = (double)rsq((float)r2);
       y = y * fma(-0.5 * r2 * y, y, 1.5);
       qN = (RE * RE) * xz * (y * y * y);
       od = __dmul_rn(qN - cq.x, cc.y);
-      dal = pl * ((hvf + ac) * g1.ir) * (stf * g1.isl);
+      dal = pl * (fmaf(hh6, at, hvf) * g1.ir) * (stf * g1.isl);
     }
     // V|| along the new field direction: the turn of the direction over the
     // step, dal = 3 (1 + cos^2) / ell dtheta, dtheta = D / r sin / sqrt(ell)
-    const float dv = fmaf(h6, a1 + 4.0f * a2 + a4, -0.5f * vparf * dal * dal);
+    const float dv = fmaf(h6, fmaf(4.0f, a2, a1) + a4, -0.5f * vparf * dal * dal);
     const double vparN = vpar + (double)dv;
     // the new cell: most ions stay well inside the cell they started the
     // step in; else the edge search (escaped ions keep the end cell and an
@@ -1376,7 +1382,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     }
     if (RUN && !THREE_D) {
       if (vpar >= VEP[0] && vpar <= VEP[c_vg.npar]) { l_vp = vpar; in_vp = true; }
-      if (m == 0u || a.icr) {  // (the speed changes only by the kicks)
+      if (m == 0u || HEAT) {  // (the speed changes only by the kicks)
         const double sp = vperp_mag(v1, v2);
         if (sp >= VE1[0] && sp <= VE1[c_vg.n1]) { l_s = sp; in_s = true; }
       }
@@ -1393,7 +1399,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     }
     if (last && a.write_qind) QI[k] = qi;
     if (!RUN && a.cxc && qi >= 0) atomicAdd(&HC[qi], 1u);
-    if (K64 && a.icr) {
+    if (K64) {
       if (qi >= 0) {
         // FP64 kick at the start-of-step point: Omega = (q/m) MDIP sqrt(ell)
         // / r^3 and 1/Omega from the FP64 radius and 1/sqrt(ell) (yl), 1/r
@@ -1425,7 +1431,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       if (!isfinite(vpar) || !isfinite(x0)) atomicOr(a.status, ST_NAN);
       X[k] = x0;
       VP[k] = vpar;
-      if (a.icr) V12[k] = make_double2(v1, v2);
+      if (HEAT) V12[k] = make_double2(v1, v2);
       if (!THREE_D) {
         const int old = I.vb[j];
         const int bp = in_vp ? vbin_tab(VTP, VEP, c_vg.npar, l_vp) : (old & 0xffff) - 1;
