@@ -890,10 +890,28 @@ struct ConvArgs {
   int mixed;
 };
 
-// |B| / B0 at (q, u = r/RE) on any field line: sqrt(1 + 3 cos^2) / u^3.
-__device__ __forceinline__ double bnorm(double q, double u) {
-  const double ct = q * u * u;
-  return sqrt(1.0 + 3.0 * ct * ct) / (u * u * u);
+// sqrt(x) within ~0.5 ulp (x well inside the FP32 range).
+__device__ __forceinline__ double sqrt_near(double x) {
+  const double y = rsq_near(x), t = x * y;
+  return fma(fma(-t, t, x), 0.5 * y, t);
+}
+
+// sqrt(B_new / B_old) at q, u_old = r/RE on the old line and u_new on the new
+// one, |B| going as sqrt(1 + 3 cos^2) / u^3: the quotient formed once, its
+// reciprocal from an FP32 seed with one third-order step and the quotient's
+// own remainder (the library's three divisions and three square roots took
+// most of the kernel's time; the error against 64-bit extended arithmetic is
+// no larger, having two roundings fewer).
+__device__ __forceinline__ double convect_factor(double q, double u_old, double u_new) {
+  const double qn = q * u_new, cn = qn * u_new, co = (q * u_old) * u_old;
+  const double n = sqrt_near(fma(3.0 * cn, cn, 1.0)) * (u_old * u_old * u_old);
+  const double d = sqrt_near(fma(3.0 * co, co, 1.0)) * (u_new * u_new * u_new);
+  double y = (double)rcpa((float)d);
+  const double e = fma(-d, y, 1.0);
+  y = fma(y * e, 1.0 + e, y);
+  double r = n * y;
+  r = fma(fma(-r, d, n), y, r);
+  return sqrt_near(r);
 }
 
 // The queued moves of one master step in one launch: blockIdx.y = the move
@@ -951,7 +969,7 @@ __device__ __forceinline__ void convect_ions(const ConvArgs &a) {
       u_old = r / RE;
     }
     const double u_new = quartic_newton_conv(q, ip_new, u_old, 8);
-    const double f = sqrt(bnorm(q, u_new) / bnorm(q, u_old));
+    const double f = convect_factor(q, u_old, u_new);
     if (a.mixed) {
       const double2 v = a.ion.v12[j];
       a.ion.v12[j] = make_double2(f * v.x, f * v.y);
