@@ -33,7 +33,7 @@ constexpr int BC_THREADS = 256;
 constexpr int BC_COMPACT_EVERY = 8;
 constexpr int64_t COUNT_STAGE = 64 * 1024;  // counters per staging buffer
 // cells per tube: the per-cell tables of a tube live in shared memory (the
-// mixed push holds 92 bytes per cell, the collision-count kernel 64)
+// mixed push holds 108 bytes per cell, the collision-count kernel 64)
 constexpr int MAX_CELLS = 2048;
 // push work-item sizes the autotuner tries (ions per item); an item's ions
 // lie in one charge-exchange selection chunk
@@ -464,7 +464,9 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
        k_push32<true, 256, 4, false, false, true, true, true>}};
   const KFn fn = run ? (h->mixed ? k32run[hk][h->three_d] : k64run[a.chunk > 256][ht][h->three_d])
                      : (h->mixed ? k32[hk][ms][h->three_d][rs][ps] : k64[ht][h->three_d][ps]);
-  if (smem > 48 * 1024)
+  // (static shared memory counts towards the 48 KB: up to 6.9 KB, the FP64
+  // push's bin edges and lookup tables and its kick's tables)
+  if (smem > 40 * 1024)
     CK(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int &occ = h->occ[h->mixed ? ms : 0][rs];
   if (ps && !occ) {
@@ -1709,7 +1711,7 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
         {(const void *)k_push_ena, ena_push_smem((int)nq, ntubes)},
         {(const void *)k_load, (nq + 1) * sizeof(double)}};
     for (const auto &b : big)  // (static shared memory counts towards the 48 KB)
-      if (b.second > 44 * 1024)
+      if (b.second > 40 * 1024)
         CK(cudaFuncSetAttribute(b.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.second));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cx_convert, 32 * CX_WARPS,

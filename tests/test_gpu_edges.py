@@ -77,6 +77,16 @@ def test_largest_velocity_grid_128_bins():
     _compare(s, 0, o)
 
 
+def test_largest_tube_heated_on_a_wider_velocity_grid():
+    """42 KB of tables and binning window beside 7 KB of the bin searches' and
+    the kick's own: above what a launch gets without asking for more."""
+    mi = ModelInput(h=0.01, ndatfac=3, ION2VPERPflag=1, ICRflag=1)
+    spec = TubeSpec(L=4.0, nq=2048, n_particles=20000, q_ub=1e-3, H=900e3,
+                    heat_rate_eV_s=5.0)
+    s, o = _run_one(mi, spec, make_vgrid(True, 32, 32, 24, 8e3), 4)
+    _compare(s, 0, o)
+
+
 def test_limits_rejected():
     mi = ModelInput(h=0.01, ndatfac=3, ION2VPERPflag=1)
     vg = make_vgrid(True, 16, 16, 24, 8e3)
