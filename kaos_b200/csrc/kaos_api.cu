@@ -216,7 +216,8 @@ struct kaos_handle {
   WorkMap rmap;  // the same for runs of steps (run_chunk)
   int wsel = 1;          // chosen map (CHUNKS[wsel] ions per item)
   int persistent = 0;    // persistent grid striding over the items
-  int tune_pending = 1;  // autotune before the next step
+  int tune_pending = 2;  // autotuner: 2 nothing timed yet, 1 the ordinary push not yet
+  int tune_singles = 0;  // ordinary steps made one by one since
   int forced = 0;        // shape given by kaos_set_launch
   int regsel = 0;        // mixed push register budget: 0 = 64, 1 = 80, 2 = 72
   int regsel_master = 0; // the same for the master-step variant of the push
@@ -1156,10 +1157,26 @@ int run_steps(kaos_handle *h, int64_t g) {
 
 // Launch-shape autotuner: the live ion state is copied into the spare
 // buffer set and the push of the next step is timed there for every
-// candidate (ions per work item x one block per item or a persistent grid);
-// the fastest is kept.  The simulation state is not touched, and results do
-// not depend on the choice (every ion is pushed by the same code).
-int autotune(kaos_handle *h) {
+// candidate; the fastest is kept.  The simulation state is not touched, and
+// results do not depend on the choice (every ion is pushed by the same code).
+//
+// The one-step push of ordinary steps is timed (ions per work item x one
+// block per item or a persistent grid x register budget) only for a handle
+// that uses it: its interval converts ions, or it has made TUNE_AFTER
+// ordinary steps that were no part of a run.  Else only the master-step
+// variant is, which every handle uses: the budgets at 4096 ions per item, the
+// smaller items at the best of them (no persistent grid: 182 us against 179 at
+// its best for the ordinary push of 1e7 ions).  At 1e7 ions 15 launches of
+// 0.35 ms in place of 54 of 0.2 and 9 of 0.39.
+constexpr int TUNE_AFTER = 4;
+int autotune(kaos_handle *h, bool ordinary) {
+  // (items of 256 ions, push_args: only the register budget is left to choose)
+  const bool fine = h->rmap.chunk == 256 && !h->forced;
+  const int nreg = h->mixed ? 3 : 1;
+  if (fine && nreg == 1) {  // nothing to choose
+    h->tune_pending = 0;
+    return KAOS_OK;
+  }
   const int other = 1 - h->cur;
   const Fields F = ion_fields(h, h->cur, other);
   for (int f = 0; f < F.n; ++f)
@@ -1168,78 +1185,75 @@ int autotune(kaos_handle *h) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
-  float best = 1e30f;
-  int bw = h->wsel, bp = h->persistent, br = h->regsel;
-  // (items of 256 ions, push_args: only the register budget is left to choose)
-  const bool fine = h->rmap.chunk == 256 && !h->forced;
-  for (int m = 0; m < (fine ? 1 : NCHUNKS); ++m)
-    for (int pm = 0; pm < (fine ? 1 : 2); ++pm)
-    for (int rs = 0; rs < (h->mixed ? 3 : 1); ++rs) {
-      h->wsel = m;
-      h->persistent = pm;
-      h->regsel = rs;
-      PushArgs a = push_args(h);
-      a.ion = h->ion[other];
-      a.step = (uint32_t)(h->n + 1);
-      a.write_qind = 1;
-      a.write_qk4 = 0;
-      float tmin = 1e30f;
-      for (int rep = 0; rep < 3; ++rep) {  // the first is a warm-up
-        CK(cudaEventRecord(e0, h->s));
-        const int npev0 = h->npev;
-        const int64_t l0 = h->launches;
-        int rc = launch_push(h, a);
-        h->npev = npev0;   // tuning pushes are not part of the step timing
-        h->launches = l0;
-        if (rc) return rc;
-        CK(cudaEventRecord(e1, h->s));
-        CK(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, e0, e1));
-        if (rep > 0) tmin = std::min(tmin, ms);
-      }
-      if (tmin < best) { best = tmin; bw = m; bp = pm; br = rs; }
+  // time of one push with the shape now set in the handle (best of two after
+  // a warm-up); a master-step push fills binning accumulators that are
+  // cleared before the next master step uses them
+  auto time_push = [&](bool master, float *tmin) -> int {
+    PushArgs a = push_args(h);
+    a.ion = h->ion[other];
+    a.step = (uint32_t)(h->n + 1);
+    a.write_qind = 1;
+    if (master) a.bin = a.prologue = 1;
+    else a.write_qk4 = 0;
+    *tmin = 1e30f;
+    for (int rep = 0; rep < 3; ++rep) {
+      CK(cudaEventRecord(e0, h->s));
+      const int npev0 = h->npev;
+      const int64_t l0 = h->launches;
+      int rc = launch_push(h, a);
+      h->npev = npev0;   // tuning pushes are not part of the step timing
+      h->launches = l0;
+      if (rc) return rc;
+      CK(cudaEventRecord(e1, h->s));
+      CK(cudaEventSynchronize(e1));
+      float ms = 0.f;
+      CK(cudaEventElapsedTime(&ms, e0, e1));
+      if (rep > 0) *tmin = std::min(*tmin, ms);
     }
-  h->wsel = bw;
-  h->persistent = bp;
-  h->regsel = br;
-  // the master-step variant (field re-interpolation and binning) has its
-  // own register needs: its budget is timed separately with the chosen
-  // work-item shape (the binning accumulators it fills are cleared before
-  // the next master step uses them)
-  int bm = br;
-  if (h->mixed) {
-    float bestm = 1e30f;
-    for (int rs = 0; rs < 3; ++rs) {
-      h->regsel_master = rs;
-      PushArgs a = push_args(h);
-      a.ion = h->ion[other];
-      a.step = (uint32_t)(h->n + 1);
-      a.write_qind = 1;
-      a.bin = 1;
-      a.prologue = 1;
-      float tmin = 1e30f;
-      for (int rep = 0; rep < 3; ++rep) {
-        CK(cudaEventRecord(e0, h->s));
-        const int npev0 = h->npev;
-        const int64_t l0 = h->launches;
-        int rc = launch_push(h, a);
-        h->npev = npev0;
-        h->launches = l0;
-        if (rc) return rc;
-        CK(cudaEventRecord(e1, h->s));
-        CK(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, e0, e1));
-        if (rep > 0) tmin = std::min(tmin, ms);
-      }
-      if (tmin < bestm) { bestm = tmin; bm = rs; }
-    }
+    return KAOS_OK;
+  };
+  float best = 1e30f, t = 0.f;
+  int rc;
+  if (ordinary) {
+    int bw = h->wsel, bp = h->persistent, br = h->regsel;
+    for (int m = 0; m < (fine ? 1 : NCHUNKS); ++m)
+      for (int pm = 0; pm < (fine ? 1 : 2); ++pm)
+        for (int rs = 0; rs < nreg; ++rs) {
+          h->wsel = m;
+          h->persistent = pm;
+          h->regsel = rs;
+          if ((rc = time_push(false, &t))) return rc;
+          if (t < best) { best = t; bw = m; bp = pm; br = rs; }
+        }
+    h->wsel = bw;
+    h->persistent = bp;
+    h->regsel = h->regsel_master = br;
+  } else {
+    if (!fine) h->wsel = NCHUNKS - 1;
+    h->persistent = 0;
+    h->regsel = h->mixed ? 1 : 0;
   }
-  h->regsel_master = bm;
+  // the master-step variant (field re-interpolation and binning) has its
+  // own register needs: its budget is timed separately
+  if (h->mixed || !ordinary) {
+    int bm = 0, bw = h->wsel;
+    best = 1e30f;
+    for (int rs = 0; rs < nreg; ++rs) {
+      h->regsel_master = rs;
+      if ((rc = time_push(true, &t))) return rc;
+      if (t < best) { best = t; bm = rs; }
+    }
+    h->regsel_master = bm;
+    for (int m = NCHUNKS - 2; m >= 0 && !ordinary && !fine; --m) {
+      h->wsel = m;
+      if ((rc = time_push(true, &t))) return rc;
+      if (t < best) { best = t; bw = m; }
+    }
+    h->wsel = bw;
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  h->tune_pending = 0;
+  h->tune_pending = ordinary ? 0 : 1;
   for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
   h->graphs.clear();
   return KAOS_OK;
@@ -1868,7 +1882,8 @@ int kaos_set_graph(kaos_handle *h, int32_t on) {
 int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode) {
   if (!h) return KAOS_ERR_PARAM;
   if (chunk == 0 || mode < 0) {
-    h->tune_pending = 1;
+    h->tune_pending = 2;
+    h->tune_singles = 0;
     h->forced = 0;
     return KAOS_OK;
   }
@@ -1991,9 +2006,14 @@ int kaos_step(kaos_handle *h, int64_t nsteps) {
     const int64_t n = h->n + 1;
     int rc;
     if ((rc = resolve_cx_idle(h))) return rc;
-    if (h->tune_pending && n >= 2 && (rc = autotune(h))) return rc;
+    if (h->tune_pending && n >= 2) {
+      const bool ordinary = (h->P.QEXCHANGEflag == 1 && !h->cx_idle) ||
+                            h->tune_singles >= TUNE_AFTER;
+      if ((ordinary || h->tune_pending == 2) && (rc = autotune(h, ordinary))) return rc;
+    }
     const int64_t r = run_length(h, n, nsteps - k);
     if (r > 0) {
+      if (r == 1 && h->tune_pending) ++h->tune_singles;
       if ((rc = run_steps(h, r))) return rc;
       k += r;
       continue;

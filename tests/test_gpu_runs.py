@@ -87,3 +87,23 @@ def test_run_ion_counts(n):
         assert np.array_equal(x, y)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("prec", PRECS)
+def test_single_steps_choose_their_shape(prec):
+    """A handle above the small-item limit (2^21 slots) stepped one by one
+    through a master step: the shape is chosen again after four of them, and
+    the state stays that of the runs."""
+    mi = ModelInput(h=0.01, ndatfac=9, ION2VPERPflag=1, ICRflag=1, precision=prec)
+    spec = TubeSpec(L=3.0, nq=24, n_particles=30000, q_ub=0.5, H=400e3, heat_rate_eV_s=2.0)
+    tubes = [make_tube(spec, mi)]
+    tubes[0].capacity = (1 << 21) + 1000
+    vg = make_vgrid(True, 16, 16, 24, 9e3)
+    init = [grids.initial_particles(tubes[0], spec, mi, seed=3)]
+    a, b = _solver(mi, tubes, init, vg), _solver(mi, tubes, init, vg)
+    for _ in range(12):
+        a.step(1)
+    b.step(12)
+    assert a.launch()[0] in (1024, 2048, 4096) and b.launch()[0] in (1024, 2048, 4096)
+    for x, y in zip(_state(a, 1), _state(b, 1)):
+        np.testing.assert_array_equal(x, y)
