@@ -64,7 +64,10 @@ def fp64_pipe_roofline(rate_per_gpu):
     return {"bound": "fp64", "achieved": achieved, "peak": FP64_NOMINAL_TFLOPS,
             "unit": "TFLOP/s (flop-equivalents)", "frac": achieved / FP64_NOMINAL_TFLOPS,
             "peak_kind": "nominal", "f_alg": F_ALG,
-            "weights": "add/mul 1, div/sqrt 4, transcendental call 20"}
+            "weights": "add/mul 1, div/sqrt 4, transcendental call 20",
+            "note": "operations of the reference formulation; the path takes the same "
+                    "trajectories with fewer (about 300 FP64 instructions per ion-step), so "
+                    "the ratio can exceed 1"}
 
 
 def clocks_sampler(stop, out):
@@ -134,7 +137,8 @@ def build_workload(precision, n_part=N_PART, heating=True, collisions=True,
 
 
 def bytes_per_particle_step(mixed, heating, collisions):
-    """Algorithmic HBM bytes per ion per ordinary step (reads + writes).
+    """Algorithmic HBM bytes per ion per push launch (reads + writes): an
+    ordinary step, or a run of them, whose state stays in registers.
     `collisions`: the charge exchange converts ions in this interval (an
     idle interval -- no converting cell, no ENA -- stores no Qindk1 or k4
     point at its ordinary steps)."""
@@ -152,7 +156,7 @@ def bytes_per_particle_step(mixed, heating, collisions):
 
 
 def profiled_traffic(name):
-    """DRAM bytes per ion-step of a push kernel from its committed ncu
+    """DRAM bytes per ion and launch of a push kernel from its committed ncu
     summary (the `traffic_bytes_per_ion:` line), or None."""
     try:
         with open(os.path.join(ROOT, "profiles", name)) as f:
@@ -199,7 +203,7 @@ def run_ours(args, precision, graph=False, ndatfac=NDATFAC, steps=None):
     # library's stream; inputs 0.5-1 GB > L2, so no explicit flush) --------
     s.step(steps)
     ms, launches = s.timing()
-    pms, pl = s.push_timing()  # events around each push launch
+    pms, pl = s.push_timing()  # events around each push launch (a run of steps is one)
     n1, ne = s.count()
     nmean = 0.5 * (n0 + n1)
     value = nmean * steps / (ms * 1e-3)
@@ -843,7 +847,9 @@ def main():
                          "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_kind": peak_kind,
                          "kernel": "k_push32 (mixed push), average over the timed "
-                                   "window's launches (ordinary and master steps)",
+                                   "window's launches (runs of ordinary steps, master "
+                                   "steps); a run reads and writes the state once for "
+                                   "all its steps and is bound by issue, not by HBM",
                          "bytes_per_particle": mixed_bytes,
                          "frozen_bytes_per_particle": FROZEN_MIXED_BYTES,
                          "achieved_at_frozen_bytes": achieved_frozen,
@@ -861,7 +867,8 @@ def main():
                                        "moment matches the FP64 path; the frozen 48 B "
                                        "counted the earlier FP32 state",
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                                           "per ion of a 6e6-ion launch, scaled to this launch"},
+                                           "per ion of a 4e6-ion run of 18 steps, scaled to this "
+                                           "launch"},
             "cpu_baseline": cpu,
             "e2e": None if e2e is None else {
                 "value": e2e["value"] * world, "unit": "particle-steps/s",
