@@ -197,6 +197,7 @@ struct kaos_handle {
   unsigned *acc_base = nullptr;
   int64_t acc_len = 0;
   kaos_reduce_fn reduce_fn = nullptr;
+  int hooked = 0;  // a reduction hook has been set
   void *reduce_ctx = nullptr;
   int rank = 0, nranks = 1;          // share of the charge-exchange counts
   std::vector<uint64_t> id_base;     // first ion id per tube
@@ -281,6 +282,13 @@ int upload(kaos_handle *h, double **dst, const std::vector<double> &v) {
   if (rc) return rc;
   CK(cudaMemcpy(*dst, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice));
   return KAOS_OK;
+}
+
+// The captured steps hold kernel arguments and launch sequences of the time
+// of their capture.
+void drop_graphs(kaos_handle *h) {
+  for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
+  h->graphs.clear();
 }
 
 bool is_master(const kaos_handle *h, int64_t n) {
@@ -627,8 +635,10 @@ int launch_moments(kaos_handle *h, uint32_t nn, int commit = 0) {
                        cudaMemcpyDeviceToHost, h->s));
     h->cx_stat_pending = 1;
     // ENA statistics from the second master step on (an idle interval has no
-    // ENA, its last master step had none either: the rows are zero already)
-    if (nn > 1 && !h->cx_idle) {
+    // ENA, its last master step had none either: the rows are zero already --
+    // unless the counters are, or lately were, sums over the ranks of a split
+    // tube, of which only this one is idle)
+    if (nn > 1 && (!h->cx_idle || h->hooked)) {
       k_ena_moments<<<moment_grid(h), 256, 0, h->s>>>(h->d_tubes, h->d_cell_tube, h->ct, h->acc);
       h->launches++;
     }
@@ -1254,8 +1264,7 @@ int autotune(kaos_handle *h, bool ordinary) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   h->tune_pending = ordinary ? 0 : 1;
-  for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-  h->graphs.clear();
+  drop_graphs(h);
   return KAOS_OK;
 }
 
@@ -1899,8 +1908,7 @@ int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode) {
   h->regsel = (mode >> 1) & 3;
   h->regsel_master = ((mode >> 3) & 3) ? ((mode >> 3) & 3) - 1 : h->regsel;
   h->tune_pending = 0;
-  for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-  h->graphs.clear();
+  drop_graphs(h);
   return KAOS_OK;
 }
 
@@ -1960,6 +1968,10 @@ int kaos_update_tube(kaos_handle *h, int32_t tube, const kaos_tube_c *T) {
 
 int kaos_set_reduce(kaos_handle *h, kaos_reduce_fn fn, void *ctx) {
   if (!h) return KAOS_ERR_PARAM;
+  if (fn && !h->hooked) {
+    h->hooked = 1;
+    drop_graphs(h);
+  }
   h->reduce_fn = fn;
   h->reduce_ctx = ctx;
   return KAOS_OK;

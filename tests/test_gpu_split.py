@@ -13,7 +13,7 @@ import torch
 from kaos_b200 import build as kbuild
 from kaos_b200 import grids
 from kaos_b200.lib import Solver
-from kaos_b200.model_input import KAOS_EAMAG, KAOS_M0, KAOS_M2, KAOS_M2PAR
+from kaos_b200.model_input import KAOS_EAMAG, KAOS_ENA_NQ, KAOS_M0, KAOS_M2, KAOS_M2PAR
 from kaos_b200.shard import _DeviceCounters, split_ions
 
 pytestmark = pytest.mark.gpu
@@ -130,3 +130,46 @@ def test_nccl_hook_on_a_one_rank_group(tmp_path):
     finally:
         dist.destroy_process_group()
     ref.close()
+
+
+def test_split_tube_ena_rows_where_one_rank_converts_nothing():
+    """Cells that convert one ion a step: rank 0's share (N + rank) / nranks
+    is none of it, rank 1's all, so rank 0's intervals hold no ENA of its own.
+    The ENA counters are summed over the ranks like the ions', and both ranks
+    report the same ENA rows."""
+    mi, spec, tube, vg = grids.config_small(n_particles=6000, three_d=True,
+                                            steps_per_master=4, collisions=True)
+    tube.nsnormCNeut = tube.nsnormCNeut * 0.03
+    init = grids.initial_particles(tube, spec, mi, seed=21)
+    red = PairReduce()
+    solvers = []
+    for r in range(2):  # every second ion: both ranks hold ions of every cell
+        s = Solver(mi, [tube], vg)
+        s.set_id_base(0, r << 20)
+        s.set_rank(r, 2)
+        s.set_reduce(red.hook(r))
+        s.load(0, *[a[r::2] for a in init])
+        solvers.append(s)
+    errors = []
+
+    def run(s):
+        try:
+            s.step(9)
+        except Exception as e:  # noqa: BLE001 - reported below
+            errors.append(e)
+            red.barrier.abort()
+
+    th = [threading.Thread(target=run, args=(s,)) for s in solvers]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join(timeout=120)
+    assert not errors, errors
+    a, b = solvers
+    assert a.count()[1] == 0 and b.count()[1] > 0  # only rank 1 converted
+    rows = range(KAOS_ENA_NQ, KAOS_ENA_NQ + 9)
+    for m in rows:
+        np.testing.assert_array_equal(a.moments(m), b.moments(m), err_msg=str(m))
+    assert a.moments(KAOS_ENA_NQ).sum() > 0
+    for s in solvers:
+        s.close()
