@@ -313,12 +313,15 @@ int run_chunk(const kaos_handle *h) {
   return cap < (int64_t)1 << 21 ? 256 : 1024;
 }
 
-// What the heating tables of a tube ask of the kick (PushArgs).
+// What the heating tables of a tube ask of the kick (PushArgs).  The flags are
+// kernel arguments: a step captured before one rises would go without.
 void note_heating(kaos_handle *h, const kaos_tube_c &T) {
+  const int lam = h->heat_lam, chi = h->heat_chi;
   for (int k = 0; k < T.nq; ++k) {
     if (T.lambdaPerp && T.lambdaPerp[k] != 0.0) h->heat_lam = 1;
     if ((T.ChiPerp1 ? T.ChiPerp1[k] : 0.0) != (T.ChiPerp2 ? T.ChiPerp2[k] : 0.0)) h->heat_chi = 1;
   }
+  if (h->heat_lam != lam || h->heat_chi != chi) drop_graphs(h);
 }
 
 PushArgs push_args(kaos_handle *h, bool run = false) {

@@ -181,3 +181,30 @@ def test_state_reads_between_steps_change_nothing(mixed):
         np.testing.assert_array_equal(a["p"][k], b["p"][k], err_msg=k)
     np.testing.assert_array_equal(a["cnt"], b["cnt"])
     np.testing.assert_array_equal(a["b"], b["b"])
+
+
+@pytest.mark.parametrize("prec", PRECISIONS)
+@pytest.mark.parametrize("collisions", [False, True])
+def test_moved_tube_with_other_heating_tables(prec, collisions):
+    """A tube whose replayed steps were captured while lambdaPerp was zero and
+    the two spectral indices equal moves to tables where neither holds: the
+    replays after the move kick as the direct launches do."""
+    def run(graph):
+        mi, spec, tube, vg = grids.config_small(n_particles=6000, three_d=True,
+                                                steps_per_master=4, heating=True,
+                                                collisions=collisions)
+        mi.precision = prec
+        s = Solver(mi, [tube], vg)
+        s.load(0, *grids.initial_particles(tube, spec, mi, seed=11))
+        s.set_graph(graph)
+        s.step(10)  # the master steps 4 and 8 captured, 8 replayed or packed
+        new = grids.moved_tube(spec, mi, tube, spec.L + 0.05)
+        new.lambdaPerp = np.full(tube.nq, 20.0)  # below the gyroradius
+        new.ChiPerp2 = new.ChiPerp1 - 1.2
+        s.update_tube(0, new)
+        s.step(31)  # the move at step 12
+        out = [s.particles()[k] for k in ("q", "vpar", "vperp1", "vperp2")] + [s.moments_all()]
+        s.close()
+        return out
+    for x, y in zip(run(False), run(True)):
+        np.testing.assert_array_equal(x, y)
