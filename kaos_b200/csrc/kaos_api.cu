@@ -217,7 +217,9 @@ struct kaos_handle {
   WorkMap rmap;  // the same for runs of steps (run_chunk)
   int wsel = 1;          // chosen map (CHUNKS[wsel] ions per item)
   int persistent = 0;    // persistent grid striding over the items
-  int tune_pending = 2;  // autotuner: 2 nothing timed yet, 1 the ordinary push not yet
+  // autotuner: what is still to be timed
+  enum { TUNE_ORDINARY = 1, TUNE_MASTER = 2 };
+  int tune_pending = TUNE_ORDINARY | TUNE_MASTER;
   int tune_singles = 0;  // ordinary steps made one by one since
   int forced = 0;        // shape given by kaos_set_launch
   int regsel = 0;        // mixed push register budget: 0 = 64, 1 = 80, 2 = 72
@@ -1176,20 +1178,25 @@ int run_steps(kaos_handle *h, int64_t g) {
 // The one-step push of ordinary steps is timed (ions per work item x one
 // block per item or a persistent grid x register budget) only for a handle
 // that uses it: its interval converts ions, or it has made TUNE_AFTER
-// ordinary steps that were no part of a run.  Else only the master-step
-// variant is, which every handle uses: the budgets at 4096 ions per item, the
-// smaller items at the best of them (no persistent grid: 182 us against 179 at
-// its best for the ordinary push of 1e7 ions).  At 1e7 ions 15 launches of
-// 0.35 ms in place of 54 of 0.2 and 9 of 0.39.
+// ordinary steps that were no part of a run.
+//
+// The master-step variant, which every handle uses, is timed directly before a
+// master step and at no other time: its pushes fill the binning accumulators,
+// which hold the counts of the latest master step (kaos_get_counts) until that
+// step clears them.  With the shape chosen by the ordinary push only its
+// register budget is left to choose; without, the budgets are timed at 4096
+// ions per item, the smaller items at the best of them (no persistent grid:
+// 182 us against 179 at its best for the ordinary push of 1e7 ions).  At 1e7
+// ions 15 launches of 0.35 ms in place of 54 of 0.2 and 9 of 0.39.
 constexpr int TUNE_AFTER = 4;
-int autotune(kaos_handle *h, bool ordinary) {
+int autotune(kaos_handle *h, bool master) {
   // (items of 256 ions, push_args: only the register budget is left to choose)
   const bool fine = h->rmap.chunk == 256 && !h->forced;
+  const bool shaped = fine || !(h->tune_pending & kaos_handle::TUNE_ORDINARY);
   const int nreg = h->mixed ? 3 : 1;
-  if (fine && nreg == 1) {  // nothing to choose
-    h->tune_pending = 0;
-    return KAOS_OK;
-  }
+  h->tune_pending &= ~(master ? kaos_handle::TUNE_MASTER : kaos_handle::TUNE_ORDINARY);
+  if (nreg == 1 && (master ? shaped : fine)) return KAOS_OK;  // nothing to choose
+  const int old[4] = {h->wsel, h->persistent, h->regsel, h->regsel_master};
   const int other = 1 - h->cur;
   const Fields F = ion_fields(h, h->cur, other);
   for (int f = 0; f < F.n; ++f)
@@ -1199,9 +1206,8 @@ int autotune(kaos_handle *h, bool ordinary) {
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   // time of one push with the shape now set in the handle (best of two after
-  // a warm-up); a master-step push fills binning accumulators that are
-  // cleared before the next master step uses them
-  auto time_push = [&](bool master, float *tmin) -> int {
+  // a warm-up)
+  auto time_push = [&](float *tmin) -> int {
     PushArgs a = push_args(h);
     a.ion = h->ion[other];
     a.step = (uint32_t)(h->n + 1);
@@ -1227,7 +1233,7 @@ int autotune(kaos_handle *h, bool ordinary) {
   };
   float best = 1e30f, t = 0.f;
   int rc;
-  if (ordinary) {
+  if (!master) {
     int bw = h->wsel, bp = h->persistent, br = h->regsel;
     for (int m = 0; m < (fine ? 1 : NCHUNKS); ++m)
       for (int pm = 0; pm < (fine ? 1 : 2); ++pm)
@@ -1235,39 +1241,38 @@ int autotune(kaos_handle *h, bool ordinary) {
           h->wsel = m;
           h->persistent = pm;
           h->regsel = rs;
-          if ((rc = time_push(false, &t))) return rc;
+          if ((rc = time_push(&t))) return rc;
           if (t < best) { best = t; bw = m; bp = pm; br = rs; }
         }
     h->wsel = bw;
     h->persistent = bp;
     h->regsel = h->regsel_master = br;
+    h->tune_pending |= kaos_handle::TUNE_MASTER;  // its budget in this shape
   } else {
-    if (!fine) h->wsel = NCHUNKS - 1;
-    h->persistent = 0;
-    h->regsel = h->mixed ? 1 : 0;
-  }
-  // the master-step variant (field re-interpolation and binning) has its
-  // own register needs: its budget is timed separately
-  if (h->mixed || !ordinary) {
+    if (!shaped) h->wsel = NCHUNKS - 1;
+    if (h->tune_pending & kaos_handle::TUNE_ORDINARY) {
+      h->persistent = 0;
+      h->regsel = h->mixed ? 1 : 0;
+    }
     int bm = 0, bw = h->wsel;
-    best = 1e30f;
     for (int rs = 0; rs < nreg; ++rs) {
       h->regsel_master = rs;
-      if ((rc = time_push(true, &t))) return rc;
+      if ((rc = time_push(&t))) return rc;
       if (t < best) { best = t; bm = rs; }
     }
     h->regsel_master = bm;
-    for (int m = NCHUNKS - 2; m >= 0 && !ordinary && !fine; --m) {
+    for (int m = NCHUNKS - 2; m >= 0 && !shaped; --m) {
       h->wsel = m;
-      if ((rc = time_push(true, &t))) return rc;
+      if ((rc = time_push(&t))) return rc;
       if (t < best) { best = t; bw = m; }
     }
     h->wsel = bw;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  h->tune_pending = ordinary ? 0 : 1;
-  drop_graphs(h);
+  if (old[0] != h->wsel || old[1] != h->persistent || old[2] != h->regsel ||
+      old[3] != h->regsel_master)
+    drop_graphs(h);
   return KAOS_OK;
 }
 
@@ -1894,7 +1899,7 @@ int kaos_set_graph(kaos_handle *h, int32_t on) {
 int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode) {
   if (!h) return KAOS_ERR_PARAM;
   if (chunk == 0 || mode < 0) {
-    h->tune_pending = 2;
+    h->tune_pending = kaos_handle::TUNE_ORDINARY | kaos_handle::TUNE_MASTER;
     h->tune_singles = 0;
     h->forced = 0;
     return KAOS_OK;
@@ -2024,11 +2029,15 @@ int kaos_step(kaos_handle *h, int64_t nsteps) {
     if (h->tune_pending && n >= 2) {
       const bool ordinary = (h->P.QEXCHANGEflag == 1 && !h->cx_idle) ||
                             h->tune_singles >= TUNE_AFTER;
-      if ((ordinary || h->tune_pending == 2) && (rc = autotune(h, ordinary))) return rc;
+      if ((h->tune_pending & kaos_handle::TUNE_ORDINARY) && ordinary && (rc = autotune(h, false)))
+        return rc;
+      if ((h->tune_pending & kaos_handle::TUNE_MASTER) && is_master(h, n) &&
+          (rc = autotune(h, true)))
+        return rc;
     }
     const int64_t r = run_length(h, n, nsteps - k);
     if (r > 0) {
-      if (r == 1 && h->tune_pending) ++h->tune_singles;
+      if (r == 1 && (h->tune_pending & kaos_handle::TUNE_ORDINARY)) ++h->tune_singles;
       if ((rc = run_steps(h, r))) return rc;
       k += r;
       continue;

@@ -107,3 +107,42 @@ def test_single_steps_choose_their_shape(prec):
     assert a.launch()[0] in (1024, 2048, 4096) and b.launch()[0] in (1024, 2048, 4096)
     for x, y in zip(_state(a, 1), _state(b, 1)):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("slots", [0, (1 << 21) + 1000])
+@pytest.mark.parametrize("collisions", [False, True])
+def test_counts_hold_between_master_steps(prec, slots, collisions):
+    """kaos_get_counts returns the counts of the latest master step whatever
+    has been stepped since -- the launch-shape timing among it, which runs at
+    the first steps and again after single steps -- and a launch shape set by
+    hand (no timing at all) gives the same ones."""
+    mi = ModelInput(h=0.01, ndatfac=5, ION2VPERPflag=1, ICRflag=1, precision=prec,
+                    QEXCHANGEflag=1 if collisions else 0)
+    spec = TubeSpec(L=3.0, nq=24, n_particles=30000, q_ub=0.5, H=400e3, heat_rate_eV_s=2.0,
+                    neut_n0=1e18 if collisions else 0.0, neut_H=300e3)
+    t = make_tube(spec, mi)
+    t.capacity = max(t.capacity, slots)
+    vg = make_vgrid(True, 8, 8, 12, 9e3)
+    init = [grids.initial_particles(t, spec, mi, seed=3)]
+    s, f = _solver(mi, [t], init, vg), _solver(mi, [t], init, vg)
+    f.set_launch(2048, 0)
+    for x in (s, f):
+        x.set_export(True)
+    last = None
+    for n in range(1, 18):
+        s.step(1)
+        f.step(1)
+        now = [s.counts(), s.counts(full=True)]
+        if n == 1 or n % 5 == 0:
+            last = now
+        for x, y, z in zip(now, last, (f.counts(), f.counts(full=True))):
+            np.testing.assert_array_equal(x, y, err_msg=str(n))
+            np.testing.assert_array_equal(x, z, err_msg=str(n))
+    assert last[0].sum() > 0
+    s.set_launch(0, 0)  # timed again, in the middle of an interval
+    s.step(1)
+    np.testing.assert_array_equal(s.counts(), last[0])
+    np.testing.assert_array_equal(s.counts(full=True), last[1])
+    s.close()
+    f.close()
