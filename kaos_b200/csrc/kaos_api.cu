@@ -601,11 +601,15 @@ int apply_pending_tubes(kaos_handle *h) {
 }
 
 // A tube split across ranks: the caller's hook sums the binning
-// accumulators of all ranks in place before the moments are taken.
+// accumulators of all ranks in place before the moments are taken.  A getter
+// that the hook calls reads the device at this step; nothing it read serves
+// the rest of the call.
 int reduce_accum(kaos_handle *h) {
   if (!h->reduce_fn) return KAOS_OK;
   CK(cudaStreamSynchronize(h->s));
+  h->stat_ok = 0;
   const int rc = h->reduce_fn(h->reduce_ctx, h->acc_base, h->acc_len, (void *)h->s);
+  h->stat_ok = 0;
   if (rc) return fail(h, KAOS_ERR_CUDA, "accumulator reduction hook returned %d", rc);
   return KAOS_OK;
 }
@@ -1132,8 +1136,10 @@ int step_once(kaos_handle *h) {
     if (lb && ub)
       for (int k = 0; k < 2; ++k)
         if ((rc = launch_inject(h, k, h->s)) || (rc = commit_inject(h, k))) return rc;
-    if ((rc = reduce_accum(h)) ||
-        (rc = launch_moments(h, nn, beside ? 1 + (int)ub : 0)))
+    // committed with the moments, or before a hook, whose getters count it
+    const bool late = beside && !h->reduce_fn;
+    if (beside && !late && (rc = commit_inject(h, ub))) return rc;
+    if ((rc = reduce_accum(h)) || (rc = launch_moments(h, nn, late ? 1 + (int)ub : 0)))
       return rc;
   }
   h->n = n;

@@ -173,3 +173,33 @@ def test_split_tube_ena_rows_where_one_rank_converts_nothing():
     assert a.moments(KAOS_ENA_NQ).sum() > 0
     for s in solvers:
         s.close()
+
+
+def test_getters_inside_the_hook_see_the_step():
+    """A hook that asks for the handle's counts and boundary fluxes gets those
+    of the statistics step it is called for, the step's injection included, at
+    every call of one kaos_step."""
+    mi, spec, tube, vg = grids.config_small(n_particles=3000, three_d=True,
+                                            steps_per_master=4)
+    tube.nsnormCLB = 30.0
+    init = grids.initial_particles(tube, spec, mi, seed=22)
+    s = Solver(mi, [tube], vg)
+    seen = []
+
+    def hook(buf, count, stream):
+        seen.append((s.count(), tuple(s.boundary())))
+        return 0
+
+    s.set_reduce(hook)
+    s.load(0, *init)
+    s.step(13)
+    want = []
+    ref = Solver(mi, [tube], vg)
+    ref.load(0, *init)
+    for n in (1, 3, 4, 4):
+        ref.step(n)
+        want.append((ref.count(), tuple(ref.boundary())))
+    assert want[1][1][2] == 30
+    assert seen == want
+    s.close()
+    ref.close()
