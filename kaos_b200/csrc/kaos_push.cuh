@@ -703,6 +703,31 @@ __device__ __forceinline__ double quartic_newton_chord(double q, double ip,
   return fma(-f, r, u);
 }
 
+// The same root from a Runge-Kutta point, which has left the field line by the
+// square of the step over the radius.  One Newton step and a chord step are
+// exact to rounding while the first moves u by less than 2^-20 (the chord
+// step's error is 4.5 times that ratio's cube: 4e-18; a step of 7 km at one
+// Earth radius, where a 5 ms step of the benchmark tubes covers 10 m); a
+// longer step takes a second Newton step between the two.  (One chord step
+// for all left 3e-13 at a step of 1e-2 of the radius and 2e-10 at 3e-2.)
+__device__ __forceinline__ double quartic_newton_rk(double q, double ip, double u) {
+  const double q2 = q * q;
+  double u2 = u * u;
+  double f = fma(q2 * u2, u2, fma(u, ip, -1.0));
+  double r = (double)rcpa((float)fma(4.0 * q2 * u2, u, ip));
+  const double u0 = u;
+  u = fma(-f, r, u);
+  u2 = u * u;
+  f = fma(q2 * u2, u2, fma(u, ip, -1.0));
+  if (!(fabs(u - u0) <= 0x1p-20 * u)) {
+    r = (double)rcpa((float)fma(4.0 * q2 * u2, u, ip));
+    u = fma(-f, r, u);
+    u2 = u * u;
+    f = fma(q2 * u2, u2, fma(u, ip, -1.0));
+  }
+  return fma(-f, r, u);
+}
+
 // Cell search starting from the cell of the previous step (particles move a
 // small fraction of a cell per step); falls back to the bisection.
 __device__ __forceinline__ int cell_search_from(const double *E, int nq,
@@ -894,9 +919,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
     const double r2 = fma(xr, xr, xz * xz);
     const double ir = rsq(r2);
     const double qN = (RE * RE) * (xz * ir) * (ir * ir);
-    // (the Runge-Kutta point leaves the field line by the square of the step
-    // over the radius, 1e-12 for 10 m: the chord step only settles rounding)
-    const double u = quartic_newton_chord(qN, ipG, r2 * ir * (1.0 / RE));
+    const double u = quartic_newton_rk(qN, ipG, r2 * ir * (1.0 / RE));
     const double s2 = u * ipG;                 // sin^2(theta)
     const double st = s2 * rsq(s2);
     const double ctn = qN * u * u;

@@ -146,3 +146,28 @@ def test_counts_hold_between_master_steps(prec, slots, collisions):
     np.testing.assert_array_equal(s.counts(full=True), last[1])
     s.close()
     f.close()
+
+
+@pytest.mark.parametrize("drift", [1e-4, 3e-3, 1e-2, 3e-2])
+def test_fp64_long_steps_end_on_the_field_line(drift):
+    """One FP64 step of a given length over radius: the re-projected point lies
+    on the tube's field line, r = RE p sin^2(theta), to rounding -- the radius,
+    the root and the two coordinates carry a few units of 2^-53 each, eight in
+    all -- however far the Runge-Kutta point had left the line."""
+    mi = ModelInput(h=10.0, ndatfac=50, ION2VPERPflag=1)
+    spec = TubeSpec(L=4.0, nq=24, n_particles=2000, q_ub=0.15, H=600e3)
+    t = make_tube(spec, mi)
+    n = 2000
+    rng = np.random.default_rng(5)
+    q = rng.uniform(t.qGC[-4], t.qGC[3], n)
+    r = grids.dipole_q_to_rtheta(q, t.pG)[0]
+    v = drift * r / mi.h * rng.choice([-1.0, 1.0], n)
+    s = Solver(mi, [t], make_vgrid(True, 8, 8, 8, 1e6))
+    s.load(0, q, v, np.zeros(n), np.zeros(n))
+    s.step(1)
+    p = s.particles()
+    s.close()
+    rho, z = p["rho"].astype(np.longdouble), p["z"].astype(np.longdouble)
+    rr = np.sqrt(rho * rho + z * z)
+    off = rr * rr * rr / (grids.RE * t.pG * rho * rho) - 1
+    assert np.max(np.abs(off)) < 8 * 2.0 ** -52
