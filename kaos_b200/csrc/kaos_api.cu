@@ -478,9 +478,9 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
        k_push32<true, 256, 4, false, false, true, true, true>}};
   const KFn fn = run ? (h->mixed ? k32run[hk][h->three_d] : k64run[a.chunk > 256][ht][h->three_d])
                      : (h->mixed ? k32[hk][ms][h->three_d][rs][ps] : k64[ht][h->three_d][ps]);
-  // (static shared memory counts towards the 48 KB: up to 6.9 KB, the FP64
+  // (static shared memory counts towards the 48 KB: up to 13 KB, the FP64
   // push's bin edges and lookup tables and its kick's tables)
-  if (smem > 40 * 1024)
+  if (smem > 34 * 1024)
     CK(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int &occ = h->occ[h->mixed ? ms : 0][rs];
   if (ps && !occ) {
@@ -1010,6 +1010,7 @@ struct SampleArgs {
   int64_t n;
   double *out;
   uint32_t rk[20];  // Philox key schedule of the seed (as PushArgs.rk)
+  const double *kx;  // kx_tables_make's tables (KAOS_SAMPLE_GAUSS64)
 };
 
 int sample_width(int kind) {
@@ -1017,7 +1018,8 @@ int sample_width(int kind) {
 }
 
 __global__ void k_sample_rng(SampleArgs a) {
-  double *kt = kf_tables();
+  double *kt = kf_tables(), *xt = kx_tables();
+  if (a.kind == KAOS_SAMPLE_GAUSS64) kx_tables_fill(xt, a.kx);
   if (a.kind == KAOS_SAMPLE_GAUSS64T)
     for (int i = threadIdx.x; i <= KF_N; i += blockDim.x) kf_tables_make(kt, i);
   __syncthreads();
@@ -1034,7 +1036,7 @@ __global__ void k_sample_rng(SampleArgs a) {
       a.out[2 * i + 1] = g2;
     } else if (a.kind == KAOS_SAMPLE_GAUSS64) {
       double g1, g2;
-      gauss2_64(a.seed, id, a.step, KAOS_RNG_HEAT, g1, g2);
+      gauss2_64x(a.rk, xt, id, a.step, g1, g2);
       a.out[2 * i] = g1;
       a.out[2 * i + 1] = g2;
     } else if (a.kind == KAOS_SAMPLE_GAUSS64T) {
@@ -1659,7 +1661,11 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
   if ((rc = dalloc(h, &h->d_vbins, 1))) return rc;
   k_vbins<<<1, 256>>>(h->d_vbins, h->vg);
   CK(cudaGetLastError());
-  if (p->ICRflag == 1 && (!h->mixed || h->kick64)) {  // the FP64 kick's tables
+  if (p->ICRflag == 1 && !h->mixed) {  // the FP64 kick's tables
+    std::vector<double> t(KX_SIZE);
+    kx_tables_make(t.data());
+    if ((rc = upload(h, &h->d_kf, t))) return rc;
+  } else if (p->ICRflag == 1 && h->kick64) {
     if ((rc = dalloc(h, &h->d_kf, 3 * (KF_N + 1)))) return rc;
     k_kf_tables<<<1, 160>>>(h->d_kf);
     CK(cudaGetLastError());
@@ -2323,8 +2329,14 @@ int kaos_sample_rng(int32_t kind, uint64_t seed, uint64_t id0, uint32_t step,
     return KAOS_ERR_PARAM;
   if (n == 0) return KAOS_OK;
   const int per = sample_width(kind);
-  double *d = nullptr;
-  if (cudaMalloc(&d, (size_t)n * per * sizeof(double)) != cudaSuccess) return KAOS_ERR_CUDA;
+  double *d = nullptr, t[KX_SIZE];
+  const size_t len = (size_t)n * per;
+  if (cudaMalloc(&d, (len + KX_SIZE) * sizeof(double)) != cudaSuccess) return KAOS_ERR_CUDA;
+  kx_tables_make(t);
+  if (cudaMemcpy(d + len, t, sizeof t, cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFree(d);
+    return KAOS_ERR_CUDA;
+  }
   SampleArgs a{};
   a.kind = kind;
   a.seed = seed;
@@ -2334,6 +2346,7 @@ int kaos_sample_rng(int32_t kind, uint64_t seed, uint64_t id0, uint32_t step,
   a.lambda = lambda;
   a.n = n;
   a.out = d;
+  a.kx = d + len;
   for (int r = 0; r < 10; ++r) {  // Philox key schedule of the seed
     a.rk[2 * r] = (uint32_t)seed + (uint32_t)r * KAOS_PHILOX_W0;
     a.rk[2 * r + 1] = (uint32_t)(seed >> 32) + (uint32_t)r * KAOS_PHILOX_W1;
@@ -2341,7 +2354,7 @@ int kaos_sample_rng(int32_t kind, uint64_t seed, uint64_t id0, uint32_t step,
   k_sample_rng<<<(int)std::min<int64_t>((n + 255) / 256, 148 * 16), 256>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
-    e = cudaMemcpy(out, d, (size_t)n * per * sizeof(double), cudaMemcpyDeviceToHost);
+    e = cudaMemcpy(out, d, len * sizeof(double), cudaMemcpyDeviceToHost);
   cudaFree(d);
   return e == cudaSuccess ? KAOS_OK : KAOS_ERR_CUDA;
 }

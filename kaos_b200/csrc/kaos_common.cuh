@@ -193,6 +193,11 @@ __device__ __forceinline__ double rsq(double x) {
   const double e = fma(-fma(x, y, -t), y, fma(-t, y, 1.0));
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
+// sqrt(x) within ~0.5 ulp (x well inside the FP32 range).
+__device__ __forceinline__ double sqrt_near(double x) {
+  const double y = rsq_near(x), t = x * y;
+  return fma(fma(-t, t, x), 0.5 * y, t);
+}
 // FP32: one MUFU operation, denormals flushed (the FP32 geometry of the
 // mixed push never comes near the denormal range).
 __device__ __forceinline__ float rsq(float x) {

@@ -1,8 +1,8 @@
 // FP64 logarithm, base-2 exponential and sine/cosine of 2 pi u by table
-// reduction, for the heating kick of the mixed push in precision mode
-// KAOS_PREC_MIXED_K64 (the FP64 path's kick, _8_1_1_0_WaveHeating.f90:
-// 141-150, to FP64 accuracy at a fraction of the cost of the general FP64
-// library functions).
+// reduction, for the heating kick (_8_1_1_0_WaveHeating.f90:141-150) at a
+// fraction of the cost of the general FP64 library functions: kf_* for the
+// mixed push in precision mode KAOS_PREC_MIXED_K64, kx_* (at the end, to the
+// library functions' error) for the FP64 push.
 //
 // Method (table-driven reduction, as in Tang's table-driven logarithm and
 // exponential, ACM TOMS 15(2) 1989 and 16(4) 1990, here with one 129-entry
@@ -133,6 +133,92 @@ KF_HD void kf_sincos2pi(const double *cs, double u, double &s, double &c) {
   const double C = cs[2 * n], S = cs[2 * n + 1];
   c = C + fma(C, cm1, -S * sx);
   s = S + fma(S, cm1, C * sx);
+}
+
+// ---------------------------------------------------------------------------
+// Logarithm and exponential for the FP64 push's heating kick, whose draw and
+// amplitude are held to the error of the library functions they stand for
+// (0.5 - 1 unit in the last place, relative, for every argument): the same
+// reduction, with tables in two parts.
+//   ln: x = 2^e z, z in [0.71, 1.42), near c(j)^-1; c(j), j = 0 .. 127, is a
+//       reciprocal of 8 bits, so t = z c(j) - 1 (|t| < 7e-3) is exact, and
+//       is 1 on both sides of x = 1, where ln x is then log1p(t) alone;
+//       ln x = e ln2 - ln c(j) + log1p(t), the first two as a sum of
+//       multiples of 2^-42 (exact) and a remainder.
+//   exp: v = n ln2/128 + g; e^v = 2^(n >> 7) 2^((n & 127)/128) e^g, the table
+//       value as the sum of two doubles.
+//   sincos(2 pi u): as kf_sincos2pi, with the table's values as sums of two
+//       doubles, 2 pi too.
+// Layout: c(j), the high parts of -ln c(j), the low parts, the high and the
+// low parts of 2^(j/128), 128 each; then (cos, sin) of 2 pi j/128, high and
+// low parts, four a point.
+constexpr int KX_N = 128, KX_CS = 5 * KX_N, KX_SIZE = KX_CS + 4 * KX_N;
+constexpr double KX_TWO_PI_LO = 2.4492935982947064e-16;          // 2 pi - KF_TWO_PI
+constexpr double KX_LN2_HI = 3048493539143.0 / 4398046511104.0;  // 2^-42 multiples
+constexpr double KX_LN2_LO = 5.497923018708371e-14;              // ln2 - KX_LN2_HI
+
+// The tables, on the host, from the C library's long double functions.
+static inline void kx_tables_make(double *t) {
+  for (int j = 0; j < KX_N; ++j) {
+    const double m = 1.0 + j / 128.0;  // the middle of the values that use j
+    const double c = j < 54 ? rint(256.0 / m) / 256.0 : rint(256.0 / m) / 128.0;
+    const long double l = -logl((long double)c), p = exp2l((long double)j / KX_N);
+    const double hi = (double)(rintl(l * 0x1p42L) * 0x1p-42L);
+    t[j] = c;
+    t[KX_N + j] = hi;
+    t[2 * KX_N + j] = (double)(l - (long double)hi);
+    t[3 * KX_N + j] = (double)p;
+    t[4 * KX_N + j] = (double)(p - (long double)(double)p);
+    // (the quarter turns exactly: the angle from the nearest one)
+    const int q = (j + 16) / 32, r = j - 32 * q;
+    const long double a = 6.283185307179586476925286766559L * r / KX_N;
+    const long double cr = cosl(a), sr = sinl(a);
+    const long double cs[2] = {q & 1 ? (q & 2 ? sr : -sr) : (q & 2 ? -cr : cr),
+                               q & 1 ? (q & 2 ? -cr : cr) : (q & 2 ? -sr : sr)};
+    for (int k = 0; k < 2; ++k) {
+      t[KX_CS + 4 * j + k] = (double)cs[k];
+      t[KX_CS + 4 * j + 2 + k] = (double)(cs[k] - (long double)(double)cs[k]);
+    }
+  }
+}
+
+// ln x of a positive normal x.
+KF_HD double kx_ln(const double *t, double x) {
+  const uint64_t b = kf_bits(x), r = b + 0x0000100000000000ull;  // to the nearest j
+  const int j = (int)(r >> 45) & (KX_N - 1);
+  const int e = (int)(r >> 52) - 1023 + (j >= 54 ? 1 : 0);
+  const double z = kf_from_bits(b - ((uint64_t)(int64_t)e << 52));
+  const double f = fma(z, t[j], -1.0), ed = (double)e;
+  const double p = fma(f, fma(f, fma(f, fma(f, fma(f, fma(f, -1.0 / 8.0, 1.0 / 7.0), -1.0 / 6.0),
+                                            0.2), -0.25), 1.0 / 3.0), -0.5);
+  const double w = fma(ed, KX_LN2_HI, t[KX_N + j]);  // exact
+  const double h = w + f, l = (w - h) + f;           // |w| > |f| or w = 0
+  return h + (l + fma(f * f, p, fma(ed, KX_LN2_LO, t[2 * KX_N + j])));
+}
+
+// e^v for |v| < 690.
+KF_HD double kx_exp(const double *t, double v) {
+  const double nd = rint(v * (128.0 * KF_LOG2E));
+  const int n = (int)nd;
+  const double g = fma(nd, -KX_LN2_LO / 128.0, fma(nd, -KX_LN2_HI / 128.0, v));
+  const double em1 =
+      g * fma(g, fma(g, fma(g, fma(g, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0);
+  const double P = t[3 * KX_N + (n & (KX_N - 1))];
+  return (P + fma(P, em1, t[4 * KX_N + (n & (KX_N - 1))])) * kf_pow2i(n >> 7);
+}
+
+// cos and sin of 2 pi u for u in [0, 1].
+KF_HD void kx_sincos2pi(const double *t, double u, double &s, double &c) {
+  const double nd = rint(u * 128.0);
+  const double f = fma(nd, -1.0 / 128.0, u);  // exact
+  const double x = fma(f, KF_TWO_PI, f * KX_TWO_PI_LO), x2 = x * x;
+  const double sx = fma(x * x2, fma(x2, fma(x2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), x);
+  const double cm1 =
+      x2 * fma(x2, fma(x2, fma(x2, 1.0 / 40320.0, -1.0 / 720.0), 1.0 / 24.0), -0.5);
+  const double *p = t + KX_CS + 4 * ((int)nd & (KX_N - 1));
+  const double C = p[0], S = p[1];
+  c = C + fma(-S, sx, fma(C, cm1, p[2]));
+  s = S + fma(C, sx, fma(S, cm1, p[3]));
 }
 
 }  // namespace kaos

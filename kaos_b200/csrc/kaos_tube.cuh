@@ -890,12 +890,6 @@ struct ConvArgs {
   int mixed;
 };
 
-// sqrt(x) within ~0.5 ulp (x well inside the FP32 range).
-__device__ __forceinline__ double sqrt_near(double x) {
-  const double y = rsq_near(x), t = x * y;
-  return fma(fma(-t, t, x), 0.5 * y, t);
-}
-
 // sqrt(B_new / B_old) at q, u_old = r/RE on the old line and u_new on the new
 // one, |B| going as sqrt(1 + 3 cos^2) / u^3: the quotient formed once, its
 // reciprocal from an FP32 seed with one third-order step and the quotient's

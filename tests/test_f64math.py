@@ -131,3 +131,61 @@ def test_log_form_kick_equals_the_reference_form():
     edge = np.abs(h * Om * s / (2.0 * np.pi) - 1.0) < 1e-12
     assert np.array_equal(on_ref[~edge], on_log[~edge])
     np.testing.assert_allclose(2.0 ** E, ref, rtol=1e-12)
+
+
+EXACT = r"""
+int main() {
+  double t[KX_SIZE];
+  kx_tables_make(t);
+  const long double twopi = 6.283185307179586476925286766559L;
+  const int N = 1000000;
+  double e_ln = 0, e_exp = 0, e_sc = 0;
+  for (int k = 0; k < N; ++k) {
+    // ln: uniforms, both sides of 1 near and next to it, many octaves
+    const double x[5] = {urand(), 1.0 - 0.03 * urand(), 1.0 + 0.03 * urand(),
+                         1.0 - (double)(k % 65536 + 1) * 0x1.0p-53, exp2(200.0 * (urand() - 0.5))};
+    for (double v : x)
+      if (v != 1.0) e_ln = fmax(e_ln, rel(kx_ln(t, v), logl((long double)v)));
+    // x^-c of the kick's ratios, and the ends of the range
+    const double E[2] = {8.0 * (urand() - 0.5), 1370.0 * (urand() - 0.5)};
+    for (double v : E) e_exp = fmax(e_exp, rel(kx_exp(t, v), expl((long double)v)));
+    double s, c, u = urand();
+    kx_sincos2pi(t, u, s, c);
+    const int q = (int)rint(4.0 * u);
+    const long double a = twopi * ((long double)u - 0.25L * q);
+    const long double cr = cosl(a), sr = sinl(a);
+    const long double C = q & 1 ? (q & 2 ? sr : -sr) : (q & 2 ? -cr : cr);
+    const long double S = q & 1 ? (q & 2 ? -cr : cr) : (q & 2 ? -sr : sr);
+    e_sc = fmax(e_sc, fmax((double)fabsl(c - C), (double)fabsl(s - S)));
+  }
+  double s, c;  // exact at the quarter turns
+  for (int q = 0; q <= 4; ++q) {
+    kx_sincos2pi(t, 0.25 * q, s, c);
+    const double C[5] = {1, 0, -1, 0, 1}, S[5] = {0, 1, 0, -1, 0};
+    if (c != C[q] || s != S[q]) e_sc = 1.0;
+  }
+  if (kx_ln(t, 1.0) != 0.0 || kx_exp(t, 0.0) != 1.0) e_ln = 1.0;
+  printf("%.4e %.4e %.4e\n", e_ln, e_exp, e_sc);
+  return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_fp64_push_functions_to_the_last_place(tmp_path):
+    """The FP64 push's logarithm, exponential, sine and cosine: half a unit of
+    the result's rounding, and a twentieth of a unit for what comes before it
+    (terms of at most 2^-7 of the result, with a rounding each), relative for
+    the first two over their whole ranges -- next to 1 too, where the
+    logarithm is small -- and absolute against 1 for the last two (whose
+    results lie below 1, so that half a unit is 2^-54)."""
+    src = tmp_path / "f64exact.cpp"
+    src.write_text(DRIVER[:DRIVER.index("int main()")] + EXACT)
+    exe = tmp_path / "f64exact"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-I", HEADER_DIR, str(src), "-o", str(exe),
+                    "-lm"], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+    e_ln, e_exp, e_sc = (float(t) for t in out.split())
+    assert e_ln < 0.55 * 2.0 ** -52, e_ln
+    assert e_exp < 0.55 * 2.0 ** -52, e_exp
+    assert e_sc < 0.60 * 2.0 ** -53, e_sc

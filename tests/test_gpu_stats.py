@@ -254,3 +254,80 @@ def test_distribution_function_ks():
     assert len(pv) >= 30
     assert np.mean(pv < 0.01) <= 0.05, np.sort(pv)[:10]
     assert pv.min() > 1e-5
+
+
+@pytest.mark.parametrize("lam,chi2", [(0.0, 1.7), (20.0, 0.9), (-20.0, 1.7)])
+def test_fp64_kick_against_extended_precision(lam, chi2):
+    """One FP64 step's kick, ion by ion, against the reference's formula in
+    64-bit mantissas on the same Philox words: the sum of the roundings on its
+    way -- the position's two coordinates and the seven operations of Omega
+    (times 0.6), the exponent's four, the roots', the product's and the draw's
+    eight -- stays below 16 units of 2^-52 of the kick's own size, also where
+    the draw's uniform is next to 1 and the radius small.  A negative
+    lambdaPerp leaves the Sigma factor out (Sigma < 1)."""
+    LD = np.longdouble
+    pi = LD("3.14159265358979323846264338327950288")
+    mi = grids.ModelInput(h=0.005, ndatfac=50, ION2VPERPflag=1, ICRflag=1, EAMBflag=0, GRAVflag=0)
+    spec = grids.TubeSpec(L=4.0, nq=97, n_particles=1000, q_ub=1e-3, heat_rate_eV_s=1e-3)
+    t = grids.make_tube(spec, mi)
+    t.lambdaPerp, t.ChiPerp2 = np.full(t.nq, lam), np.full(t.nq, chi2)
+    n = 1 << 19
+    t.capacity = n
+    rng = np.random.default_rng(3)
+    q = rng.uniform(t.qGC[-2], t.qGC[1], n)
+    vpar = rng.normal(size=n) * 2e3 * 10.0 ** rng.uniform(-3, 1, n)
+    v = rng.normal(size=(2, n)) * 3e3 if lam else np.zeros((2, n))
+    s = Solver(mi, [t], grids.make_vgrid(True, 16, 16, 16, 1e5))
+    s.load(0, q, vpar, *v)
+    s.step(1)
+    got = s.state()
+    s.close()
+    w = klib.sample_rng(klib.SAMPLE_PHILOX, n, seed=mi.seed, id0=0, step=1,
+                        c3=1 << 24).astype(np.uint64)
+    u = [(((w[:, k] << np.uint64(32)) | w[:, k + 1]) >> np.uint64(11)).astype(float) + 0.5
+         for k in (0, 2)]
+    u1, u2 = (x * 2.0 ** -53 for x in u)
+    assert np.max(u1) > 1 - 1e-5
+    R = np.sqrt(-2 * np.log(u1.astype(LD)))
+    k = np.rint(4 * u2)
+    a = 2 * pi * (u2.astype(LD) - k.astype(LD) / 4)
+    c_, s_ = np.cos(a), np.sin(a)
+    k = k.astype(int) & 3
+    g = [R * np.choose(k, [c_, -s_, -c_, s_]), R * np.choose(k, [s_, c_, -s_, -c_])]
+    Q, pG, r0 = q.astype(LD), LD(t.pG), LD(grids.RE)
+    x = np.full(n, LD(1.5))
+    for _ in range(20):
+        x = x - (Q * Q * x ** 4 + x / pG - 1) / (4 * Q * Q * x ** 3 + 1 / pG)
+    ell = 1 + 3 * (Q * x * x) ** 2
+    Om = LD(mi.qs) / LD(mi.ms) * LD(8.06e15) * np.sqrt(ell) / (x * r0) ** 3
+    cell = np.clip(np.searchsorted(-t.qGH, -q), 0, t.nq - 1)
+    y = Om * np.abs(vpar.astype(LD)) / LD(t.sumdsICR)
+    on = y <= (2 * pi / LD(mi.h)) ** 2
+    amp = np.sqrt(np.sqrt(y))
+    if lam > 0:
+        sig = 2 * pi * np.sqrt(v[0].astype(LD) ** 2 + v[1].astype(LD) ** 2) / (Om * LD(lam))
+        amp = np.where(sig >= 1, amp * sig ** LD(-1.5), amp)
+        on &= np.abs(sig - 1) > 1e-12  # (the factor jumps there)
+    pre = (LD(mi.qs) ** 2 / (2 * LD(mi.ms) ** 2)) * t.S0[cell] * t.EtaLH[cell]
+    for key, v0, xi, chi, gi in (("vperp1", v[0], t.XiPerp1, t.ChiPerp1, g[0]),
+                                 ("vperp2", v[1], t.XiPerp2, t.ChiPerp2, g[1])):
+        kick = LD(mi.h) * np.sqrt(pre * xi[cell] / LD(np.pi)) * amp * gi * \
+            (Om / t.OmegaG0[cell].astype(LD)) ** (-chi[cell].astype(LD) / 2)
+        scale = np.abs(v0) + np.abs(kick)
+        use = on & (np.abs(gi) > 1e-6 * R)  # (a zero of the sine has no relative error)
+        err = (np.abs(got[key] - (v0 + kick)) / scale)[use]
+        assert np.max(err) < 16 * 2.0 ** -52, key
+
+
+def test_fp64_pair_radius_next_to_zero():
+    """The radius of the FP64 push's Gaussian pair, relative, against 64-bit
+    mantissas on the same Philox words, uniforms next to 1 among them: a
+    quarter unit of 2^-52 from the logarithm and half a unit each from the
+    root, the products and the sine and cosine."""
+    n = 1 << 21
+    g = klib.sample_rng(klib.SAMPLE_GAUSS64, n, seed=77, id0=5, step=9).astype(np.longdouble)
+    w = klib.sample_rng(klib.SAMPLE_PHILOX, n, seed=77, id0=5, step=9, c3=1 << 24).astype(np.uint64)
+    u1 = ((((w[:, 0] << np.uint64(32)) | w[:, 1]) >> np.uint64(11)).astype(float) + 0.5) * 2.0 ** -53
+    assert np.max(u1) > 1 - 1e-5
+    R = np.sqrt(-2 * np.log(u1.astype(np.longdouble)))
+    assert np.max(np.abs(np.sqrt((g ** 2).sum(axis=1)) / R - 1)) < 2 * 2.0 ** -52
