@@ -295,12 +295,11 @@ template <typename T> struct HeatC {
 // eps = |V|/(Omega sum ds), tau = 1/((Omega/2pi) sqrt eps) and the kick
 // (h/tau) sqrt(2 D_i tau) G_i, the algebra reduces to
 //   kick_i = K_i x^(-chi_i/2) Sigma^(-3/2) sqrt(Omega s) G_i,  s = sqrt(eps),
-// applied while h <= tau, i.e. h Omega s <= 2 pi, in the stochastic branch
-// (heat64x, heat64t and heat32); the coherent branch, here, kicks |Vperp| by
-// sqrt(k1^2+k2^2) G1 with a uniform gyro-angle.  invOm = 1/Omega is passed in
-// (no division needed).
+// applied while h <= tau, i.e. h Omega s <= 2 pi (stochastic branch);
+// the coherent branch kicks |Vperp| by sqrt(k1^2+k2^2) G1 with a uniform
+// gyro-angle.  invOm = 1/Omega is passed in (no division needed).
 template <typename T>
-__device__ __forceinline__ void heat_coherent(const PushArgs &a, uint32_t step,
+__device__ __forceinline__ void heat(const PushArgs &a, uint32_t step,
                                      const HeatC<T> &c, uint64_t id,
                                      T invsumds, T Om, T invOm, T vparabs,
                                      T &v1, T &v2) {
@@ -328,22 +327,31 @@ __device__ __forceinline__ void heat_coherent(const PushArgs &a, uint32_t step,
       k2 *= f;
     }
   }
-  T G1;
+  T G1, G2;
   if (f64) {
     double g1, g2;
     gauss2_64(a.seed, id, step, KAOS_RNG_HEAT, g1, g2);
     G1 = (T)g1;
+    G2 = (T)g2;
   } else {
     float g1, g2;
     gauss2_32(a.seed, id, step, KAOS_RNG_HEAT, g1, g2);
     G1 = (T)g1;
+    G2 = (T)g2;
   }
-  const T vpn = fabs(sqrt(v1 * v1 + v2 * v2) + sqrt(k1 * k1 + k2 * k2) * G1);
-  kaos_u32x4 r = kaos_philox((uint32_t)id, (uint32_t)(id >> 32), step,
-                             (KAOS_RNG_HEAT << 24) | 2u, a.seed);
-  const T ga = (T)kaos_u01(r.v[0], r.v[1]) * T(2.0 * PI);
-  v1 = vpn * cos(ga);
-  v2 = vpn * sin(ga);
+  if (a.icrcoh) {
+    const T vpn = fabs(sqrt(v1 * v1 + v2 * v2) + sqrt(k1 * k1 + k2 * k2) * G1);
+    kaos_u32x4 r = kaos_philox((uint32_t)id, (uint32_t)(id >> 32), step,
+                               (KAOS_RNG_HEAT << 24) | 2u, a.seed);
+    const T ga = (T)kaos_u01(r.v[0], r.v[1]) * T(2.0 * PI);
+    v1 = vpn * cos(ga);
+    v2 = vpn * sin(ga);
+    return;
+  }
+  if (a.h * (double)(Om * s) <= 2.0 * PI) {
+    v1 = v1 + k1 * G1;
+    v2 = v2 + k2 * G2;
+  }
 }
 
 // Philox4x32-10 (include/kaos_philox.h) with the key schedule, the same for
@@ -534,7 +542,7 @@ __device__ __forceinline__ void gauss2_mix(const uint32_t (&rk)[20], uint64_t id
 }
 
 // The stochastic WaveHeatingSub kick in the mixed push, in log form: the
-// product K_i x^(-c_i) (Om s)^(1/2) of the kick is one base-2 exponential,
+// product K_i x^(-c_i) (Om s)^(1/2) of heat() is one base-2 exponential,
 //   kick_i = K_i G_i 2^(-c_i log2(Om/Om0) + log2(Om |V||| / sum ds)/4 - pen),
 // the branch test h Om s <= 2 pi becomes Om |V||| / sum ds <= (2 pi/h)^2 and
 // Sigma^(-3/2) for lambda != 0 becomes pen = 1.5 log2 Sigma when Sigma >= 1,
@@ -971,7 +979,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push64(PushArgs a) {
         const double r = 1.0 / g1.ir;
         const double invOm = c_invOm * (r * r * r) * g1.isl;
         const HeatC<double> hc = heat_consts<double>(a.ct, (int64_t)T.coff + qi);
-        heat_coherent<double>(a, step, hc, pid, invsumds, Om, invOm, fabs(vpar), v1n, v2n);
+        heat<double>(a, step, hc, pid, invsumds, Om, invOm, fabs(vpar), v1n, v2n);
       }
     }
     // ---- k2: half step along V_R (KineticUpdateB) -----------------------
@@ -1363,7 +1371,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
         const float invOm = c_invOm * (rr * rr * rr) * g1.isl;
         const HeatC<float> hc{hk[0], hk[1], hk[2], hk[3], hk[4], hk[5]};
         float w1 = v1f, w2 = v2f;
-        heat_coherent<float>(a, step, hc, pid, invsumds, Om, invOm, fabsf(vparf), w1, w2);
+        heat<float>(a, step, hc, pid, invsumds, Om, invOm, fabsf(vparf), w1, w2);
         v1n = (double)w1;
         v2n = (double)w2;
       }
@@ -1512,7 +1520,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
         // FP64 kick at the start-of-step point: Omega = (q/m) MDIP sqrt(ell)
         // / r^3 and 1/Omega from the FP64 radius and 1/sqrt(ell) (yl), 1/r
         // from the FP32 reciprocal and one FP64 Newton step (relative error
-        // ~1e-14); the RK above used the pre-kick Vperp, as the FP64 push does
+        // ~1e-14); the RK above used the pre-kick Vperp, as heat() does
         const double r = u * RE;
         double ir = (double)rcpa((float)r);
         ir = ir * fma(-r, ir, 2.0);
@@ -1523,7 +1531,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
         } else {  // coherent branch: the general form
           const double invOm = c_invOm64 * (r * r * r) * yl;
           const HeatC<double> hc = heat_consts<double>(a.ct, (int64_t)T.coff + qi);
-          heat_coherent<double>(a, step, hc, pid, invsumds64, Om, invOm, fabs(vpar), v1n, v2n);
+          heat<double>(a, step, hc, pid, invsumds64, Om, invOm, fabs(vpar), v1n, v2n);
         }
       }
       if (!RUN) V12[k] = make_double2(v1n, v2n);
