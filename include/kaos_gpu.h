@@ -369,9 +369,10 @@ int kaos_set_graph(kaos_handle *h, int32_t on);
  * step at a time: before a step whose interval converts ions, or after four
  * ordinary steps made one by one.  The counts of the latest master step
  * (kaos_get_counts) are not touched by it.  Runs of steps
- * (kaos_step) have a shape of their own, and a handle of fewer than 2^21
- * slots takes items of 256 ions while no shape is set here (reported as 1024,
- * the smallest that can be set).  Results do not depend on the shape.  No reference counterpart (the reference has one MPI rank per core,
+ * (kaos_step) have a shape of their own, and a small handle (up to 2^18
+ * slots, fewer with more than 256 cells) takes items of 256 ions while no
+ * shape is set here (reported as 1024, the smallest that can be set).  Results
+ * do not depend on the shape.  No reference counterpart (the reference has one MPI rank per core,
  * _8_KineticSolver.f90:43-44). */
 int kaos_set_launch(kaos_handle *h, int32_t chunk, int32_t mode);
 

@@ -214,7 +214,8 @@ struct kaos_handle {
     int64_t *d_start = nullptr;
   };
   WorkMap wmap[NCHUNKS];
-  WorkMap rmap;  // the same for runs of steps (run_chunk)
+  WorkMap fmap;  // items of FINE ions: handles of fewer than FINE_SLOTS slots
+  int fine = 0;  // one-step pushes take them while no shape is set (fine_items)
   int wsel = 1;          // chosen map (CHUNKS[wsel] ions per item)
   int persistent = 0;    // persistent grid striding over the items
   // autotuner: what is still to be timed
@@ -303,16 +304,50 @@ int max_nq(const kaos_handle *h) {
   return m;
 }
 
-// Ions per work item of a run of steps (256-thread blocks, 4 per SM): one
-// ion per thread while that is what it takes to fill the SMs, four once there
-// are several waves of blocks, which then build their tube's tables a quarter
-// as often.  The 19-step runs of a master interval, us per interval: 1e6 ions
-// (97 cells) 256: 388, 1024: 401, 4096: 467; 1e7 ions (256 cells) 3193,
-// 3101, 3156; 256 uneven tubes, 5.7e7 ions 17700, 16970, 16870.
-int run_chunk(const kaos_handle *h) {
-  int64_t cap = 0;
-  for (const TubeD &T : h->th) cap += T.cap;
-  return cap < (int64_t)1 << 21 ? 256 : 1024;
+int64_t slots(const kaos_handle *h) {
+  int64_t n = 0;
+  for (const TubeD &T : h->th) n += T.cap;
+  return n;
+}
+
+static int sm_count(kaos_handle *h);
+
+// Items of 256 ions -- one ion per thread -- fill the SMs of a small handle,
+// and make every block build its tube's tables (88 - 108 bytes a cell in the
+// mixed push, 20 in the FP64 one) for that one ion per thread.
+constexpr int FINE = 256;
+constexpr int64_t FINE_SLOTS = (int64_t)1 << 21;
+
+// One-step pushes: a small handle's are latency, not throughput, and take the
+// small items while their tables stay few; else the autotuner chooses.  The
+// line lies where the two meet (us per step of converting intervals, small
+// items / tuned; 64, 512, 2048 cells): mixed, 1e5 ions 29 / 31, 48 / 54,
+// 75 / 58; 4e5 ions 37 / 35, 66 / 56, 152 / 76; 2e4 ions of 2048 cells 52 / 57;
+// FP64, 1e5 ions 35 / 39, 49 / 53, 59 / 60; 4e5 ions 56 / 55, 74 / 72, 89 / 81.
+bool fine_items(const kaos_handle *h) {
+  const int64_t n = slots(h);
+  return n <= (int64_t)1 << 18 && n * max_nq(h) <= (int64_t)1 << (h->mixed ? 26 : 27);
+}
+
+// Runs of steps (256-thread blocks, 4 per SM), ions per item: 256 below
+// FINE_SLOTS, 1024 above, where there are several waves of blocks, which then
+// build their tables a quarter as often.  Mixed runs of 19 steps, us per run
+// at 256, 1024, 4096 ions an item: 1e6 ions (97 cells) 251, 266, 344; 1e7 ions
+// (256 cells) 2333, 2256, 2327; 256 uneven tubes, 5.7e7 ions, 13260, 12600,
+// 12550; FP64, 1e5 ions 55, 115, 398, 1e7 ions 5564, 5473, 5674.  A short run of a tube of many cells in the mixed push
+// is mostly table building: four times the ions per item while a thread's
+// ion-steps in an item stay below two per 256 cells and the blocks still make
+// three waves (2 steps, 2048 cells, us per step at 256, 1024, 4096 ions an
+// item: 2e5 ions 37, 22, 29; 8e5 104, 54, 50; 1.5e6 193, 93, 76).
+const kaos_handle::WorkMap &run_map(kaos_handle *h, int64_t nsub) {
+  const kaos_handle::WorkMap *M[3] = {&h->fmap, &h->wmap[0], &h->wmap[NCHUNKS - 1]};
+  const int nq = max_nq(h);
+  int k = h->fmap.n ? 0 : 1;
+  if (!h->mixed) return *M[k];
+  const int64_t per_sm = std::min<int64_t>(4, std::max<int64_t>(1, 227 * 1024 / ((int64_t)88 * nq + 1024)));
+  const int64_t wave = per_sm * sm_count(h);
+  while (k < 2 && M[k]->chunk * nsub < 2 * (int64_t)nq && M[k]->n >= 3 * wave) ++k;
+  return *M[k];
 }
 
 // What the heating tables of a tube ask of the kick (PushArgs).  The flags are
@@ -326,14 +361,12 @@ void note_heating(kaos_handle *h, const kaos_tube_c &T) {
   if (h->heat_lam != lam || h->heat_chi != chi) drop_graphs(h);
 }
 
-PushArgs push_args(kaos_handle *h, bool run = false) {
+PushArgs push_args(kaos_handle *h, int64_t nsub = 1) {
   PushArgs a{};
   a.tubes = h->d_tubes;
-  // a small handle's single steps are latency, not throughput: one ion per
-  // thread in items of 256 unless the caller chose a shape (3e5 ions, every
-  // step a master step: push 28 us with items of 1024, 15 with 256)
-  const bool fine = run || (h->rmap.chunk == 256 && !h->forced);
-  const kaos_handle::WorkMap &M = fine ? h->rmap : h->wmap[h->wsel];
+  const kaos_handle::WorkMap &M = nsub > 1               ? run_map(h, nsub)
+                                  : h->fine && !h->forced ? h->fmap
+                                                          : h->wmap[h->wsel];
   a.blk_tube = M.d_tube;
   a.blk_start = M.d_start;
   a.nitems = M.n;
@@ -1166,7 +1199,7 @@ int64_t run_length(const kaos_handle *h, int64_t n, int64_t most) {
 int run_steps(kaos_handle *h, int64_t g) {
   const int64_t n = h->n + 1;
   const bool next_master = is_master(h, n + g);
-  PushArgs p = push_args(h, g > 1);
+  PushArgs p = push_args(h, g);
   p.step = (uint32_t)n;
   p.nsub = (unsigned)g;
   if (h->dstep_valid) p.dstep_w = h->d_step;
@@ -1194,12 +1227,13 @@ int run_steps(kaos_handle *h, int64_t g) {
 // step clears them.  With the shape chosen by the ordinary push only its
 // register budget is left to choose; without, the budgets are timed at 4096
 // ions per item, the smaller items at the best of them (no persistent grid:
-// 182 us against 179 at its best for the ordinary push of 1e7 ions).  At 1e7
-// ions 15 launches of 0.35 ms in place of 54 of 0.2 and 9 of 0.39.
+// 182 us against 179 at its best for the ordinary push of 1e7 ions; 1.5e6 ions
+// of 2048 cells, every step a master step, 219 us with and 214 without).  At
+// 1e7 ions 15 launches of 0.35 ms in place of 54 of 0.2 and 9 of 0.39.
 constexpr int TUNE_AFTER = 4;
 int autotune(kaos_handle *h, bool master) {
-  // (items of 256 ions, push_args: only the register budget is left to choose)
-  const bool fine = h->rmap.chunk == 256 && !h->forced;
+  // (small items, fine_items: only the register budget is left to choose)
+  const bool fine = h->fine && !h->forced;
   const bool shaped = fine || !(h->tune_pending & kaos_handle::TUNE_ORDINARY);
   const int nreg = h->mixed ? 3 : 1;
   h->tune_pending &= ~(master ? kaos_handle::TUNE_MASTER : kaos_handle::TUNE_ORDINARY);
@@ -1622,8 +1656,8 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
   };
   for (int m = 0; m < NCHUNKS; ++m)
     if ((rc = work_map(h->wmap[m], CHUNKS[m]))) return rc;
-  h->rmap = h->wmap[0];
-  if (h->rmap.chunk != run_chunk(h) && (rc = work_map(h->rmap, run_chunk(h)))) return rc;
+  if (slots(h) < FINE_SLOTS && (rc = work_map(h->fmap, FINE))) return rc;
+  h->fine = fine_items(h);
   if ((rc = dalloc(h, &h->d_nlive_new, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_next_id, ntubes))) return rc;
   if ((rc = dalloc(h, &h->d_blkcnt, bt.size()))) return rc;

@@ -171,3 +171,26 @@ def test_fp64_long_steps_end_on_the_field_line(drift):
     rr = np.sqrt(rho * rho + z * z)
     off = rr * rr * rr / (grids.RE * t.pG * rho * rho) - 1
     assert np.max(np.abs(off)) < 8 * 2.0 ** -52
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("nq,slots", [(2048, 0), (2048, 600_000), (700, 0), (24, 300_000)])
+def test_runs_of_many_cells(prec, nq, slots):
+    """Runs of two and of seventeen steps and one-step pushes on both sides of
+    the lines where the items grow with the cells, the slots and the run's
+    length, and of the small items of one-step pushes: bit for bit."""
+    mi = ModelInput(h=0.01, ndatfac=18, ION2VPERPflag=1, ICRflag=1, precision=prec)
+    spec = TubeSpec(L=4.0, nq=nq, n_particles=6000, q_ub=0.1, H=600e3, heat_rate_eV_s=5.0)
+    t = make_tube(spec, mi)
+    t.capacity = max(t.capacity, slots)
+    vg = make_vgrid(True, 16, 16, 24, 8e3)
+    init = [grids.initial_particles(t, spec, mi, seed=2)]
+    a, b = _solver(mi, [t], init, vg), _solver(mi, [t], init, vg)
+    for n in (1, 16, 1, 2, 15, 1):
+        a.step(n)
+        for _ in range(n):
+            b.step(1)
+    for x, y in zip(_state(a, 1), _state(b, 1)):
+        np.testing.assert_array_equal(x, y)
+    a.close()
+    b.close()
