@@ -334,11 +334,12 @@ bool fine_items(const kaos_handle *h) {
 // build their tables a quarter as often.  Mixed runs of 19 steps, us per run
 // at 256, 1024, 4096 ions an item: 1e6 ions (97 cells) 251, 266, 344; 1e7 ions
 // (256 cells) 2333, 2256, 2327; 256 uneven tubes, 5.7e7 ions, 13260, 12600,
-// 12550; FP64, 1e5 ions 55, 115, 398, 1e7 ions 5564, 5473, 5674.  A short run of a tube of many cells in the mixed push
-// is mostly table building: four times the ions per item while a thread's
-// ion-steps in an item stay below two per 256 cells and the blocks still make
-// three waves (2 steps, 2048 cells, us per step at 256, 1024, 4096 ions an
-// item: 2e5 ions 37, 22, 29; 8e5 104, 54, 50; 1.5e6 193, 93, 76).
+// 12550; FP64, 1e5 ions 55, 115, 398, 1e7 ions 5564, 5473, 5674.  A short run
+// of a tube of many cells in the mixed push is mostly table building: four
+// times the ions per item while an item has fewer than two ion-steps per cell
+// and the items make three waves of blocks (2 steps, 2048 cells, us per step at
+// 256, 1024, 4096 ions an item: 2e5 ions 37, 22, 29; 8e5 104, 54, 50; 1.5e6
+// 193, 93, 76).
 const kaos_handle::WorkMap &run_map(kaos_handle *h, int64_t nsub) {
   const kaos_handle::WorkMap *M[3] = {&h->fmap, &h->wmap[0], &h->wmap[NCHUNKS - 1]};
   const int nq = max_nq(h);
@@ -2049,7 +2050,8 @@ int kaos_set_id_base(kaos_handle *h, int32_t tube, uint64_t base) {
 
 int kaos_get_launch(kaos_handle *h, int32_t *chunk, int32_t *mode) {
   if (!h || !chunk || !mode) return KAOS_ERR_PARAM;
-  *chunk = CHUNKS[h->wsel];
+  // (small items are no shape that can be set: the smallest that can)
+  *chunk = CHUNKS[h->fine && !h->forced ? 0 : h->wsel];
   *mode = h->persistent | (h->regsel << 1) |
           (h->regsel_master != h->regsel ? (h->regsel_master + 1) << 3 : 0);
   return KAOS_OK;

@@ -10,7 +10,7 @@ from kaos_b200 import grids
 from kaos_b200.grids import TubeSpec, make_tube, make_vgrid
 from kaos_b200.lib import KaosError, Solver
 from kaos_b200.model_input import (KAOS_M0, KAOS_M1PAR, KAOS_M2, KAOS_M2PAR,
-                                   KAOS_PREC_MIXED, ModelInput)
+                                   KAOS_PREC_FP64, KAOS_PREC_MIXED, KAOS_PREC_MIXED_K64, ModelInput)
 from oracle.oracle import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -229,4 +229,21 @@ def test_charge_exchange_odd_cell_counts(nq):
     s, o = _run_one(mi, spec, make_vgrid(True, 16, 16, 24, 8e3), 7)
     assert s.count(0)[1] > 0
     _compare(s, 0, o)
+    s.close()
+
+
+@pytest.mark.parametrize("prec", [KAOS_PREC_FP64, KAOS_PREC_MIXED, KAOS_PREC_MIXED_K64])
+def test_reported_launch_shape_of_a_small_handle(prec):
+    """A handle below the small-item limit reports items of 1024 ions, the
+    smallest that can be set, and the reported shape can be set."""
+    mi, spec, t, vg = grids.config_small(n_particles=3000, heating=True, steps_per_master=4)
+    mi.precision = prec
+    s = Solver(mi, [t], vg)
+    s.load(0, *grids.initial_particles(t, spec, mi, seed=2))
+    for n in (1, 6, 1, 1, 1, 1, 1, 1):
+        s.step(n)
+        assert s.launch()[0] == 1024
+    s.set_launch(*s.launch())
+    s.step(3)
+    assert s.launch()[0] == 1024
     s.close()
