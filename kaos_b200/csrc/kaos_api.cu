@@ -454,9 +454,12 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
   }
   if (timed) CK(cudaEventRecord(h->pev[2 * h->npev], h->s));
   size_t smem = (size_t)(2 * nq + 1) * sizeof(double) + (size_t)nq * sizeof(unsigned);
-  if (h->mixed) smem += (size_t)nq * (sizeof(CellS) + sizeof(float2));
+  // heating: 0 none, 1 the FP32 kick (FP64 mode: its own), 2 the FP64 kick
+  const int hk = h->P.ICRflag == 1 ? 1 + h->kick64 : 0;
+  const size_t cell = hk == 2 ? sizeof(CellP) : sizeof(CellS);
+  if (h->mixed) smem += (size_t)nq * (cell + sizeof(float2));
   if (h->mixed && a.nsub > 1)  // a run: cell records and edges
-    smem = (size_t)nq * sizeof(CellS) + (size_t)(nq + 1) * sizeof(double);
+    smem = (size_t)nq * cell + (size_t)(nq + 1) * sizeof(double);
   else smem += (size_t)BIN_WIN * (1 + h->vg.npar + h->vg.n1 + (h->three_d ? h->vg.n2 : 0)) *
           sizeof(unsigned);  // block-private binning window
   const bool bins_variant = a.bin || a.prologue || a.bin_only || !h->three_d;
@@ -477,7 +480,6 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
    {KAOS_K32(true, false, K, H), KAOS_K32(true, true, K, H)}}
   // [no heating, FP32 kick, FP64 kick][master-step work][three_d][register
   // budget][persistent]
-  const int hk = h->P.ICRflag == 1 ? 1 + h->kick64 : 0;
   static const KFn k32[3][2][2][3][2] = {KAOS_K32S(false, false), KAOS_K32S(false, true),
                                          KAOS_K32S(true, true)};
 #undef KAOS_K32S

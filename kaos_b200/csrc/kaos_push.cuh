@@ -1113,12 +1113,18 @@ __device__ __forceinline__ bool well_inside(double o) {
 // 16-byte loads from one address (the arrays per quantity it replaces took a
 // load and an address each; 80 bytes a record keeps neighbouring cells'
 // loads on different banks).
-struct __align__(16) CellS {
+struct __align__(16) CellP {
   double ql, dq;   // lower edge, width in q
   double ul, ud;   // quadratic guess of the quartic root: uL, uH - uL
   double uc, idq;  // ... its curvature term; 1 / dq
+};
+struct __align__(16) CellS : CellP {
   float hk[8];     // heat32's constants
 };
+// The FP64 kick reads its constants from global memory: without heat32's, its
+// tables leave room beside 2048 cells and 128 bins per axis.
+template <bool K64> struct CellOf { using T = CellS; };
+template <> struct CellOf<true> { using T = CellP; };
 
 // ---------------------------------------------------------------------------
 // Mixed kernel: FP32 arithmetic on FP64 state.  The position is one FP64
@@ -1165,7 +1171,8 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
              bin_only = MASTER && a.bin_only;
   extern __shared__ __align__(16) double sm[];
   const int nqmax = a.nqs;
-  CellS *CS = (CellS *)sm;
+  using Cell = typename CellOf<K64>::T;
+  Cell *CS = (Cell *)sm;
   double *E = (double *)(CS + nqmax), *Cc = E + nqmax + 1;
   // the cell fields (EAmag, EG) of the field re-interpolation; the selection
   // counts (runs hold neither these nor the cell centres)
@@ -1211,7 +1218,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     for (int k = threadIdx.x; k < T.nq; k += blockDim.x) {
       const int64_t g = T.coff + k;
       const double ql = a.ct.qGL[g], qh = a.ct.qGH[g];
-      CellS &C = CS[k];
+      Cell &C = CS[k];
       C.ql = ql;
       C.dq = qh - ql;
       C.idq = 1.0 / (qh - ql);
@@ -1219,7 +1226,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
       C.ud = a.ct.uH[g] - a.ct.uL[g];
       // quadratic in the offset through the edges and the midpoint
       C.uc = 4.0 * a.ct.uM[g] - 2.0 * (a.ct.uL[g] + a.ct.uH[g]);
-      if (HEAT) {
+      if constexpr (HEAT && !K64) {
         const double lam = a.ct.lambdaPerp[g];
         C.hk[0] = (float)a.ct.hK1[g];
         C.hk[1] = (float)a.ct.hK2[g];
@@ -1356,7 +1363,7 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     double v1n = v1, v2n = v2;  // after the wave-heating kick
     // (the FP64 kick of K64 runs after the position and V|| stores below:
     // nothing before them reads the kicked pair)
-    if (!K64 && HEAT && qi >= 0) {
+    if constexpr (!K64 && HEAT) if (qi >= 0) {
       const float sl = g1.ell * g1.isl;
       const float ir3 = g1.ir * g1.ir * g1.ir;
       const float Om = qs_ms * (float)MDIP * sl * ir3;

@@ -2,6 +2,8 @@
 cells) and velocity grid (128 bins per axis) the library accepts, and
 batches holding an empty entry and a single-ion entry (injection fills
 the empty one)."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -246,4 +248,26 @@ def test_reported_launch_shape_of_a_small_handle(prec):
     s.set_launch(*s.launch())
     s.step(3)
     assert s.launch()[0] == 1024
+    s.close()
+
+
+def test_largest_tube_and_grid_fp64_kick():
+    """The FP64 kick's tables beside the tables of 2048 cells and the binning
+    window of 128 bins per axis."""
+    mi = ModelInput(h=0.01, ndatfac=3, ION2VPERPflag=1, ICRflag=1, precision=KAOS_PREC_MIXED_K64)
+    spec = TubeSpec(L=4.0, nq=2048, n_particles=20000, q_ub=1e-3, H=900e3, heat_rate_eV_s=5.0)
+    t = make_tube(spec, mi)
+    init = grids.initial_particles(t, spec, mi, seed=1)
+    vg = make_vgrid(True, 128, 128, 128, 8e3)
+    s = Solver(mi, [t], vg)
+    s.load(0, *init)
+    s.step(4)
+    o = Oracle(dataclasses.replace(mi, precision=KAOS_PREC_FP64), t, vg)
+    o.load(*init)
+    o.step(4)
+    assert s.count() == o.count()
+    assert rel_norm(s.moments(KAOS_M0), o.moments(KAOS_M0)) < 2e-2
+    po, ps = o.particles(), s.particles()
+    for key in ("vperp1", "vperp2"):
+        assert rel_norm(ps[key], po[key]) < 1e-6, key
     s.close()
