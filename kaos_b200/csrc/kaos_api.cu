@@ -202,9 +202,12 @@ struct kaos_handle {
   int rank = 0, nranks = 1;          // share of the charge-exchange counts
   std::vector<uint64_t> id_base;     // first ion id per tube
   // tube moves (kaos_update_tube) applied at the next master step
-  struct PendingTube {  // entry k's tables: row block k of conv_host.stage
+  // (entry k's tables: row block k of conv_host.stage, or its own until the
+  // first move has made the staging)
+  struct PendingTube {
     int tube;
     TubeD d;
+    std::vector<double> raw;
   };
   std::vector<PendingTube> pending;
   // push work items: (tube, chunk of ions) maps, one per candidate chunk
@@ -592,10 +595,11 @@ int conv_staging(kaos_handle *h) {
 int apply_pending_tubes(kaos_handle *h) {
   const int np = (int)h->pending.size();
   if (!np) return KAOS_OK;
-  const int nqm = max_nq(h);
+  const int nqm = max_nq(h), rc = conv_staging(h);
+  if (rc) return rc;
   // the moves' descriptors; their tables lie in the pinned staging since
   // kaos_update_tube, which runs between calls of kaos_step, so never while
-  // this copy is under way
+  // this copy is under way (the first moves' come from where they were kept)
   auto &S = h->conv_host;
   S.td.resize(np);
   S.tube.resize(np);
@@ -605,6 +609,7 @@ int apply_pending_tubes(kaos_handle *h) {
     S.td[p] = pt.d;
     S.tube[p] = pt.tube;
     S.pnew[p] = pt.d.pG;
+    std::copy(pt.raw.begin(), pt.raw.end(), S.stage + (size_t)p * CONV_RAW * nqm);
   }
   CK(cudaMemcpyAsync(h->d_conv_stage, S.stage, (size_t)np * CONV_RAW * nqm * sizeof(double),
                      cudaMemcpyHostToDevice, h->s));
@@ -2011,15 +2016,22 @@ int kaos_update_tube(kaos_handle *h, int32_t tube, const kaos_tube_c *T) {
   pt.d.sumdsICR = T->sumdsICR;
   host_rho_z(T->qGC[0], T->pG, &pt.d.rhoLB, &pt.d.zLB);
   host_rho_z(T->qGC[T->nq - 1], T->pG, &pt.d.rhoUB, &pt.d.zUB);
-  const int rc = conv_staging(h);
-  if (rc) return rc;
   note_heating(h, *T);
   size_t k = 0;
   while (k < h->pending.size() && h->pending[k].tube != tube) ++k;
-  if (k == h->pending.size()) h->pending.push_back(pt);
-  else h->pending[k] = pt;
+  if (k == h->pending.size()) h->pending.push_back(std::move(pt));
+  else h->pending[k] = std::move(pt);
   const int nqm = max_nq(h);
-  tube_tables(*T, h->conv_host.stage + k * CONV_RAW * nqm, nqm);
+  double *out = h->conv_host.stage;
+  if (out) {
+    // (a call of kaos_step that failed may have left a copy of it under way)
+    if (!h->stat_ok) CK(cudaStreamSynchronize(h->s));
+    out += k * CONV_RAW * nqm;
+  } else {
+    h->pending[k].raw.resize((size_t)CONV_RAW * nqm);
+    out = h->pending[k].raw.data();
+  }
+  tube_tables(*T, out, nqm);
   return KAOS_OK;
 }
 

@@ -268,3 +268,47 @@ def test_largest_tube_and_grid_fp64_kick():
     assert s.counts().sum() > 0
     s.close()
     small.close()
+
+
+def test_moves_before_the_first_master_step_and_after():
+    """Tube moves queued before any move has been made, one of them replaced
+    before it is, and later ones: two tubes of unequal cells end where single
+    moves of the same tables end."""
+    mi = ModelInput(h=0.01, ndatfac=3, ION2VPERPflag=1, ICRflag=1)
+    specs = [TubeSpec(L=L, nq=nq, n_particles=3000, q_ub=0.15, H=600e3, heat_rate_eV_s=5.0)
+             for L, nq in ((4.0, 24), (5.0, 31))]
+    tubes = [make_tube(sp, mi) for sp in specs]
+    vg = make_vgrid(True, 16, 16, 24, 8e3)
+    init = [grids.initial_particles(t, sp, mi, seed=1) for t, sp in zip(tubes, specs)]
+    moved = [[grids.moved_tube(sp, mi, t, sp.L + d) for d in (0.02, 0.05, -0.03)]
+             for t, sp in zip(tubes, specs)]
+
+    def make():
+        s = Solver(mi, tubes, vg)
+        for k, a in enumerate(init):
+            s.load(k, *a)
+        return s
+
+    a, b = make(), make()
+    a.update_tube(1, moved[1][2])  # replaced before the master step
+    a.update_tube(0, moved[0][0])
+    a.update_tube(1, moved[1][1])
+    a.step(4)
+    a.update_tube(1, moved[1][0])
+    a.step(5)
+    b.step(2)  # queued directly before the master step
+    b.update_tube(0, moved[0][0])
+    b.update_tube(1, moved[1][1])
+    b.step(3)
+    b.update_tube(1, moved[1][0])
+    b.step(4)
+    for k in range(2):
+        pa, pb = a.particles(k), b.particles(k)
+        for key in pa:
+            np.testing.assert_array_equal(pa[key], pb[key], err_msg=key)
+        np.testing.assert_array_equal(a.moments_all(k), b.moments_all(k))
+        r = np.hypot(pa["rho"], pa["z"])
+        p = moved[k][0].pG
+        assert np.max(np.abs(r ** 3 / (grids.RE * p * pa["rho"] ** 2) - 1)) < 1e-13
+    a.close()
+    b.close()
