@@ -556,7 +556,7 @@ void tube_tables(const kaos_tube_c &T, double *out, int nqm) {
       {T.qGL, 0}, {T.qGH, 0}, {T.qGC, 0}, {T.hqC, 0}, {T.dqC, 0}, {T.d3xC, 1}, {T.rGC, 0},
       {T.thetaGC, 0}, {T.ellGC, 1}, {T.TeG, 0}, {T.TsG, 0}, {T.nsnormCNeut, 0},
       {T.lambdaPerp, 0}, {T.EtaLH, 0}, {T.XiPerp1, 0}, {T.XiPerp2, 0}, {T.S0, 0},
-      {T.OmegaG0, 1}, {T.ChiPerp1, 0}, {T.ChiPerp2, 0}};
+      {T.OmegaG0, 0}, {T.ChiPerp1, 0}, {T.ChiPerp2, 0}};  // (1/OmegaG0 of none: 0)
   for (int k = 0; k < CONV_RAW; ++k, out += nqm)
     if (in[k].src) memcpy(out, in[k].src, (size_t)T.nq * sizeof(double));
     else std::fill(out, out + T.nq, in[k].dflt);

@@ -312,3 +312,23 @@ def test_moves_before_the_first_master_step_and_after():
         assert np.max(np.abs(r ** 3 / (grids.RE * p * pa["rho"] ** 2) - 1)) < 1e-13
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("prec", [KAOS_PREC_FP64, KAOS_PREC_MIXED])
+def test_missing_reference_frequency_of_a_moved_tube(prec):
+    """A NULL OmegaG0 table stands for zeros: a heated tube created with one,
+    or moved to one, has no finite kick and reports it."""
+    import ctypes as C
+    from kaos_b200 import lib as klib
+    mi, spec, t, vg = grids.config_small(n_particles=500, heating=True, steps_per_master=2)
+    mi.precision = prec
+    s = Solver(mi, [t], vg)
+    s.load(0, *grids.initial_particles(t, spec, mi, seed=2))
+    s.step(3)
+    new = grids.moved_tube(spec, mi, t, spec.L + 0.01)  # (holds the record's tables)
+    c = new.to_c()
+    c.OmegaG0 = None
+    assert klib.load().kaos_update_tube(s.h, 0, C.addressof(c)) == 0
+    with pytest.raises(KaosError, match="status 3"):
+        s.step(4)
+    s.close()
