@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes as C
 import dataclasses
+import operator
 import struct
 from typing import Optional
 
@@ -194,9 +195,11 @@ class Tube:
             a = np.ascontiguousarray(getattr(self, k), dtype=np.float64)
             setattr(self, k, a)
             ptr.append(a.__array_interface__["data"][0])
+        # (what a field's assignment takes: whole numbers, and what float takes)
         return KaosTube.from_buffer_copy(_TUBE_PACK.pack(
-            self.nq, self.capacity, self.pG, self.phiG, self.nsnormfac, self.nsnormCLB,
-            self.nsnormCUB, self.sumdsICR, *ptr, self.ms, self.qs))
+            operator.index(self.nq), operator.index(self.capacity), float(self.pG),
+            float(self.phiG), float(self.nsnormfac), float(self.nsnormCLB),
+            float(self.nsnormCUB), float(self.sumdsICR), *ptr, float(self.ms), float(self.qs)))
 
 
 @dataclasses.dataclass
