@@ -1938,8 +1938,11 @@ int kaos_set_export(kaos_handle *h, int32_t on) {
   if (on && !h->acc.hist) {
     int rc = dalloc(h, &h->acc.hist, (size_t)h->ncell * h->nv);
     if (rc) return rc;
-    CK(cudaMallocHost((void **)&h->cnt_stage, 2 * COUNT_STAGE * sizeof(unsigned)));
+    // dalloc's clearing, before the next step counts on its own stream
+    CK(cudaDeviceSynchronize());
   }
+  if (on && !h->cnt_stage)
+    CK(cudaMallocHost((void **)&h->cnt_stage, 2 * COUNT_STAGE * sizeof(unsigned)));
   h->export_on = on ? 1 : 0;
   return KAOS_OK;
 }

@@ -332,3 +332,38 @@ def test_missing_reference_frequency_of_a_moved_tube(prec):
     with pytest.raises(KaosError, match="status 3"):
         s.step(4)
     s.close()
+
+
+def test_export_switched_on_directly_before_a_step():
+    """A full histogram of 1 GB, cleared when it is made, counts the step that
+    follows at once."""
+    mi = ModelInput(h=0.01, ndatfac=50, ION2VPERPflag=1)
+    spec = TubeSpec(L=4.0, nq=256, n_particles=50000, q_ub=1e-3, H=600e3)
+    t = make_tube(spec, mi)
+    init = grids.initial_particles(t, spec, mi, seed=4)
+    s = Solver(mi, [t], make_vgrid(True, 100, 100, 100, 2e4))
+    s.load(0, *init)
+    s.set_export(True)
+    s.step(1)
+    full = s.counts(full=True).reshape(t.nq, -1).sum(axis=1)
+    np.testing.assert_array_equal(full, s.counts())
+    assert full.sum() == len(init[0])
+    s.close()
+
+
+def test_upper_boundary_injection_beside_the_push():
+    """Only the upper boundary open: its injection runs beside the push and is
+    committed with the moments."""
+    mi = ModelInput(h=0.01, ndatfac=3, ION2VPERPflag=1, LBCONDITIONflag=0, UBCONDITIONflag=1)
+    spec = TubeSpec(L=4.0, nq=24, n_particles=6000, q_ub=0.15, H=600e3)
+    t = make_tube(spec, mi)
+    t.nsnormCUB = 37.0
+    init = grids.initial_particles(t, spec, mi, seed=1)
+    vg = make_vgrid(True, 16, 16, 24, 8e3)
+    s, o = Solver(mi, [t], vg), Oracle(mi, t, vg)
+    for x in (s, o):
+        x.load(0, *init) if x is s else x.load(*init)
+        x.step(11)
+    assert s.boundary()[3] == 37
+    _compare(s, 0, o)
+    s.close()
