@@ -335,13 +335,13 @@ def test_missing_reference_frequency_of_a_moved_tube(prec):
 
 
 def test_export_switched_on_directly_before_a_step():
-    """A full histogram of 1 GB, cleared when it is made, counts the step that
+    """A full histogram of 256 MB, cleared when it is made, counts the step that
     follows at once."""
     mi = ModelInput(h=0.01, ndatfac=50, ION2VPERPflag=1)
     spec = TubeSpec(L=4.0, nq=256, n_particles=50000, q_ub=1e-3, H=600e3)
     t = make_tube(spec, mi)
     init = grids.initial_particles(t, spec, mi, seed=4)
-    s = Solver(mi, [t], make_vgrid(True, 100, 100, 100, 2e4))
+    s = Solver(mi, [t], make_vgrid(True, 64, 64, 64, 2e4))
     s.load(0, *init)
     s.set_export(True)
     s.step(1)
