@@ -292,9 +292,15 @@ int upload(kaos_handle *h, double **dst, const std::vector<double> &v) {
 
 // The captured steps hold kernel arguments and launch sequences of the time
 // of their capture.
-void drop_graphs(kaos_handle *h) {
-  for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-  h->graphs.clear();
+constexpr uint64_t GRAPH_MASTER = 1 << 16;  // bit of a captured step's key
+void drop_graphs(kaos_handle *h, bool masters_only = false) {
+  for (auto g = h->graphs.begin(); g != h->graphs.end();)
+    if (!masters_only || (g->first & GRAPH_MASTER)) {
+      cudaGraphExecDestroy(g->second.exec);
+      g = h->graphs.erase(g);
+    } else {
+      ++g;
+    }
 }
 
 bool is_master(const kaos_handle *h, int64_t n) {
@@ -330,6 +336,21 @@ constexpr int64_t FINE_SLOTS = (int64_t)1 << 21;
 bool fine_items(const kaos_handle *h) {
   const int64_t n = slots(h);
   return n <= (int64_t)1 << 18 && n * max_nq(h) <= (int64_t)1 << (h->mixed ? 26 : 27);
+}
+
+// Master-step pushes of the handles between those and FINE_SLOTS: items of 2048
+// ions, 4096 where a tube has more than 1024 cells, smaller while they make
+// less than 0.7 of a wave of blocks (us per step, every step a master step, at
+// these items / at the best of all shapes, 3e5 and 1.5e6 ions: mixed, 64 cells
+// 47 / 47 and 96 / 94, 1024 cells 69 / 63 and 176 / 177, 2048 cells 78 / 78
+// and 217 / 217; FP64, 64 cells 55 / 55 and 173 / 159).
+int mid_items(kaos_handle *h) {
+  const int nq = max_nq(h);
+  const int64_t fit = 227 * 1024 / ((int64_t)108 * nq + 4096);
+  const int64_t per_sm = h->mixed ? std::min<int64_t>(3, std::max<int64_t>(1, fit)) : 2;
+  int k = h->mixed && nq > 1024 ? NCHUNKS - 1 : 1;
+  while (k > 0 && 10 * h->wmap[k].n < 7 * per_sm * sm_count(h)) --k;
+  return k;
 }
 
 // Runs of steps (256-thread blocks, 4 per SM), ions per item: 256 below
@@ -1233,8 +1254,11 @@ int run_steps(kaos_handle *h, int64_t g) {
 // master step and at no other time: its pushes fill the binning accumulators,
 // which hold the counts of the latest master step (kaos_get_counts) until that
 // step clears them.  With the shape chosen by the ordinary push only its
-// register budget is left to choose; without, the budgets are timed at 4096
-// ions per item, the smaller items at the best of them (no persistent grid:
+// register budget is left to choose; without, a handle below FINE_SLOTS takes
+// the items of mid_items, since timing the sizes costs it more than a master
+// interval (1e6 ions, 97 cells: first interval 5.6 ms with, 3.6 without); above,
+// the budgets are timed at 4096 ions per item, the smaller items at the best of
+// them (no persistent grid:
 // 182 us against 179 at its best for the ordinary push of 1e7 ions; 1.5e6 ions
 // of 2048 cells, every step a master step, 219 us with and 214 without).  At
 // 1e7 ions 15 launches of 0.35 ms in place of 54 of 0.2 and 9 of 0.39.
@@ -1242,11 +1266,22 @@ constexpr int TUNE_AFTER = 4;
 int autotune(kaos_handle *h, bool master) {
   // (small items, fine_items: only the register budget is left to choose)
   const bool fine = h->fine && !h->forced;
-  const bool shaped = fine || !(h->tune_pending & kaos_handle::TUNE_ORDINARY);
+  const bool pushed = !(h->tune_pending & kaos_handle::TUNE_ORDINARY);
+  const bool shaped = fine || pushed || h->fmap.n > 0;
   const int nreg = h->mixed ? 3 : 1;
   h->tune_pending &= ~(master ? kaos_handle::TUNE_MASTER : kaos_handle::TUNE_ORDINARY);
-  if (nreg == 1 && (master ? shaped : fine)) return KAOS_OK;  // nothing to choose
   const int old[4] = {h->wsel, h->persistent, h->regsel, h->regsel_master};
+  auto changed = [&] {
+    if (old[0] != h->wsel || old[1] != h->persistent || old[2] != h->regsel) drop_graphs(h);
+    else if (old[3] != h->regsel_master) drop_graphs(h, true);
+    return KAOS_OK;
+  };
+  if (master && !pushed) {
+    if (!fine) h->wsel = h->fmap.n ? mid_items(h) : NCHUNKS - 1;
+    h->persistent = 0;
+    h->regsel = h->mixed ? 1 : 0;
+  }
+  if (nreg == 1 && (master ? shaped : fine)) return changed();  // nothing to time
   const int other = 1 - h->cur;
   const Fields F = ion_fields(h, h->cur, other);
   for (int f = 0; f < F.n; ++f)
@@ -1299,11 +1334,6 @@ int autotune(kaos_handle *h, bool master) {
     h->regsel = h->regsel_master = br;
     h->tune_pending |= kaos_handle::TUNE_MASTER;  // its budget in this shape
   } else {
-    if (!shaped) h->wsel = NCHUNKS - 1;
-    if (h->tune_pending & kaos_handle::TUNE_ORDINARY) {
-      h->persistent = 0;
-      h->regsel = h->mixed ? 1 : 0;
-    }
     int bm = 0, bw = h->wsel;
     for (int rs = 0; rs < nreg; ++rs) {
       h->regsel_master = rs;
@@ -1320,10 +1350,7 @@ int autotune(kaos_handle *h, bool master) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (old[0] != h->wsel || old[1] != h->persistent || old[2] != h->regsel ||
-      old[3] != h->regsel_master)
-    drop_graphs(h);
-  return KAOS_OK;
+  return changed();
 }
 
 // Steps of one kind replayed from a cached CUDA graph.  A graph holds g
@@ -1336,7 +1363,7 @@ int graph_steps(kaos_handle *h, int g) {
   const int64_t n = h->n + 1;
   // a master step is replayed alone; whether it compacts is decided first
   const int compact = is_master(h, n) ? bc_decide(h, n) : 0;
-  const uint64_t key = (uint64_t)g | ((uint64_t)is_master(h, n) << 16) |
+  const uint64_t key = (uint64_t)g | (is_master(h, n) ? GRAPH_MASTER : 0) |
                        ((uint64_t)compact << 21) |
                        ((uint64_t)is_master(h, n + 1) << 17) |
                        ((uint64_t)h->cur << 18) | ((uint64_t)h->ecur << 19) |
