@@ -362,13 +362,13 @@ int kaos_set_graph(kaos_handle *h, int32_t on);
  * per SM), 1 = 80 registers (3 blocks of 256), 2 = 72 registers (7 blocks
  * of 128); bits 3-4 (mixed): the budget of the master-step variant plus
  * one (0 = the same as bits 1-2).  chunk = 0 or mode < 0 re-arms the
- * autotuner, which is on by default: directly before the first master step it
+ * autotuner, which is on by default: before the first step after step 1 it
  * times the master-step variant of the push for every register budget and
- * item size on a copy of the ion state and keeps the fastest; the push of
- * ordinary steps is timed too (every candidate) where the handle uses it one
- * step at a time: before a step whose interval converts ions, or after four
- * ordinary steps made one by one.  The counts of the latest master step
- * (kaos_get_counts) are not touched by it.  Runs of steps
+ * (handles of 2^21 slots or more) item size on a copy of the ion state and
+ * keeps the fastest; the push of ordinary steps is timed too (every candidate)
+ * where the handle uses it one step at a time: before a step whose interval
+ * converts ions, or after four ordinary steps made one by one.  The counts of
+ * the latest master step (kaos_get_counts) stay what they were.  Runs of steps
  * (kaos_step) have a shape of their own, and a small handle (up to 2^18
  * slots, fewer with more than 256 cells) takes items of 256 ions while no
  * shape is set here (reported as 1024, the smallest that can be set).  Results

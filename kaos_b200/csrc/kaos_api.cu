@@ -119,6 +119,7 @@ struct kaos_handle {
   size_t stat_bytes = 0, zero_bytes = 0;
   unsigned *cnt_stage = nullptr;  // kaos_get_counts: 2 x COUNT_STAGE, pinned
   int stat_ok = 0;  // stat_host holds the device's values
+  unsigned *d_cnt_keep = nullptr;  // the ion counts during the shape timing
   // device
   TubeD *d_tubes = nullptr;
   int *d_blk_tube = nullptr;
@@ -1250,10 +1251,10 @@ int run_steps(kaos_handle *h, int64_t g) {
 // that uses it: its interval converts ions, or it has made TUNE_AFTER
 // ordinary steps that were no part of a run.
 //
-// The master-step variant, which every handle uses, is timed directly before a
-// master step and at no other time: its pushes fill the binning accumulators,
-// which hold the counts of the latest master step (kaos_get_counts) until that
-// step clears them.  With the shape chosen by the ordinary push only its
+// The master-step variant, which every handle uses, bins the copy into the
+// accumulators.  Of those a caller reads the ion counts and the full histogram
+// until the next master step clears them all (kaos_get_counts): the counts are
+// put back afterwards, and the timing leaves the histogram out.  With the shape chosen by the ordinary push only its
 // register budget is left to choose; without, a handle below FINE_SLOTS takes
 // the items of mid_items, since timing the sizes costs it more than a master
 // interval (1e6 ions, 97 cells: first interval 5.6 ms with, 3.6 without); above,
@@ -1297,7 +1298,10 @@ int autotune(kaos_handle *h, bool master) {
     a.ion = h->ion[other];
     a.step = (uint32_t)(h->n + 1);
     a.write_qind = 1;
-    if (master) a.bin = a.prologue = 1;
+    if (master) {
+      a.bin = a.prologue = 1;
+      a.exporting = 0;
+    }
     else a.write_qk4 = 0;
     *tmin = 1e30f;
     for (int rep = 0; rep < 3; ++rep) {
@@ -1334,6 +1338,8 @@ int autotune(kaos_handle *h, bool master) {
     h->regsel = h->regsel_master = br;
     h->tune_pending |= kaos_handle::TUNE_MASTER;  // its budget in this shape
   } else {
+    const size_t counts = (size_t)h->ncell * sizeof(unsigned);
+    CK(cudaMemcpyAsync(h->d_cnt_keep, h->acc.cnt, counts, cudaMemcpyDeviceToDevice, h->s));
     int bm = 0, bw = h->wsel;
     for (int rs = 0; rs < nreg; ++rs) {
       h->regsel_master = rs;
@@ -1347,6 +1353,7 @@ int autotune(kaos_handle *h, bool master) {
       if (t < best) { best = t; bw = m; }
     }
     h->wsel = bw;
+    CK(cudaMemcpyAsync(h->acc.cnt, h->d_cnt_keep, counts, cudaMemcpyDeviceToDevice, h->s));
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1698,6 +1705,7 @@ int kaos_create(const kaos_params_c *p, const kaos_tube_c *tubes,
   if ((rc = dalloc(h, &h->d_blkcnt, bt.size()))) return rc;
   if ((rc = dalloc(h, &h->d_blkoff, bt.size()))) return rc;
   if ((rc = dalloc(h, &h->d_step, 1))) return rc;
+  if ((rc = dalloc(h, &h->d_cnt_keep, coff))) return rc;
   // particle arrays (two buffer sets for the order-preserving compaction)
   const int64_t cap = poff;
   h->ion_len = cap;
@@ -2123,9 +2131,7 @@ int kaos_step(kaos_handle *h, int64_t nsteps) {
                             h->tune_singles >= TUNE_AFTER;
       if ((h->tune_pending & kaos_handle::TUNE_ORDINARY) && ordinary && (rc = autotune(h, false)))
         return rc;
-      if ((h->tune_pending & kaos_handle::TUNE_MASTER) && is_master(h, n) &&
-          (rc = autotune(h, true)))
-        return rc;
+      if ((h->tune_pending & kaos_handle::TUNE_MASTER) && (rc = autotune(h, true))) return rc;
     }
     const int64_t r = run_length(h, n, nsteps - k);
     if (r > 0) {
