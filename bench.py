@@ -66,7 +66,7 @@ def fp64_pipe_roofline(rate_per_gpu):
             "peak_kind": "nominal", "f_alg": F_ALG,
             "weights": "add/mul 1, div/sqrt 4, transcendental call 20",
             "note": "operations of the reference formulation; the path takes the same "
-                    "trajectories with fewer (about 300 FP64 instructions per ion-step), so "
+                    "trajectories with fewer (about 350 FP64 instructions per ion-step), so "
                     "the ratio can exceed 1"}
 
 

@@ -517,19 +517,19 @@ int launch_push(kaos_handle *h, const PushArgs &a) {
       {{k_push64<false, 256, 2, false, false, true>, k_push64<false, 256, 2, true, false, true>},
        {k_push64<true, 256, 2, false, false, true>, k_push64<true, 256, 2, true, false, true>}}};
   // FP64 runs, [many items][heating][three_d]: 64 registers (32 warps per SM,
-  // 120-150 B of spills) where there are several waves of blocks, else 80 (24
-  // warps, 60-80 B): ms per 20 steps 1e7 ions 6.20 / 6.35, 1e5 ions 0.143 /
-  // 0.127 (124 registers, 16 warps, no spills: 6.75, 0.137)
+  // 120 B of spills) where there are several waves of blocks, else 80 (24
+  // warps, 40 B), ms per 20 steps at 64 / 80: heated 1e7 ions 6.32 / 6.36, 1e5
+  // ions 0.152 / 0.128, unheated 1e5 ions 0.110 / 0.095
   static const KFn k64run[2][2][2] = {
       {{k_push64<false, 256, 3, false, true, false>, k_push64<true, 256, 3, false, true, false>},
        {k_push64<false, 256, 3, false, true, true>, k_push64<true, 256, 3, false, true, true>}},
       {{k_push64<false, 256, 4, false, true, false>, k_push64<true, 256, 4, false, true, false>},
        {k_push64<false, 256, 4, false, true, true>, k_push64<true, 256, 4, false, true, true>}}};
   // runs of steps: [no heating, FP32 kick, FP64 kick][three_d].  64 registers
-  // (32 warps per SM; 8 B of spills, 100 B with the FP64 kick) against 79 (24
-  // warps, 0 and 28 B), ms per 20 steps: 1e7 ions 2.78 / 2.81, FP64 kick 4.30
-  // / 4.33, 1e8 ions 26.6 / 27.0, 256 uneven tubes 15.16 / 15.40; 128-thread
-  // blocks are up to 30 % slower on the uneven tubes (twice the table set-ups)
+  // (32 warps per SM; 8 B of spills, 96 B with the FP64 kick) against 80 (24
+  // warps) and 72 (28 warps in 128-thread blocks, twice the table set-ups), ms
+  // per 20 steps: 1e7 ions 2.67 / 2.77 / 2.76, FP64 kick 4.09 / 4.10 / 4.11,
+  // 1e8 ions 25.7 / 26.9 / 27.8, 256 uneven tubes 14.74 / 15.40 / 15.92
   static const KFn k32run[3][2] = {
       {k_push32<false, 256, 4, false, false, false, true, false>,
        k_push32<true, 256, 4, false, false, false, true, false>},

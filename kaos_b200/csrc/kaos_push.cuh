@@ -297,7 +297,11 @@ template <typename T> struct HeatC {
 //   kick_i = K_i x^(-chi_i/2) Sigma^(-3/2) sqrt(Omega s) G_i,  s = sqrt(eps),
 // applied while h <= tau, i.e. h Omega s <= 2 pi (stochastic branch);
 // the coherent branch kicks |Vperp| by sqrt(k1^2+k2^2) G1 with a uniform
-// gyro-angle.  invOm = 1/Omega is passed in (no division needed).
+// gyro-angle.  invOm = 1/Omega is passed in (no division needed).  Every caller
+// is coherent: the stochastic kick has a form of its own in each mode (heat32,
+// heat64t, heat64x).  Its branch at the end is kept for the code around it:
+// without it the compiler spills 72 bytes of the mixed run in place of 8, 2.81
+// ms per 20 steps of 1e7 ions in place of 2.67.
 template <typename T>
 __device__ __forceinline__ void heat(const PushArgs &a, uint32_t step,
                                      const HeatC<T> &c, uint64_t id,
@@ -1430,9 +1434,9 @@ __global__ void __launch_bounds__(NT, MINB) k_push32(PushArgs a) {
     // hemisphere sign of the start.  The general expressions serve the rest.
     // (Every multiply-add written out: the same rounding in every variant of
     // the kernel.)
-    // (All through the meridian point in FP64, as the general ones are: 367
-    // instructions per ion and step where this takes 319, 3.05 ms per 20
-    // steps of 1e7 ions where this takes 2.83, and an error of q some 20
+    // (All through the meridian point in FP64, as the general ones are: 338
+    // instructions per ion and step where this takes 324, 2.86 ms per 20
+    // steps of 1e7 ions where this takes 2.67, and an error of q some 20
     // times larger after 100 steps, from the refinements' ~1e-14 a step.)
     double qN, dq = 0.0, od;
     float a2 = fmaf(dM, ds2, M1), a4 = fmaf(dM, ds4, M1), dal;
