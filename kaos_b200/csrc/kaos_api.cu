@@ -597,7 +597,6 @@ const double *conv_table_ptr(const CellTables &c, int k) {
 // their ions with the old tables and descriptors (k_convect_many), then put
 // the new tables and descriptors in place (k_apply_tables) from one staging
 // copy.
-static int sm_count(kaos_handle *h);
 
 // Staging of the moves of one master step: room for every entry at once.
 int conv_staging(kaos_handle *h) {
