@@ -593,11 +593,6 @@ const double *conv_table_ptr(const CellTables &c, int k) {
   return p[k];
 }
 
-// Move the tubes given to kaos_update_tube, all in two launches: re-project
-// their ions with the old tables and descriptors (k_convect_many), then put
-// the new tables and descriptors in place (k_apply_tables) from one staging
-// copy.
-
 // Staging of the moves of one master step: room for every entry at once.
 int conv_staging(kaos_handle *h) {
   if (h->conv_host.stage) return KAOS_OK;
@@ -613,6 +608,10 @@ int conv_staging(kaos_handle *h) {
   return KAOS_OK;
 }
 
+// Move the tubes given to kaos_update_tube, all in two launches: re-project
+// their ions with the old tables and descriptors (k_convect_many), then put
+// the new tables and descriptors in place (k_apply_tables) from one staging
+// copy.
 int apply_pending_tubes(kaos_handle *h) {
   const int np = (int)h->pending.size();
   if (!np) return KAOS_OK;
